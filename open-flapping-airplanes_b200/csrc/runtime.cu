@@ -14,6 +14,8 @@
 #include <vector>
 #include <map>
 #include <algorithm>
+#include <atomic>
+#include <mutex>
 
 using namespace ofa;
 
@@ -37,16 +39,12 @@ int shuffle_multiplier(unsigned seed, int phase, int n) {
 struct HostPhase { std::string name; PhaseDesc d; std::vector<Dep> deps; std::vector<char> rb_grain;   // per dependency: 1 = wait per 128-token row block instead of for the whole producer phase
                    int rb_map = 0; };                                                                   // how this phase's tasks map to row blocks (RbKind | a << 8), 0 = they do not
 
-struct DevJob {
-  Job j{};
-  PhaseDesc* ph = nullptr; SchedRec* rec = nullptr; int *prefix = nullptr, *ntasks = nullptr, *dep_off = nullptr, *dep_cnt = nullptr; Dep* deps = nullptr;
-  int* done = nullptr; int* done_rb = nullptr; unsigned* ticket = nullptr;
-  int nph = 0;
-  std::vector<SchedRec> hrec;   // host copy of the scheduling records: they also travel inside the kernel parameter when they fit
-  void free_all() {
-    cudaFree(ph); cudaFree(rec); rec = nullptr; cudaFree(prefix); cudaFree(ntasks); cudaFree(dep_off); cudaFree(dep_cnt); cudaFree(deps); cudaFree(done); cudaFree(done_rb); cudaFree(ticket);
-    *this = DevJob();
-  }
+// A job on the device: its tables (phase descriptors, scheduling records, prefix sums, dependencies) and its counters. Both live in
+// memory of the caller: a context uploads the tables once and only clears the counters before each launch; ofa_run_phases packs
+// them into its workspace.
+struct HostJob {
+  std::vector<PhaseDesc> pd; std::vector<SchedRec> rec; std::vector<int> prefix, nt, doff, dcnt; std::vector<Dep> deps;
+  int nph = 0, last_phase = 0, rb_total = 0;
 };
 
 struct Span { size_t off, n; };
@@ -100,6 +98,7 @@ bool encode_map(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer
 struct Arena {   // device allocations owned by one context / one ofa_run_phases call
   std::vector<void*> ptrs;
   bool ok = true;
+  cudaStream_t stream = nullptr;   // zero fills and uploads are ordered on this stream, so the owner's launches on it follow them
   bool dry = false;            // planning mode (no device): hands out distinct, aligned, never-dereferenced addresses
   uintptr_t bump = 0x100000000ull;
   template <class T> T* alloc(size_t n, bool zero = true) {
@@ -107,28 +106,50 @@ struct Arena {   // device allocations owned by one context / one ofa_run_phases
     if (n == 0) n = 1;
     if (dry) { p = reinterpret_cast<void*>(bump); bump += (n * sizeof(T) + 1023) / 1024 * 1024; return reinterpret_cast<T*>(p); }
     if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) { ok = false; return nullptr; }
-    if (zero) cudaMemset(p, 0, n * sizeof(T));
+    if (zero) cudaMemsetAsync(p, 0, n * sizeof(T), stream);
     ptrs.push_back(p);
     return reinterpret_cast<T*>(p);
   }
-  void h2d(void* dst, const void* src, size_t bytes) { if (!dry) cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice); }
+  void h2d(void* dst, const void* src, size_t bytes) { if (!dry) cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream); }   // pageable source: staged before the call returns
   void free_all() { for (void* p : ptrs) cudaFree(p); ptrs.clear(); }
 };
 
+// Where the TMA descriptors of phases go: one by one into a context's arena, or (ofa_run_phases) into the call's packed tables, which
+// are uploaded in one copy.
+struct MapSink {
+  Arena* ar = nullptr;
+  unsigned char *host = nullptr, *dev = nullptr; size_t used = 0, cap = 0;
+  bool dry() const { return ar && ar->dry; }
+  // device address of n descriptors with the given contents, 64-byte aligned
+  const void* put(const void* maps, size_t bytes) {
+    if (ar) {
+      unsigned char* d = ar->alloc<unsigned char>(bytes, false);
+      if (d && !ar->dry) ar->h2d(d, maps, bytes);
+      return d;
+    }
+    if (used + bytes > cap) return nullptr;
+    memcpy(host + used, maps, bytes);
+    const void* d = dev + used;
+    used += (bytes + 63) / 64 * 64;
+    return d;
+  }
+};
+
 // TMA descriptors of one layer's attention operands (qkv [N, 3D] and, for the backward tasks, dO [N, D]) in device memory
-const void* make_attn_maps(Arena& ar, const void* qkv, const void* dO, int N, int D, std::string& err) {
-  attn_tc::Maps* dm = ar.alloc<attn_tc::Maps>(1, false);
-  if (ar.dry || !dm) return dm;
+const void* make_attn_maps(MapSink& sink, const void* qkv, const void* dO, int N, int D, std::string& err) {
   attn_tc::Maps hm; memset(&hm, 0, sizeof hm);
-  bool ok = encode_map(&hm.qkv128, qkv, 3 * D, N, 3 * D, 64, 128) && encode_map(&hm.qkv64, qkv, 3 * D, N, 3 * D, 64, 64);
-  if (dO) ok = ok && encode_map(&hm.dO128, dO, D, N, D, 64, 128) && encode_map(&hm.dO64, dO, D, N, D, 64, 64);
-  if (!ok) { err = "cuTensorMapEncodeTiled failed (attention)"; return nullptr; }
-  ar.h2d(dm, &hm, sizeof hm);
-  return dm;
+  if (!sink.dry()) {
+    bool ok = encode_map(&hm.qkv128, qkv, 3 * D, N, 3 * D, 64, 128) && encode_map(&hm.qkv64, qkv, 3 * D, N, 3 * D, 64, 64);
+    if (dO) ok = ok && encode_map(&hm.dO128, dO, D, N, D, 64, 128) && encode_map(&hm.dO64, dO, D, N, D, 64, 64);
+    if (!ok) { err = "cuTensorMapEncodeTiled failed (attention)"; return nullptr; }
+  }
+  const void* d = sink.put(&hm, sizeof hm);
+  if (!d) err = "out of device memory (attention maps)";
+  return d;
 }
 
 // Validates a GEMM description for the tensor-core path and fills task counts + TMA descriptors (device memory).
-bool prepare_gemm_bf16(PhaseDesc& d, Arena& ar, int nsub_cfg, int nblocks, std::string& err) {
+bool prepare_gemm_bf16(PhaseDesc& d, MapSink& sink, int nsub_cfg, int nblocks, std::string& err) {
   GemmArgs& g = d.g;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.M % 128 || g.N % 128 || g.K % 64 || g.lda % 8 || g.ldb % 8 || g.ldc % 8 ||
@@ -165,15 +186,15 @@ bool prepare_gemm_bf16(PhaseDesc& d, Arena& ar, int nsub_cfg, int nblocks, std::
   g.nsub = nsub;
   d.tiles_m = tm;
   d.ntasks = tm * ((tn + nsub - 1) / nsub);
-  if (ar.dry) { g.tmA = ar.alloc<CUtensorMap>(2, false); g.tmB = reinterpret_cast<const CUtensorMap*>(g.tmA) + 1; return true; }
-  CUtensorMap hm[2];
-  const bool a_kmajor = d.layout != GL_TN, b_kmajor = d.layout == GL_NT;
-  bool ok = a_kmajor ? encode_map(&hm[0], g.A, g.K, g.M, g.lda, 64, 128) : encode_map(&hm[0], g.A, g.M, g.K, g.lda, 64, 64);
-  ok = ok && (b_kmajor ? encode_map(&hm[1], g.B, g.K, g.N, g.ldb, 64, 128) : encode_map(&hm[1], g.B, g.N, g.K, g.ldb, 64, 64));
-  if (!ok) { err = "cuTensorMapEncodeTiled failed"; return false; }
-  CUtensorMap* dm = ar.alloc<CUtensorMap>(2, false);
-  if (!dm) { err = "cudaMalloc failed"; return false; }
-  cudaMemcpy(dm, hm, sizeof hm, cudaMemcpyHostToDevice);
+  CUtensorMap hm[2]; memset(hm, 0, sizeof hm);
+  if (!sink.dry()) {
+    const bool a_kmajor = d.layout != GL_TN, b_kmajor = d.layout == GL_NT;
+    bool ok = a_kmajor ? encode_map(&hm[0], g.A, g.K, g.M, g.lda, 64, 128) : encode_map(&hm[0], g.A, g.M, g.K, g.lda, 64, 64);
+    ok = ok && (b_kmajor ? encode_map(&hm[1], g.B, g.K, g.N, g.ldb, 64, 128) : encode_map(&hm[1], g.B, g.N, g.K, g.ldb, 64, 64));
+    if (!ok) { err = "cuTensorMapEncodeTiled failed"; return false; }
+  }
+  const CUtensorMap* dm = reinterpret_cast<const CUtensorMap*>(sink.put(hm, sizeof hm));
+  if (!dm) { err = "out of device memory (TMA descriptors)"; return false; }
   g.tmA = dm; g.tmB = dm + 1;
   return true;
 }
@@ -184,9 +205,11 @@ void prepare_gemm_f32(PhaseDesc& d) {
 }
 
 // nrb = number of 128-token row blocks (0: no phase counts completions per row block, every dependency is phase-level)
-bool upload_job(const std::vector<HostPhase>& ph, int last_phase, int nsteps, DevJob& dj, std::string& err, int nrb = 0) {
+bool make_job(const std::vector<HostPhase>& ph, int last_phase, HostJob& hj, std::string& err, int nrb = 0) {
   const int nph = (int)ph.size();
-  std::vector<PhaseDesc> pd(nph); std::vector<int> prefix(nph + 1, 0), nt(nph), doff(nph), dcnt(nph); std::vector<Dep> deps;
+  hj = HostJob();
+  std::vector<PhaseDesc>& pd = hj.pd; std::vector<int>&prefix = hj.prefix, &nt = hj.nt, &doff = hj.doff, &dcnt = hj.dcnt; std::vector<Dep>& deps = hj.deps;
+  pd.resize(nph); prefix.assign(nph + 1, 0); nt.resize(nph); doff.resize(nph); dcnt.resize(nph);
   for (int i = 0; i < nph; i++) {
     pd[i] = ph[i].d; nt[i] = ph[i].d.ntasks; prefix[i + 1] = prefix[i] + nt[i];
     doff[i] = (int)deps.size(); dcnt[i] = (int)ph[i].deps.size();
@@ -196,7 +219,6 @@ bool upload_job(const std::vector<HostPhase>& ph, int last_phase, int nsteps, De
     }
     if (nt[i] <= 0) { err = "phase without tasks: " + ph[i].name; return false; }
   }
-  if ((double)prefix[nph] * (double)nsteps >= 4.0e9) { err = "ticket counter would overflow"; return false; }
   if (nph >= 65536) { err = "too many phases"; return false; }
   // which phases count their completions per row block: those that say how their tasks map to row blocks, have a whole number of
   // tasks per row block, and are waited for at that grain by somebody
@@ -207,7 +229,7 @@ bool upload_job(const std::vector<HostPhase>& ph, int last_phase, int nsteps, De
         const int p = ph[i].deps[k].phase;
         if (k < ph[i].rb_grain.size() && ph[i].rb_grain[k] && ph[i].rb_map && ph[p].rb_map && nt[p] % nrb == 0 && rb_off[p] < 0) { rb_off[p] = rb_total; rb_total += nrb; }
       }
-  std::vector<SchedRec> rec(nph);
+  std::vector<SchedRec>& rec = hj.rec; rec.resize(nph);
   for (int i = 0; i < nph; i++) {
     SchedRec& r = rec[i]; memset(&r, 0, sizeof(r));
     r.lo = prefix[i]; r.hi = prefix[i + 1];
@@ -223,43 +245,59 @@ bool upload_job(const std::vector<HostPhase>& ph, int last_phase, int nsteps, De
     }
   }
   if (deps.empty()) deps.push_back(Dep{0, 0});
-  dj.free_all();
-  bool ok = cudaMalloc(&dj.ph, sizeof(PhaseDesc) * nph) == cudaSuccess && cudaMalloc(&dj.prefix, 4 * (nph + 1)) == cudaSuccess &&
-            cudaMalloc(&dj.ntasks, 4 * nph) == cudaSuccess && cudaMalloc(&dj.dep_off, 4 * nph) == cudaSuccess &&
-            cudaMalloc(&dj.dep_cnt, 4 * nph) == cudaSuccess && cudaMalloc(&dj.deps, sizeof(Dep) * deps.size()) == cudaSuccess &&
-            cudaMalloc(&dj.done, 4 * nph) == cudaSuccess && cudaMalloc(&dj.ticket, 4) == cudaSuccess &&
-            cudaMalloc(&dj.rec, sizeof(SchedRec) * nph) == cudaSuccess && cudaMalloc(&dj.done_rb, 4 * (size_t)std::max(1, rb_total)) == cudaSuccess;
-  if (!ok) { err = "cudaMalloc failed (job tables)"; return false; }
-  cudaMemcpy(dj.ph, pd.data(), sizeof(PhaseDesc) * nph, cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.rec, rec.data(), sizeof(SchedRec) * nph, cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.prefix, prefix.data(), 4 * (nph + 1), cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.ntasks, nt.data(), 4 * nph, cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.dep_off, doff.data(), 4 * nph, cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.dep_cnt, dcnt.data(), 4 * nph, cudaMemcpyHostToDevice);
-  cudaMemcpy(dj.deps, deps.data(), sizeof(Dep) * deps.size(), cudaMemcpyHostToDevice);
-  cudaMemset(dj.done, 0, 4 * nph); cudaMemset(dj.ticket, 0, 4); cudaMemset(dj.done_rb, 0, 4 * (size_t)std::max(1, rb_total));
-  dj.nph = nph; dj.hrec = rec;
-  dj.j.nph = nph; dj.j.tasks_per_step = prefix[nph]; dj.j.nsteps = nsteps; dj.j.last_phase = last_phase;
-  dj.j.ph = dj.ph; dj.j.prefix = dj.prefix; dj.j.ntasks = dj.ntasks; dj.j.dep_off = dj.dep_off; dj.j.dep_cnt = dj.dep_cnt; dj.j.deps = dj.deps; dj.j.rec = dj.rec;
-  dj.j.done = dj.done; dj.j.done_rb = dj.done_rb; dj.j.ticket = dj.ticket;
+  hj.nph = nph; hj.last_phase = last_phase; hj.rb_total = rb_total;
   return true;
+}
+bool tickets_fit(const HostJob& hj, long nsteps, std::string& err) {
+  if ((double)hj.prefix[hj.nph] * (double)nsteps >= 4.0e9) { err = "ticket counter would overflow"; return false; }
+  return true;
+}
+constexpr size_t up64(size_t n) { return (n + 63) / 64 * 64; }
+size_t job_table_bytes(const HostJob& h) {
+  return up64(sizeof(PhaseDesc) * h.nph) + up64(sizeof(SchedRec) * h.nph) + up64(4 * ((size_t)h.nph + 1)) + 3 * up64(4 * (size_t)h.nph) + up64(sizeof(Dep) * h.deps.size());
+}
+size_t job_counter_bytes(const HostJob& h) { return 64 + up64(4 * (size_t)h.nph) + up64(4 * (size_t)std::max(1, h.rb_total)); }
+// writes the tables to `host` (an image of `dev`) and fills the job's pointers; `cnt` = its counters, to be zero before a launch
+Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* dev, unsigned char* cnt) {
+  Job j{};
+  size_t o = 0;
+  auto put = [&](const void* src, size_t bytes) { memcpy(host + o, src, bytes); const void* d = dev + o; o += up64(bytes); return d; };
+  j.ph = reinterpret_cast<const PhaseDesc*>(put(h.pd.data(), sizeof(PhaseDesc) * h.nph));
+  j.rec = reinterpret_cast<const SchedRec*>(put(h.rec.data(), sizeof(SchedRec) * h.nph));
+  j.prefix = reinterpret_cast<const int*>(put(h.prefix.data(), 4 * ((size_t)h.nph + 1)));
+  j.ntasks = reinterpret_cast<const int*>(put(h.nt.data(), 4 * (size_t)h.nph));
+  j.dep_off = reinterpret_cast<const int*>(put(h.doff.data(), 4 * (size_t)h.nph));
+  j.dep_cnt = reinterpret_cast<const int*>(put(h.dcnt.data(), 4 * (size_t)h.nph));
+  j.deps = reinterpret_cast<const Dep*>(put(h.deps.data(), sizeof(Dep) * h.deps.size()));
+  j.ticket = reinterpret_cast<unsigned*>(cnt); j.done = reinterpret_cast<int*>(cnt + 64); j.done_rb = reinterpret_cast<int*>(cnt + 64 + up64(4 * (size_t)h.nph));
+  j.nph = h.nph; j.tasks_per_step = h.prefix[h.nph]; j.nsteps = nsteps; j.last_phase = h.last_phase;
+  return j;
 }
 
 // copies a job's scheduling records into the kernel parameter when they fit
-void fill_param_records(Ctx& C, const DevJob* train, const DevJob* dec) {
+void fill_param_records(Ctx& C, const HostJob* train, const HostJob* dec) {
   C.train_rec_n = 0; C.dec_rec_n = 0;
   C.sched_flags = getenv("OFA_B200_LATE_TICKETS") ? 4 : 0;     // A/B switch for measurements: tickets only at the end of a task
   if (getenv("OFA_B200_GLOBAL_RECS")) return;      // A/B switch for measurements: keep using the records in global memory
-  if (train && train->nph > 0 && train->nph <= PARAM_TRAIN_PH) { memcpy(C.train_rec, train->hrec.data(), sizeof(SchedRec) * train->nph); C.train_rec_n = train->nph; }
-  if (dec && dec->nph > 0 && dec->nph <= PARAM_DEC_PH) { memcpy(C.dec_rec, dec->hrec.data(), sizeof(SchedRec) * dec->nph); C.dec_rec_n = dec->nph; }
+  if (train && train->nph > 0 && train->nph <= PARAM_TRAIN_PH) { memcpy(C.train_rec, train->rec.data(), sizeof(SchedRec) * train->nph); C.train_rec_n = train->nph; }
+  if (dec && dec->nph > 0 && dec->nph <= PARAM_DEC_PH) { memcpy(C.dec_rec, dec->rec.data(), sizeof(SchedRec) * dec->nph); C.dec_rec_n = dec->nph; }
 }
 
-template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nblocks, int smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
-  // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
-  cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nblocks, int smem, int device, cudaStream_t s) {
+  static std::atomic<int> allowed[64];     // per device: the largest dynamic shared memory the kernel has been allowed so far
+  std::atomic<int>* a = device >= 0 && device < 64 ? &allowed[device] : nullptr;
+  if (!a || a->load(std::memory_order_acquire) < smem) {
+    static std::mutex mu;                  // two threads must not lower the limit below what the other just raised it to
+    std::lock_guard<std::mutex> lk(mu);
+    if (!a || a->load(std::memory_order_relaxed) < smem) {
+      cudaError_t e = cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return e;
+      // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
+      // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
+      cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (a) a->store(smem, std::memory_order_release);
+    }
+  }
   ofa_kernel<T, D, DH><<<nblocks, NTHR, smem, s>>>(C);
   return cudaGetLastError();
 }
@@ -309,7 +347,10 @@ struct ofa_ctx {
   uint32_t* d_tokens = nullptr; size_t ntok = 0; uint32_t* d_starts = nullptr; int nstarts = 0;
   std::map<std::string, std::pair<void*, size_t>> bufs;
   std::vector<HostPhase> train_ph, dec_ph; int train_last = 0, dec_last = 0;
-  DevJob train_job, dec_job;
+  HostJob train_job, dec_job;        // the uploaded jobs
+  unsigned char* d_jobs = nullptr; size_t jobs_cnt_off = 0, jobs_cnt_bytes = 0;   // tables of both jobs, then everything a launch starts from zero: counters, status, finished words
+  bool jobs_ready = false; unsigned jobs_seed = 0;
+  unsigned char* h_back = nullptr;   // pinned: what every launch copies back (device status, then the decoder's scalars)
   Ctx C{};
   DevStatus* d_status = nullptr;
   int* d_finished = nullptr; unsigned long long* d_t_end = nullptr;
@@ -322,7 +363,7 @@ struct ofa_ctx {
   int* d_forced = nullptr; int* d_scal = nullptr;
   int* d_ext_ready = nullptr; int* d_ext_done = nullptr;   // device flags [32] each: gradients of bucket b ready / all-reduce of bucket b done
   std::vector<Span> buckets;
-  cudaStream_t stream = nullptr, abort_stream = nullptr; cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaStream_t stream = nullptr, abort_stream = nullptr; cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;   // start, end of the kernel, results copied back
   bool dry = false;
   int step_done_cap = 0; size_t starts_cap = 0, tokens_cap = 0;
   bool abort_requested = false;      // ofa_abort was called for the launch in flight (also honoured if the device word was cleared by a launch that had not started yet)
@@ -390,6 +431,7 @@ bool build_train_graph(ofa_ctx* c) {
     std::vector<std::string> pv; for (auto& e : deps_prev) if (!e.empty()) pv.push_back(e);
     prevdeps.push_back(pv);
   };
+  MapSink sink; sink.ar = &c->ar;
   auto mk = [&](int kind, int ntasks) { PhaseDesc d; memset(&d, 0, sizeof d); d.kind = kind; d.ntasks = ntasks; return d; };
   // wide = 1: 128 x 256 tiles where the width allows (a long K and more tiles than blocks: only the LM head's weight gradient)
   auto mkgemm = [&](int layout, int epi, const void* A, int lda, const void* B, int ldb, void* Cc, int ldc, void* aux, int ldaux,
@@ -400,7 +442,7 @@ bool build_train_graph(ofa_ctx* c) {
     // wide: 128 x 256 tiles, one tile per task, tasks ordered along N first (the three readers of a 128-row slice of the large
     // operand run side by side and share it through L2); OFA_B200_HEAD_DW_128 / _STRIPS keep the other two forms for A/B runs
     const int nsub_cfg = (wide && cfg.gemm_nsub == 0 && !getenv("OFA_B200_HEAD_DW_128")) ? (getenv("OFA_B200_HEAD_DW_STRIPS") ? 2000 : 4001) : cfg.gemm_nsub;
-    if (bf) { std::string e; if (!prepare_gemm_bf16(d, c->ar, nsub_cfg, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }   // waves are counted over the blocks that train
+    if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, nsub_cfg, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }   // waves are counted over the blocks that train
     else prepare_gemm_f32(d);
     return d;
   };
@@ -455,7 +497,7 @@ bool build_train_graph(ofa_ctx* c) {
       addp(s + "ln1", d, {prev}, {opt_layer(l)}, {prev}); }
     addp(s + "qkv", mkgemm(GL_NN, GE_STORE, ln1[l], D, Wact + lay.wqkv[l], 3 * D, qkv[l], 3 * D, nullptr, 0, N, 3 * D, D, 0), {s + "ln1"}, {}, {s + "ln1"});
     { PhaseDesc d = mk(TK_ATT_FWD, attn_fwd_tasks); d.p[0] = qkv[l]; d.p[1] = att[l]; d.p[2] = lse[l];
-      if (bf) { std::string e; d.p[6] = const_cast<void*>(make_attn_maps(c->ar, qkv[l], nullptr, N, D, e)); if (!d.p[6]) { ok = false; err = e; } }
+      if (bf) { std::string e; d.p[6] = const_cast<void*>(make_attn_maps(sink, qkv[l], nullptr, N, D, e)); if (!d.p[6]) { ok = false; err = e; } }
       addp(s + "attn", d, {s + "qkv"}, {}, {s + "qkv"}); }
     addp(s + "wo+res", mkgemm(GL_NN, GE_RES, att[l], D, Wact + lay.wo[l], D, hb[l], D, xs[l], D, N, D, D, 0), {s + "attn"}, {}, {s + "attn"});
     { PhaseDesc d = mk(TK_LN_FWD, rows16); d.p[0] = ln2[l]; d.p[1] = mean2[l]; d.p[2] = rstd2[l]; d.p[3] = hb[l]; d.p[4] = Wact + lay.g2[l];
@@ -476,7 +518,7 @@ bool build_train_graph(ofa_ctx* c) {
     PhaseDesc d = mk(TK_GEMM, 0); d.layout = GL_NT; d.epi = fuse_head ? GE_LSE : GE_STORE;
     d.g.A = lnf; d.g.B = Wact + lay.head; d.g.C = logits; d.g.aux = nullptr; d.g.M = (int)N; d.g.N = (int)V; d.g.K = (int)D; d.g.lda = (int)D; d.g.ldb = (int)D; d.g.ldc = (int)V;
     d.g.dr = reinterpret_cast<float*>(lse_part);
-    if (bf) { std::string e; if (!prepare_gemm_bf16(d, c->ar, cfg.gemm_nsub, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }
+    if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, cfg.gemm_nsub, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }
     else prepare_gemm_f32(d);
     addp("logits", d, {"lnf"}, {opt_head}, {"lnf"});
   }
@@ -651,7 +693,7 @@ bool build_train_graph(ofa_ctx* c) {
       addb(s + "dWo", mkgemm(GL_TN, wepi, att[l], D, dh[l], D, G(lay.wo[l]), D, nullptr, 0, D, D, N, 0), {s + "ln2 bwd"}, {});
       if (!bf) { PhaseDesc d = mk(TK_ATT_PREP, 1); d.p[0] = att[l]; d.p[1] = dob[l]; d.p[2] = Dr[l]; addb(s + "attn prep", d, {s + "dO"}, {}); }
       { PhaseDesc d = mk(TK_ATT_BWD, attn_bwd_tasks); d.p[0] = qkv[l]; d.p[1] = dob[l]; d.p[2] = lse[l]; d.p[3] = Dr[l]; d.p[4] = dqkv[l]; d.p[5] = att[l];
-        if (bf) { std::string e; d.p[6] = const_cast<void*>(make_attn_maps(c->ar, qkv[l], dob[l], N, D, e)); if (!d.p[6]) { ok = false; err = e; } }
+        if (bf) { std::string e; d.p[6] = const_cast<void*>(make_attn_maps(sink, qkv[l], dob[l], N, D, e)); if (!d.p[6]) { ok = false; err = e; } }
         addb(s + "attn bwd", d, {bf ? s + "dO" : s + "attn prep"}, {}, {s + "dO"}); }
       addb(s + "dln1", mkgemm(GL_NT, GE_STORE, dqkv[l], 3 * D, Wact + lay.wqkv[l], 3 * D, dln1[l], D, nullptr, 0, N, D, 3 * D, 0), {s + "attn bwd"}, {}, {s + "attn bwd"});
       addb(s + "dWqkv", mkgemm(GL_TN, wepi, ln1[l], D, dqkv[l], 3 * D, G(lay.wqkv[l]), 3 * D, nullptr, 0, D, 3 * D, N, 0), {s + "attn bwd"}, {});
@@ -741,11 +783,9 @@ bool build_decode_graph(ofa_ctx* c) {
   st.xw = c->ar.alloc<unsigned long long>(D); st.xr = c->ar.alloc<unsigned long long>(D);
   st.q = c->ar.alloc<T>(D);
   st.cand_v = c->ar.alloc<float>(2 * nchunk); st.cand_i = c->ar.alloc<int>(2 * nchunk);
-  c->d_scal = c->ar.alloc<int>(8); st.scal = c->d_scal;
   st.kv = c->ar.alloc<T>((size_t)L * 2 * m.H * m.T * m.DH);
   st.logits = c->ar.alloc<float>(m.V);
   c->bufs["dec_kv"] = std::make_pair((void*)st.kv, (size_t)L * 2 * m.H * m.T * m.DH * sizeof(T));   // [L][2][H][T][DH], for parity checks
-  c->bufs["dec_scal"] = std::make_pair((void*)c->d_scal, sizeof(int) * 8);                               // token, pos, step, ctx_full, astep, poskey, epoch
   c->out_cap = cfg.decode_out_cap > 0 ? cfg.decode_out_cap : 65536;
   if (c->ar.dry) { c->d_out = c->ar.alloc<int>(c->out_cap); }
   else {
@@ -760,8 +800,6 @@ bool build_decode_graph(ofa_ctx* c) {
   c->ar.h2d(c->d_forced, cfg.prompt, sizeof(int) * cfg.n_prompt);
   dp.forced = c->d_forced; dp.nforced = cfg.n_prompt; dp.answer_len = cfg.answer_len; dp.auto_reset = 1;
   dp.temperature = cfg.temperature; dp.seed = cfg.decode_seed;
-  int scal[8] = {cfg.prompt[0], 0, 0, 0, 0, 0, 0, 0};
-  c->ar.h2d(c->d_scal, scal, sizeof scal);
 
   std::vector<HostPhase>& P = c->dec_ph; P.clear();
   auto mk = [&](const std::string& name, int kind, int ntasks, int layer) {
@@ -783,6 +821,42 @@ bool build_decode_graph(ofa_ctx* c) {
   return true;
 }
 
+// Device memory of the two jobs: tables, the decoder's scalars, then everything a launch starts from zero (device status, finished
+// and arrival words, both jobs' counters) so that one fill prepares a launch. Called once at creation, and again (same sizes) when
+// the test hook for the task order changed.
+bool place_jobs(ofa_ctx* c) {
+  const bool train = !c->train_ph.empty(), dec = c->cfg.use_decode != 0;
+  if (train && !make_job(c->train_ph, c->train_last, c->train_job, c->err, (c->bf && c->md.N % 128 == 0) ? c->md.N / 128 : 0)) return false;
+  if (dec && !make_job(c->dec_ph, c->dec_last, c->dec_job, c->err)) return false;
+  c->jobs_seed = g_task_shuffle_seed;
+  const size_t tt = train ? job_table_bytes(c->train_job) : 0, td = dec ? job_table_bytes(c->dec_job) : 0;
+  const size_t ct = train ? job_counter_bytes(c->train_job) : 0, cd = dec ? job_counter_bytes(c->dec_job) : 0;
+  const size_t tab = tt + td;
+  if (!c->d_jobs) {
+    c->d_jobs = c->ar.alloc<unsigned char>(tab + 192 + ct + cd);
+    if (!c->d_jobs) { c->err = "out of device memory (job tables)"; return false; }
+    unsigned char* p = c->d_jobs + tab;
+    c->d_scal = reinterpret_cast<int*>(p); c->d_status = reinterpret_cast<DevStatus*>(p + 64); c->d_finished = reinterpret_cast<int*>(p + 128);
+    c->jobs_cnt_off = tab + 64; c->jobs_cnt_bytes = 128 + ct + cd;
+    if (dec) {
+      c->C.dp.st.scal = c->d_scal;
+      c->bufs["dec_scal"] = std::make_pair((void*)c->d_scal, sizeof(int) * 8);                             // token, pos, step, ctx_full, astep, poskey, epoch
+      const int scal[8] = {c->cfg.prompt[0], 0, 0, 0, 0, 0, 0, 0};
+      c->ar.h2d(c->d_scal, scal, sizeof scal);
+    }
+  }
+  Ctx& C = c->C;
+  std::vector<unsigned char> img(tab);
+  unsigned char* cnt = c->d_jobs + tab + 192;
+  if (train) C.train = place_job(c->train_job, 0, img.data(), c->d_jobs, cnt);
+  if (dec) C.dec = place_job(c->dec_job, 0, img.data() + tt, c->d_jobs + tt, cnt + ct);
+  c->ar.h2d(c->d_jobs, img.data(), tab);
+  fill_param_records(C, train ? &c->train_job : nullptr, dec ? &c->dec_job : nullptr);
+  C.use_train = train ? 1 : 0;
+  C.status = c->d_status; C.finished = c->d_finished; C.arrived = c->d_finished + 1;
+  return true;
+}
+
 bool probe_smids(ofa_ctx* c) {
   unsigned* seen = c->ar.alloc<unsigned>(64);
   if (!seen) return false;
@@ -790,7 +864,7 @@ bool probe_smids(ofa_ctx* c) {
   cudaFuncSetAttribute(smid_probe_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   smid_probe_kernel<<<c->nblocks, NTHR, c->smem, c->stream>>>(seen);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return false;
-  unsigned h[64]; cudaMemcpy(h, seen, sizeof h, cudaMemcpyDeviceToHost);
+  unsigned h[64]; if (cudaMemcpy(h, seen, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
   std::vector<int> rank(2048, -1); int n = 0; bool dense = true;
   for (int i = 0; i < 2048; i++) if (h[i >> 5] >> (i & 31) & 1u) { if (i != n) dense = false; rank[i] = n++; }
   if (n == 0) return false;
@@ -798,7 +872,7 @@ bool probe_smids(ofa_ctx* c) {
     for (int i = 0; i < 2048; i++) if (rank[i] < 0) rank[i] = 1 << 20;   // unknown SM: idle
     c->d_smid_rank = c->ar.alloc<int>(2048);
     if (!c->d_smid_rank) return false;
-    cudaMemcpy(c->d_smid_rank, rank.data(), 2048 * sizeof(int), cudaMemcpyHostToDevice);
+    c->ar.h2d(c->d_smid_rank, rank.data(), 2048 * sizeof(int));
   }
   return true;
 }
@@ -860,19 +934,20 @@ extern "C" void ofa_destroy(ofa_ctx* c) {
     // never block forever: ask the kernel to drain, give it a few seconds, and otherwise leak the device memory it may still use
     ofa_abort(c);
     bool done = false;
-    for (int i = 0; i < 25000 && !done; i++) { done = cudaEventQuery(c->ev1) != cudaErrorNotReady; if (!done) { if (i % 64 == 63) post_abort(c); struct timespec sl = {0, 200000}; nanosleep(&sl, nullptr); } }
+    for (int i = 0; i < 25000 && !done; i++) { done = cudaEventQuery(c->ev2) != cudaErrorNotReady; if (!done) { if (i % 64 == 63) post_abort(c); struct timespec sl = {0, 200000}; nanosleep(&sl, nullptr); } }
     if (!done) { delete c; return; }
   }
   ofa_dp_shutdown(c);
-  c->train_job.free_all(); c->dec_job.free_all();
   if (c->d_step_done) cudaFree(c->d_step_done);
   if (c->d_tokens) cudaFree(c->d_tokens);
   if (c->d_starts) cudaFree(c->d_starts);
   c->ar.free_all();
   if (c->h_live) cudaFreeHost(c->h_live);
   if (c->h_out) cudaFreeHost(c->h_out);
+  if (c->h_back) cudaFreeHost(c->h_back);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->ev2) cudaEventDestroy(c->ev2);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->abort_stream) cudaStreamDestroy(c->abort_stream);
   delete c;
@@ -924,7 +999,8 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   }
   if (!dry) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(OFA_CUDA_ERROR, "stream");
-    cudaEventCreate(&c->ev0); cudaEventCreate(&c->ev1);
+    cudaEventCreate(&c->ev0); cudaEventCreate(&c->ev1); cudaEventCreateWithFlags(&c->ev2, cudaEventDisableTiming);
+    c->ar.stream = c->stream;
   }
   // SM split
   int infer = cfg->use_decode ? std::max(0, cfg->infer_sms) : 0, resv = std::max(0, cfg->reserved_sms);
@@ -940,11 +1016,12 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   c->W32 = c->ar.alloc<float>(NP); c->M32 = c->ar.alloc<float>(NP); c->V32 = c->ar.alloc<float>(NP);
   c->Wact = c->bf ? (void*)c->ar.alloc<bf16>(NP) : (void*)c->ar.alloc<float>(NP);
   if (cfg->grad_bf16) c->Gbf = c->ar.alloc<bf16>(NP); else c->G32 = c->ar.alloc<float>(NP);
-  c->d_status = c->ar.alloc<DevStatus>(1); c->d_finished = c->ar.alloc<int>(2); c->d_t_end = c->ar.alloc<unsigned long long>(1);
+  c->d_t_end = c->ar.alloc<unsigned long long>(1);
   if (!c->ar.ok) return bail(OFA_CUDA_ERROR, "out of device memory (parameters)");
   if (!dry) {
     if (cudaHostAlloc(&c->h_live, sizeof(Live), cudaHostAllocMapped) != cudaSuccess) return bail(OFA_CUDA_ERROR, "cudaHostAlloc failed");
     memset(c->h_live, 0, sizeof(Live)); cudaHostGetDevicePointer(&c->d_live, c->h_live, 0);
+    if (cudaHostAlloc(&c->h_back, 128, cudaHostAllocDefault) != cudaSuccess) return bail(OFA_CUDA_ERROR, "cudaHostAlloc failed");
   }
   c->d_ext_ready = c->ar.alloc<int>(64); c->d_ext_done = c->d_ext_ready ? c->d_ext_ready + 32 : nullptr;
   if (!c->ar.ok) return bail(OFA_CUDA_ERROR, "out of device memory");
@@ -957,7 +1034,7 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   C.hp.warmup = cfg->warmup; C.hp.sched_steps = std::max(cfg->sched_steps, cfg->warmup + 1); C.hp.constant_lr = cfg->constant_lr; C.hp.grad_scale = 1.0f / (float)cfg->dp_world;
   C.seed = cfg->data_seed;
   C.infer_sms = infer; C.reserved_sms = resv; C.train_sms = train; C.use_decode = cfg->use_decode ? 1 : 0; C.use_train = 1;
-  C.smid_rank = c->d_smid_rank; C.live = c->d_live; C.status = c->d_status; C.finished = c->d_finished; C.t_end = c->d_t_end;
+  C.smid_rank = c->d_smid_rank; C.live = c->d_live; C.t_end = c->d_t_end;
   C.dep_timeout_ns = (unsigned long long)((cfg->timeout_s > 0 ? cfg->timeout_s : 20.0) * 1e9);
   C.prof_step = -1;
   bool ok = decode_only ? true : (c->bf ? build_train_graph<bf16>(c) : build_train_graph<float>(c));
@@ -973,6 +1050,16 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   c->d_dec_phase_busy = c->ar.alloc<unsigned long long>(std::max<size_t>(1, c->dec_ph.size()));
   c->d_blk_info = c->ar.alloc<int>(c->nblocks); C.blk_info = c->d_blk_info;
   C.phase_busy = c->d_phase_busy; C.phase_first = c->d_phase_first; C.phase_last = c->d_phase_last; C.blk_busy = c->d_blk_busy; C.blk_wait = c->d_blk_busy + 2 * c->nblocks; C.dec_phase_busy = c->d_dec_phase_busy;
+  if (!place_jobs(c)) return bail(OFA_BAD_CONFIG, c->err);
+  C.smem_bytes = c->smem;
+  if (!dry && train > 0) {
+    c->loss_cap = 4096; c->d_loss_hist = c->ar.alloc<float>(c->loss_cap);
+    if (!c->d_loss_hist) return bail(OFA_CUDA_ERROR, "out of device memory");
+  }
+  if (!dry) {
+    cudaMemsetAsync(c->d_phase_first, 0xFF, sizeof(unsigned long long) * nph, c->stream);
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return bail(OFA_CUDA_ERROR, cudaGetErrorString(cudaGetLastError()));   // whatever reads or writes the buffers next, on any stream, finds them filled
+  }
   *out = c;
   return OFA_OK;
 }
@@ -1029,7 +1116,8 @@ extern "C" int ofa_load_adam_state(ofa_ctx* c, const float* mm, const float* vv,
   if (!c || !mm || !vv || n != c->lay.total || step_base < 0) return fail(c, OFA_BAD_ARGUMENT, "bad optimizer state");
   if (c->in_flight) return fail(c, OFA_BAD_ARGUMENT, "launch in flight");
   cudaSetDevice(c->device);
-  if (cudaMemcpy(c->M32, mm, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess || cudaMemcpy(c->V32, vv, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (cudaMemcpyAsync(c->M32, mm, n * sizeof(float), cudaMemcpyHostToDevice, c->stream) != cudaSuccess || cudaMemcpyAsync(c->V32, vv, n * sizeof(float), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+      cudaStreamSynchronize(c->stream) != cudaSuccess)
     return fail(c, OFA_CUDA_ERROR, std::string("H2D failed: ") + cudaGetErrorString(cudaGetLastError()));
   c->steps_total = step_base;
   return OFA_OK;
@@ -1049,7 +1137,7 @@ extern "C" int ofa_set_tokens(ofa_ctx* c, const uint32_t* tokens, size_t n) {
   }
   c->ntok = n;
   c->nstarts = 0;                                   // a starts table was validated against the old stream: it has to be set again
-  return cudaMemcpy(c->d_tokens, tokens, n * 4, cudaMemcpyHostToDevice) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
+  return cudaMemcpyAsync(c->d_tokens, tokens, n * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
 }
 extern "C" int ofa_set_starts(ofa_ctx* c, const uint32_t* starts, size_t nsteps) {
   if (!c) return OFA_BAD_ARGUMENT;
@@ -1066,7 +1154,7 @@ extern "C" int ofa_set_starts(ofa_ctx* c, const uint32_t* starts, size_t nsteps)
     c->starts_cap = n;
   }
   c->nstarts = (int)nsteps;
-  return cudaMemcpy(c->d_starts, starts, n * 4, cudaMemcpyHostToDevice) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
+  return cudaMemcpyAsync(c->d_starts, starts, n * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
 }
 
 extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
@@ -1076,14 +1164,15 @@ extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
   const bool train_on = c->C.train_sms > 0;
   if (train_on && (!c->d_tokens || c->ntok < (size_t)c->md.T + 2)) return fail(c, OFA_BAD_ARGUMENT, "no tokens set");
   cudaSetDevice(c->device);
-  std::string err;
+  if (c->jobs_seed != g_task_shuffle_seed && !place_jobs(c)) return fail(c, OFA_BAD_CONFIG, c->err);
+  Ctx& C = c->C;
   if (train_on) {
-    if (!upload_job(c->train_ph, c->train_last, nsteps, c->train_job, err, (c->bf && c->md.N % 128 == 0) ? c->md.N / 128 : 0)) return fail(c, OFA_BAD_CONFIG, err);
+    if (!tickets_fit(c->train_job, nsteps, c->err)) return OFA_BAD_CONFIG;
     if (c->steps_total + nsteps > c->loss_cap) {
       const int cap = std::max(4096, 2 * (c->steps_total + nsteps));
       float* nl = c->ar.alloc<float>(cap);
       if (!nl) return fail(c, OFA_CUDA_ERROR, "out of device memory");
-      if (c->d_loss_hist) cudaMemcpy(nl, c->d_loss_hist, sizeof(float) * c->loss_cap, cudaMemcpyDeviceToDevice);
+      if (c->d_loss_hist) cudaMemcpyAsync(nl, c->d_loss_hist, sizeof(float) * c->loss_cap, cudaMemcpyDeviceToDevice, c->stream);
       c->d_loss_hist = nl; c->loss_cap = cap;
     }
     if (nsteps > c->step_done_cap) {               // grown, never re-allocated per launch: a loop of short launches must not leak
@@ -1093,44 +1182,41 @@ extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
       if (cudaMalloc(&c->d_step_done, sizeof(unsigned long long) * cap) != cudaSuccess) return fail(c, OFA_CUDA_ERROR, "out of device memory");
       c->step_done_cap = cap;
     }
+    C.train.nsteps = nsteps;
+    C.data = c->d_tokens; C.ntok = c->ntok; C.starts = c->nstarts > 0 ? c->d_starts : nullptr; C.nstarts = c->nstarts;
+    C.loss_hist = c->d_loss_hist + c->steps_total;    // history, LR schedule and data windows continue across launches
+    C.step_done = c->d_step_done;
   }
   if (c->cfg.use_decode) {
-    const int dsteps = train_on ? (1 << 20) : nsteps;
-    if (!upload_job(c->dec_ph, c->dec_last, dsteps, c->dec_job, err)) return fail(c, OFA_BAD_CONFIG, err);
+    C.dec.nsteps = train_on ? (1 << 20) : nsteps;
+    if (!tickets_fit(c->dec_job, C.dec.nsteps, c->err)) return OFA_BAD_CONFIG;
   }
-  Ctx C = c->C;
-  C.use_train = train_on ? 1 : 0;
-  if (train_on) C.train = c->train_job.j;
-  if (c->cfg.use_decode) C.dec = c->dec_job.j;
-  fill_param_records(C, train_on ? &c->train_job : nullptr, c->cfg.use_decode ? &c->dec_job : nullptr);
   if (c->cfg.sched_profile) C.sched_flags |= 2;
-  C.data = c->d_tokens; C.ntok = c->ntok; C.starts = c->nstarts > 0 ? c->d_starts : nullptr; C.nstarts = c->nstarts;
-  C.loss_hist = c->d_loss_hist ? c->d_loss_hist + c->steps_total : nullptr;   // history, LR schedule and data windows continue across launches
-  C.step_done = c->d_step_done;
   C.step_base = c->steps_total;
+  C.prof_step = nsteps - 1;       // wall-clock window of every phase in the last step of this launch (the reference's "phase wall-clock at step" table, ofa.cu:735-743)
   c->abort_requested = false;
-  cudaMemsetAsync(c->d_status, 0, sizeof(DevStatus), c->stream);
-  cudaMemsetAsync(c->d_finished, 0, 2 * sizeof(int), c->stream);
+  cudaMemsetAsync(c->d_jobs + c->jobs_cnt_off, 0, c->jobs_cnt_bytes, c->stream);
   if (c->cfg.use_decode) {
     // The serving blocks of the previous launch left when training finished, normally in the middle of a token: the residual then
     // holds the contributions of some layers. The token is decoded again from layer 0 (the serving job's counters restart), so the
     // residual is rebuilt from the token and position the last completed sample step stored; K/V rows, q and candidates are rewritten.
-    if (c->bf) decode_init_embed_kernel<bf16, 768><<<1, NTHR, 0, c->stream>>>(c->C.dp); else decode_init_embed_kernel<float, 64><<<1, NTHR, 0, c->stream>>>(c->C.dp);
+    if (c->bf) decode_init_embed_kernel<bf16, 768><<<1, NTHR, 0, c->stream>>>(C.dp); else decode_init_embed_kernel<float, 64><<<1, NTHR, 0, c->stream>>>(C.dp);
   }
-  C.arrived = c->d_finished + 1;
-  cudaMemsetAsync(c->d_phase_busy, 0, sizeof(unsigned long long) * 2 * std::max<size_t>(1, c->train_ph.size()), c->stream);
-  cudaMemsetAsync(c->d_blk_busy, 0, sizeof(unsigned long long) * 6 * c->nblocks, c->stream);
-  cudaMemsetAsync(c->d_dec_phase_busy, 0, sizeof(unsigned long long) * std::max<size_t>(1, c->dec_ph.size()), c->stream);
-  C.smem_bytes = c->smem;
-  // wall-clock window of every phase in the last step of this launch (the reference's "phase wall-clock at step" table, ofa.cu:735-743)
-  C.prof_step = nsteps - 1;
-  cudaMemsetAsync(c->d_phase_first, 0xFF, sizeof(unsigned long long) * std::max<size_t>(1, c->train_ph.size()), c->stream);
-  cudaMemsetAsync(c->d_phase_last, 0, sizeof(unsigned long long) * std::max<size_t>(1, c->train_ph.size()), c->stream);
-  const Ctx& L = C;
+  if (c->cfg.sched_profile) {     // the tables are only written then
+    const size_t nph = std::max<size_t>(1, c->train_ph.size());
+    cudaMemsetAsync(c->d_phase_busy, 0, sizeof(unsigned long long) * 2 * nph, c->stream);
+    cudaMemsetAsync(c->d_blk_busy, 0, sizeof(unsigned long long) * 6 * c->nblocks, c->stream);
+    cudaMemsetAsync(c->d_dec_phase_busy, 0, sizeof(unsigned long long) * std::max<size_t>(1, c->dec_ph.size()), c->stream);
+    cudaMemsetAsync(c->d_phase_first, 0xFF, sizeof(unsigned long long) * nph, c->stream);
+    cudaMemsetAsync(c->d_phase_last, 0, sizeof(unsigned long long) * nph, c->stream);
+  }
   cudaEventRecord(c->ev0, c->stream);
-  cudaError_t e = c->bf ? launch_kernel<bf16, 768, 64>(L, c->nblocks, c->smem, c->stream) : launch_kernel<float, 64, 16>(L, c->nblocks, c->smem, c->stream);
+  cudaError_t e = c->bf ? launch_kernel<bf16, 768, 64>(C, c->nblocks, c->smem, c->device, c->stream) : launch_kernel<float, 64, 16>(C, c->nblocks, c->smem, c->device, c->stream);
   cudaEventRecord(c->ev1, c->stream);
   if (e != cudaSuccess) return fail(c, OFA_CUDA_ERROR, std::string("kernel launch failed: ") + cudaGetErrorString(e));
+  // what ofa_wait looks at comes back behind the kernel: the decoder's scalars and the device status, 128 adjacent bytes
+  cudaMemcpyAsync(c->h_back, c->d_scal, 128, cudaMemcpyDeviceToHost, c->stream);
+  cudaEventRecord(c->ev2, c->stream);
   c->in_flight = true; c->last_nsteps = nsteps;
   return OFA_OK;
 }
@@ -1143,20 +1229,22 @@ extern "C" int ofa_wait(ofa_ctx* c, int timeout_ms, ofa_status_t* status) {
   struct timespec ts0; clock_gettime(CLOCK_MONOTONIC, &ts0);
   unsigned polls = 0;
   for (;;) {
-    cudaError_t q = cudaEventQuery(c->ev1);
+    cudaError_t q = cudaEventQuery(c->ev2);
     if (q == cudaSuccess) break;
     if (q != cudaErrorNotReady) { c->in_flight = false; if (status) status->code = OFA_CUDA_ERROR; return fail(c, OFA_CUDA_ERROR, std::string("device error: ") + cudaGetErrorString(q)); }
     struct timespec ts; clock_gettime(CLOCK_MONOTONIC, &ts);
     const double ms = (ts.tv_sec - ts0.tv_sec) * 1e3 + (ts.tv_nsec - ts0.tv_nsec) * 1e-6;
     if (timeout_ms >= 0 && ms > timeout_ms) { if (status) status->code = OFA_TIMEOUT; return OFA_TIMEOUT; }
     // an abort requested before the launch's own set-up ran may have been cleared by it: keep posting it while the launch lives
-    if (c->abort_requested && (++polls % 64) == 0) post_abort(c);
-    struct timespec sl = {0, 200000}; nanosleep(&sl, nullptr);
+    if (c->abort_requested && (++polls % (ms > 2.0 ? 64 : 65536)) == 0) post_abort(c);
+    // a short launch is polled without a pause (a sleep of 200 us used to cost up to that much on every launch); a longer one is
+    // polled at about a hundredth of the time it has taken so far, at most every 200 us
+    if (ms > 2.0) { struct timespec sl = {0, (long)std::min(200000.0, ms * 1e4)}; nanosleep(&sl, nullptr); }
   }
   c->in_flight = false;
   cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);
-  DevStatus ds; cudaMemcpy(&ds, c->d_status, sizeof ds, cudaMemcpyDeviceToHost);
-  if (c->cfg.use_decode) { int scal[8]; cudaMemcpy(scal, c->d_scal, sizeof scal, cudaMemcpyDeviceToHost); c->dec_steps_total = scal[DS_STEP]; }
+  DevStatus ds; memcpy(&ds, c->h_back + 64, sizeof ds);
+  if (c->cfg.use_decode) c->dec_steps_total = reinterpret_cast<const int*>(c->h_back)[DS_STEP];
   if (ds.code != 0 || ds.abort != 0) {
     if (status) { status->code = OFA_DEVICE_ABORT; status->dev_code = ds.code; status->phase = ds.phase; status->task = ds.task; status->block = ds.block; status->aux = ds.aux; }
     std::string nm = (ds.phase >= 0 && ds.phase < (int)c->train_ph.size()) ? c->train_ph[ds.phase].name : "?";
@@ -1288,6 +1376,61 @@ extern "C" int ofa_dev_free(void* p) { return cudaFree(p) == cudaSuccess ? OFA_O
 extern "C" int ofa_h2d(void* dst, const void* src, size_t bytes) { return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? OFA_OK : OFA_CUDA_ERROR; }
 extern "C" int ofa_d2h(void* dst, const void* src, size_t bytes) { return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost) == cudaSuccess ? OFA_OK : OFA_CUDA_ERROR; }
 
+namespace {
+
+// Memory and events of one ofa_run_phases call, kept between calls: allocating and freeing them on each call (some twenty
+// cudaMalloc / cudaFree, every one a device-wide wait, and a query of all device properties) cost 3 ms beside a kernel of 0.1 to
+// 1 ms. A call takes a workspace of its device from the pool or makes one, and hands it back when its kernel has finished, so
+// threads and streams never share one. The pool keeps at most four, none above 4 MB; the rest are freed.
+struct Workspace {
+  int device = -1;
+  unsigned char *dev = nullptr, *host = nullptr, *rep = nullptr, *back = nullptr;   // tables on the device, their pinned image, per-repeat words on the device, pinned status
+  size_t bytes = 0, rep_bytes = 0;
+  cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
+  bool make(int d, size_t n, size_t nrep) {
+    device = d; bytes = up64(std::max<size_t>(n, 64 << 10)); rep_bytes = std::max<size_t>(nrep, 4096);
+    return cudaMalloc(&dev, bytes) == cudaSuccess && cudaMalloc(&rep, rep_bytes) == cudaSuccess && cudaHostAlloc(&host, bytes, cudaHostAllocDefault) == cudaSuccess &&
+           cudaHostAlloc(&back, 64, cudaHostAllocDefault) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess &&
+           cudaEventCreateWithFlags(&e2, cudaEventDisableTiming) == cudaSuccess;
+  }
+  ~Workspace() {
+    if (dev) cudaFree(dev);
+    if (rep) cudaFree(rep);
+    if (host) cudaFreeHost(host);
+    if (back) cudaFreeHost(back);
+    for (cudaEvent_t e : {e0, e1, e2}) if (e) cudaEventDestroy(e);
+  }
+};
+struct WorkspacePool {
+  std::mutex mu; std::vector<Workspace*> idle;
+  ~WorkspacePool() { for (Workspace* w : idle) delete w; }
+};
+WorkspacePool g_workspaces;
+struct WorkspaceLease {
+  Workspace* w = nullptr;
+  WorkspaceLease(int dev, size_t bytes, size_t rep_bytes) {
+    {
+      std::lock_guard<std::mutex> lk(g_workspaces.mu);
+      for (size_t i = 0; i < g_workspaces.idle.size() && !w; i++) {
+        Workspace* c = g_workspaces.idle[i];
+        if (c->device == dev && c->bytes >= bytes && c->rep_bytes >= rep_bytes) { w = c; g_workspaces.idle.erase(g_workspaces.idle.begin() + i); }
+      }
+    }
+    if (!w) { w = new Workspace(); if (!w->make(dev, bytes, rep_bytes)) { cudaGetLastError(); delete w; w = nullptr; } }
+  }
+  ~WorkspaceLease() {
+    if (!w) return;
+    if (w->bytes + w->rep_bytes <= (4u << 20)) {
+      std::lock_guard<std::mutex> lk(g_workspaces.mu);
+      if (g_workspaces.idle.size() < 4) { g_workspaces.idle.push_back(w); return; }
+    }
+    delete w;
+  }
+  WorkspaceLease(const WorkspaceLease&) = delete; WorkspaceLease& operator=(const WorkspaceLease&) = delete;
+};
+
+}  // namespace
+
 extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* phases, int nph, int repeats, const float* adam,
                               float* ms, ofa_status_t* status) {
   if (status) memset(status, 0, sizeof *status);
@@ -1305,11 +1448,20 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
     const std::string e = smem_fit_error(bf, m.T, m.N, emb, false, smem);
     if (!e.empty()) return fail(nullptr, OFA_BAD_CONFIG, e);
   }
-  int dev = 0; cudaDeviceProp prop;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return fail(nullptr, OFA_CUDA_ERROR, "no CUDA device");
-  if (prop.major != 10) return fail(nullptr, OFA_CUDA_ERROR, "sm_100a code only");
-  const int nblocks = 2 * prop.multiProcessorCount;
-  Arena ar; DevJob dj; std::string err;
+  int dev = 0, major = 0, num_sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return fail(nullptr, OFA_CUDA_ERROR, "no CUDA device");
+  if (major != 10) return fail(nullptr, OFA_CUDA_ERROR, "sm_100a code only");
+  const int nblocks = 2 * num_sms;
+  std::string err;
+  // upper bound of the call's tables, to size the workspace before the phases are prepared: descriptors, records, one dependency
+  // per phase (two for the first), at most four TMA descriptors per phase, counters, and what the kernel reports per repeat
+  const size_t map_cap = (size_t)nph * sizeof(attn_tc::Maps), tab_cap = (size_t)nph * (sizeof(PhaseDesc) + sizeof(SchedRec) + 24 + sizeof(Dep)) + 1024;
+  const size_t rep_bytes = up64(sizeof(unsigned long long) * (size_t)repeats) + up64(sizeof(float) * (size_t)repeats);
+  const size_t cnt_cap = 64 + up64(4 * (size_t)nph) + 64;
+  WorkspaceLease ws(dev, map_cap + tab_cap + 192 + cnt_cap, rep_bytes);
+  if (!ws.w) return fail(nullptr, OFA_CUDA_ERROR, "out of memory (workspace)");
+  MapSink sink; sink.host = ws.w->host; sink.dev = ws.w->dev; sink.cap = map_cap;
   std::vector<HostPhase> P(nph);
   for (int i = 0; i < nph; i++) {
     const ofa_phase& s = phases[i];
@@ -1323,71 +1475,74 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
         d.g.A = s.p[0]; d.g.B = s.p[1]; d.g.C = s.p[2]; d.g.aux = s.p[3]; d.g.M = s.M; d.g.N = s.N; d.g.K = s.K; d.g.lda = s.lda; d.g.ldb = s.ldb; d.g.ldc = s.ldc; d.g.ldaux = s.ldaux;
         d.g.accumulate = s.accumulate;
         if (s.epi == GE_LSE) {  // p[4] = softmax partials [M, N / 128] float2
-          if (!bf || !s.p[4] || s.layout != GL_NT) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "softmax-partial epilogue: bf16, NT layout, p[4] = output [M, N/128] float2"); }
+          if (!bf || !s.p[4] || s.layout != GL_NT) { return fail(nullptr, OFA_BAD_ARGUMENT, "softmax-partial epilogue: bf16, NT layout, p[4] = output [M, N/128] float2"); }
           d.g.dr = reinterpret_cast<float*>(s.p[4]);
         }
         if (s.epi == GE_DR) {   // p[4] = row-term output [B, H, T]; needs the tensor-core path, heads of 64 columns and whole rows of heads in C
-          if (!bf || !s.p[4] || s.layout != GL_NT || s.N != m.D || s.M != m.N) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "row-term epilogue: bf16, NT layout, C = [tokens, d_model], p[4] = output"); }
+          if (!bf || !s.p[4] || s.layout != GL_NT || s.N != m.D || s.M != m.N) { return fail(nullptr, OFA_BAD_ARGUMENT, "row-term epilogue: bf16, NT layout, C = [tokens, d_model], p[4] = output"); }
           d.g.dr = reinterpret_cast<float*>(s.p[4]); d.g.dr_T = m.T; d.g.dr_H = m.H;
         }
-        if (bf) { if (!prepare_gemm_bf16(d, ar, s.nsub, nblocks, err)) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, err); } }
+        if (bf) { if (!prepare_gemm_bf16(d, sink, s.nsub, nblocks, err)) { return fail(nullptr, OFA_BAD_ARGUMENT, err); } }
         else prepare_gemm_f32(d);
         break;
       case TK_EMBED: case TK_LN_FWD: case TK_LN_BWD: d.ntasks = rows16; break;
       case TK_LN_DG: d.ntasks = (m.D + NTHR - 1) / NTHR; break;
       case TK_ATT_FWD: d.ntasks = bf ? BH * (m.T / attn::QTILE) : BH;
-        if (bf) { d.p[6] = const_cast<void*>(make_attn_maps(ar, s.p[0], nullptr, m.N, m.D, err)); if (!d.p[6]) { ar.free_all(); return fail(nullptr, OFA_CUDA_ERROR, err); } }
+        if (bf) { d.p[6] = const_cast<void*>(make_attn_maps(sink, s.p[0], nullptr, m.N, m.D, err)); if (!d.p[6]) { return fail(nullptr, OFA_CUDA_ERROR, err); } }
         break;
       case TK_ATT_PREP: d.ntasks = bf ? BH * (m.T / attn::QTILE) : 1; break;
       case TK_ATT_BWD: d.ntasks = bf ? 2 * BH * (m.T / attn::QTILE) : BH;
-        if (bf) { d.p[6] = const_cast<void*>(make_attn_maps(ar, s.p[0], s.p[1], m.N, m.D, err)); if (!d.p[6]) { ar.free_all(); return fail(nullptr, OFA_CUDA_ERROR, err); } }
+        if (bf) { d.p[6] = const_cast<void*>(make_attn_maps(sink, s.p[0], s.p[1], m.N, m.D, err)); if (!d.p[6]) { return fail(nullptr, OFA_CUDA_ERROR, err); } }
         break;
       case TK_CE: d.ntasks = (m.N + ew::CE_ROWS - 1) / ew::CE_ROWS;
-        if (s.p[3]) { if (!bf || m.V % 128) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "cross-entropy with softmax partials: bf16, vocab a multiple of 128"); } d.i2 = m.V / 128; }
+        if (s.p[3]) { if (!bf || m.V % 128) { return fail(nullptr, OFA_BAD_ARGUMENT, "cross-entropy with softmax partials: bf16, vocab a multiple of 128"); } d.i2 = m.V / 128; }
         d.i0 = (int)(std::min<size_t>((size_t)((bf ? gemm_tc::BAR_OFFSET : smem - CTRL_BYTES) - 64), (size_t)m.V * (bf ? 2 : 4)) / 16 * 16); break;
       case TK_CE_MEAN: d.ntasks = 1; break;
       case TK_BARRIER: d.ntasks = s.n > 0 ? (int)std::min<size_t>(s.n, 1u << 24) : 1; break;     // n empty tasks: what a task costs the scheduler alone
       case TK_EMB_WTE: d.ntasks = (m.V + ew::EMB_VCHUNK - 1) / ew::EMB_VCHUNK; break;
       case TK_EMB_WPE: d.ntasks = (m.T + ew::WPE_ROWS - 1) / ew::WPE_ROWS; break;
-      case TK_ADAMW: d.ntasks = (int)((s.n + ew::OPT_CHUNK - 1) / ew::OPT_CHUNK); if (s.n == 0 || s.n % 4) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "AdamW n must be a positive multiple of 4"); } break;
-      default: ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "task kind not available at task level");
+      case TK_ADAMW: d.ntasks = (int)((s.n + ew::OPT_CHUNK - 1) / ew::OPT_CHUNK); if (s.n == 0 || s.n % 4) { return fail(nullptr, OFA_BAD_ARGUMENT, "AdamW n must be a positive multiple of 4"); } break;
+      default: return fail(nullptr, OFA_BAD_ARGUMENT, "task kind not available at task level");
     }
-    if (bf && (s.kind == TK_ATT_FWD || s.kind == TK_ATT_BWD || s.kind == TK_ATT_PREP) && m.T % attn::QTILE) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, "ctx_len must be a multiple of 128"); }
+    if (bf && (s.kind == TK_ATT_FWD || s.kind == TK_ATT_BWD || s.kind == TK_ATT_PREP) && m.T % attn::QTILE) { return fail(nullptr, OFA_BAD_ARGUMENT, "ctx_len must be a multiple of 128"); }
     if (i > 0) hp.deps.push_back(Dep{i - 1, 0});
   }
   P[0].deps.push_back(Dep{nph - 1, -1});
-  if (!upload_job(P, nph - 1, repeats, dj, err)) { ar.free_all(); return fail(nullptr, OFA_BAD_ARGUMENT, err); }
+  HostJob hj;
+  if (!make_job(P, nph - 1, hj, err) || !tickets_fit(hj, repeats, err)) return fail(nullptr, OFA_BAD_ARGUMENT, err);
+  // one image of everything the launch needs: TMA descriptors | tables | status, finished word, end time | counters (zero), uploaded
+  // in one copy behind the caller's earlier work on the default stream
+  const size_t o_tab = map_cap, o_st = o_tab + job_table_bytes(hj), o_cnt = o_st + 192, total = o_cnt + job_counter_bytes(hj);
+  if (total > ws.w->bytes) return fail(nullptr, OFA_CUDA_ERROR, "workspace too small");
+  memset(ws.w->host + o_st, 0, total - o_st);
   static thread_local Ctx C;      // 31 KB: not on the stack
-  memset(&C, 0, sizeof C);
-  C.train = dj.j; C.md = m;
-  fill_param_records(C, &dj, nullptr);
+  memset(&C, 0, offsetof(Ctx, train_rec));
+  C.train = place_job(hj, repeats, ws.w->host + o_tab, ws.w->dev + o_tab, ws.w->dev + o_cnt); C.md = m;
+  fill_param_records(C, &hj, nullptr);
   if (adam) { C.hp.lr_max = adam[0]; C.hp.lr_min = adam[0]; C.hp.beta1 = adam[1]; C.hp.beta2 = adam[2]; C.hp.eps = adam[3]; C.hp.wd = adam[4]; C.hp.grad_scale = adam[5]; C.hp.constant_lr = 1; }
-  C.train_sms = prop.multiProcessorCount; C.use_train = 1;
-  C.status = ar.alloc<DevStatus>(1); C.finished = ar.alloc<int>(1); C.t_end = ar.alloc<unsigned long long>(1);
-  C.step_done = ar.alloc<unsigned long long>(repeats); C.loss_hist = ar.alloc<float>(repeats);
-  C.tok_in = nullptr; C.tok_tgt = nullptr;
+  C.train_sms = num_sms; C.use_train = 1;
+  C.status = reinterpret_cast<DevStatus*>(ws.w->dev + o_st); C.finished = reinterpret_cast<int*>(ws.w->dev + o_st + 64); C.t_end = reinterpret_cast<unsigned long long*>(ws.w->dev + o_st + 128);
+  C.step_done = reinterpret_cast<unsigned long long*>(ws.w->rep); C.loss_hist = reinterpret_cast<float*>(ws.w->rep + up64(sizeof(unsigned long long) * (size_t)repeats));
   C.dep_timeout_ns = 20000000000ull;
   C.smem_bytes = smem;
   C.prof_step = -1;
-  if (!ar.ok) { ar.free_all(); dj.free_all(); return fail(nullptr, OFA_CUDA_ERROR, "out of device memory"); }
-  cudaEvent_t e0, e1; cudaEventCreate(&e0); cudaEventCreate(&e1);
-  cudaEventRecord(e0, 0);
-  cudaError_t e = bf ? launch_kernel<bf16, 768, 64>(C, nblocks, smem, 0) : launch_kernel<float, 64, 16>(C, nblocks, smem, 0);
-  cudaEventRecord(e1, 0);
-  int rc = OFA_OK;
-  if (e != cudaSuccess) { rc = fail(nullptr, OFA_CUDA_ERROR, std::string("launch failed: ") + cudaGetErrorString(e)); }
-  else if ((e = cudaEventSynchronize(e1)) != cudaSuccess) { rc = fail(nullptr, OFA_CUDA_ERROR, std::string("kernel failed: ") + cudaGetErrorString(e)); }
-  else {
-    float t = 0.f; cudaEventElapsedTime(&t, e0, e1); if (ms) *ms = t;
-    DevStatus ds; cudaMemcpy(&ds, C.status, sizeof ds, cudaMemcpyDeviceToHost);
-    if (ds.code || ds.abort) {
-      if (status) { status->code = OFA_DEVICE_ABORT; status->dev_code = ds.code; status->phase = ds.phase; status->task = ds.task; status->block = ds.block; status->aux = ds.aux; }
-      rc = fail(nullptr, OFA_DEVICE_ABORT, "device-side bounded wait expired: code " + std::to_string(ds.code) + " phase " + std::to_string(ds.phase) + " task " + std::to_string(ds.task) + " aux " + std::to_string(ds.aux));
-    }
+  cudaError_t e = cudaMemcpyAsync(ws.w->dev, ws.w->host, total, cudaMemcpyHostToDevice, 0);
+  if (e == cudaSuccess) {
+    cudaEventRecord(ws.w->e0, 0);
+    e = bf ? launch_kernel<bf16, 768, 64>(C, nblocks, smem, dev, 0) : launch_kernel<float, 64, 16>(C, nblocks, smem, dev, 0);
+    cudaEventRecord(ws.w->e1, 0);
   }
-  cudaEventDestroy(e0); cudaEventDestroy(e1);
-  ar.free_all(); dj.free_all();
-  return rc;
+  if (e != cudaSuccess) { cudaStreamSynchronize(0); return fail(nullptr, OFA_CUDA_ERROR, std::string("launch failed: ") + cudaGetErrorString(e)); }
+  DevStatus& ds = *reinterpret_cast<DevStatus*>(ws.w->back);
+  cudaMemcpyAsync(&ds, C.status, sizeof ds, cudaMemcpyDeviceToHost, 0);
+  cudaEventRecord(ws.w->e2, 0);
+  if ((e = cudaEventSynchronize(ws.w->e2)) != cudaSuccess) return fail(nullptr, OFA_CUDA_ERROR, std::string("kernel failed: ") + cudaGetErrorString(e));
+  float t = 0.f; cudaEventElapsedTime(&t, ws.w->e0, ws.w->e1); if (ms) *ms = t;
+  if (ds.code || ds.abort) {
+    if (status) { status->code = OFA_DEVICE_ABORT; status->dev_code = ds.code; status->phase = ds.phase; status->task = ds.task; status->block = ds.block; status->aux = ds.aux; }
+    return fail(nullptr, OFA_DEVICE_ABORT, "device-side bounded wait expired: code " + std::to_string(ds.code) + " phase " + std::to_string(ds.phase) + " task " + std::to_string(ds.task) + " aux " + std::to_string(ds.aux));
+  }
+  return OFA_OK;
 }
 
 // Test hook: seed != 0 makes every phase uploaded afterwards (ofa_launch, ofa_run_phases) hand its tasks out in a permuted order;
