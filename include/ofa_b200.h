@@ -138,6 +138,7 @@ int ofa_read_decode_logits(ofa_ctx* ctx, float* out, size_t n);            /* fp
 #define OFA_OUT_FORCED ((1 << 24) + 1)
 /* named activation / gradient buffers for parity checks: "logits","lnf","x<l>","qkv<l>","att<l>","dx<l>", ... */
 int ofa_read_buffer(ofa_ctx* ctx, const char* name, void* out, size_t bytes);
+int ofa_read_buffer_bf16(ofa_ctx* ctx, const char* name, float* out, size_t n);   /* n elements of a bf16 buffer, widened to fp32 */
 
 /* data-parallel hooks (no counterpart in the single-GPU reference): the gradient buffer (bf16 when grad_bf16, else fp32),
  * its buckets, and the two device flag arrays (int32 per bucket). The communication side waits until ready[b] >= s+1,

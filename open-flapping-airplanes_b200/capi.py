@@ -80,6 +80,7 @@ PROTOTYPES = {
     "ofa_read_decode_tokens": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "ofa_read_decode_logits": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "ofa_read_buffer": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_size_t]),
+    "ofa_read_buffer_bf16": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_size_t]),
     "ofa_num_buckets": (C.c_int, [C.c_void_p]),
     "ofa_bucket_span": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
     "ofa_grad_buffer": (C.c_void_p, [C.c_void_p]),

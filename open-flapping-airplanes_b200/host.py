@@ -227,10 +227,13 @@ class Megakernel:
 
     def read_buffer(self, name, shape, dtype):
         """dtype: 'bf16' or a numpy dtype. Returns float32 for bf16."""
-        from .tasks import from_bf16_bits
-        host = np.empty(shape, dtype=np.uint16 if dtype == "bf16" else dtype)
+        if dtype == "bf16":
+            host = np.empty(shape, dtype=np.float32)
+            self._chk(self.lib.ofa_read_buffer_bf16(self.h, name.encode(), host.ctypes.data_as(C.c_void_p), host.size))
+            return host
+        host = np.empty(shape, dtype=dtype)
         self._chk(self.lib.ofa_read_buffer(self.h, name.encode(), host.ctypes.data_as(C.c_void_p), host.nbytes))
-        return from_bf16_bits(host).reshape(shape) if dtype == "bf16" else host
+        return host
 
     # ---- data-parallel hooks
     def buckets(self):
