@@ -19,10 +19,17 @@ namespace ew {
 
 constexpr int ROWS_PER_TASK = 16;    // embed / LayerNorm granularity
 constexpr int CE_ROWS = 4;           // rows per cross-entropy task
-constexpr int EMB_VCHUNK = 128;      // vocabulary rows per embedding-backward task
-constexpr int OPT_CHUNK = 65536;     // elements per AdamW task
+constexpr int EMB_VCHUNK = 128;      // most vocabulary rows per embedding-backward task
+constexpr int OPT_CHUNK = 65536;     // most elements per AdamW task
 constexpr int WPE_ROWS = 4;          // positions per wpe-backward task
 constexpr int SUM_CHUNK = 16384;     // elements per split-K reduce task
+
+// Task sizes of the phases that a small model would leave on a few blocks. AdamW: about four tasks per block over the whole parameter
+// vector, between 2,048 elements (one staged tile) and 65,536 (from about 78M parameters on a full GPU: a task then amortises its start);
+// the char model's 115k parameters were two tasks of 67 us. Embedding backward: half a task per block, between 8 rows (one per warp)
+// and 128; its one task of 65 rows took 60 us.
+inline int opt_chunk(size_t params, int nblocks) { int c = OPT_CHUNK; while (c > 2048 && params / c < 4 * (size_t)nblocks) c /= 2; return c; }
+inline int emb_vchunk(int V, int nblocks) { int c = EMB_VCHUNK; while (c > 8 && V / c < nblocks / 2) c /= 2; return c; }
 
 // global -> shared bulk copy by the copy engine (16-byte aligned addresses, size a multiple of 16), completion counted in bytes on `bar`
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -303,6 +310,30 @@ __device__ __forceinline__ void ce_task(int task, T* logits, const int* targets,
   }
 }
 
+// fp32 rows of a small vocabulary: one warp per row and no block-wide reductions, the row is read three times (from L1 after the
+// first). With 256 threads on each 65-entry row in turn a task of four rows took 4.3 us. Up to 2,048 entries (64 per lane); a longer
+// row keeps more lanes busy in ce_task.
+constexpr int CE_WARP_MAX_V = 2048;
+__device__ __forceinline__ void ce_task_warp(int task, float* logits, const int* targets, float* loss, int N, int V, float inv_n) {
+  constexpr float L2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = task * CE_ROWS + warp;
+  if (warp >= CE_ROWS || r >= N) return;
+  float* row = logits + (size_t)r * V;
+  const int tgt = targets[r];
+  float m = -INFINITY;
+#pragma unroll 4
+  for (int v = lane; v < V; v += 32) m = fmaxf(m, row[v]);
+  const float M = warp_max(m) * L2E;
+  float s = 0.f;
+#pragma unroll 4
+  for (int v = lane; v < V; v += 32) s += exp2f(fmaf(row[v], L2E, -M));
+  const float S = warp_sum(s), invS = 1.f / S;
+  if (lane == 0) loss[r] = M * LN2 + logf(S) - row[tgt];
+  __syncwarp();
+#pragma unroll 4
+  for (int v = lane; v < V; v += 32) row[v] = (exp2f(fmaf(row[v], L2E, -M)) * invS - (v == tgt ? 1.f : 0.f)) * inv_n;
+}
+
 // The same task for bf16 rows that fit the cache entirely: the row is brought into shared memory by bulk copies (the copy
 // engine streams it without occupying the threads or their registers; with the loop of 16-byte loads above a thread had one
 // or two loads in flight and the phase ran at a third of the HBM rate), then both passes read shared memory. The arithmetic
@@ -472,7 +503,8 @@ __device__ __forceinline__ float ce_mean_task(float* mean_loss, const float* los
 __host__ __device__ constexpr size_t embed_bwd_wte_smem_bytes(int N) { return 1024 + 5 * (size_t)N; }
 
 // dwte[v,:] (=|+=) sum over tokens n with tok[n] == v of dx0[n,:], added in increasing n (the reference's order,
-// llm/elementwise/ew_loss.cuh:101-177, so that the sum does not depend on the schedule). Task = 128 vocabulary rows.
+// llm/elementwise/ew_loss.cuh:101-177, so that the sum does not depend on the schedule). Task = `vchunk` vocabulary rows: 128, fewer
+// when the vocabulary is too small to give every block a task (see emb_vchunk).
 //   1. Each warp looks at its own contiguous eighth of the token positions, 32 at a time: ballots count its matches (and a shared
 //      counter per row says how many each row has; most rows of a chunk have none), the eight warp counts give it its place in an
 //      ORDERED list of (position, row) pairs, and a second look at the same positions fills the list.
@@ -481,7 +513,7 @@ __host__ __device__ constexpr size_t embed_bwd_wte_smem_bytes(int N) { return 10
 // Without `accumulate` every row of the chunk is written (zeros where the token is absent), so the gradient buffer needs no
 // clearing between steps. Shared memory: 8 warp counts + 128 row counts, then int list[N], then one byte per list entry.
 template <class T, int D, class GT>
-__device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0, const int* tok, int N, int V, int accumulate,
+__device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0, const int* tok, int N, int V, int vchunk, int accumulate,
                                                 unsigned char* smem) {
   using R = RowRegs<T, D>;
   constexpr int VN = R::VN, NV = R::NV;
@@ -489,7 +521,7 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
   int* rowcnt = wcnt + 8;                              // [EMB_VCHUNK]
   int* list = reinterpret_cast<int*>(smem + 1024);     // [N] matching positions, increasing
   unsigned char* rowof = smem + 1024 + 4 * (size_t)N;  // [N] row within the chunk of each list entry
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, lo = task * EMB_VCHUNK;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, lo = task * vchunk;
   if (t < EMB_VCHUNK) rowcnt[t] = 0;
   __syncthreads();
   // warp w owns positions [w * per, (w + 1) * per): its matches follow those of the warps before it, in position order
@@ -515,7 +547,7 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
     slot += __popc(b);
   }
   __syncthreads();
-  for (int r = warp; r < EMB_VCHUNK; r += NTHR / 32) {
+  for (int r = warp; r < vchunk; r += NTHR / 32) {
     if (lo + r >= V) break;
     GT* dst = dwte + (size_t)(lo + r) * D;
     const int mine = rowcnt[r];
@@ -559,16 +591,31 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
 }
 
 // dwpe32[p,:] (=) sum_b dx0[b*Tctx + p,:], b increasing. Task = 4 positions.
+// A thread owns four columns of one position and asks for four sequences at a time (one 2- or 4-byte load in flight per thread took
+// 14 us for the char model's 16 sequences and 23 us at 4 x 768).
 template <class T, class GT>
 __device__ __forceinline__ void embed_bwd_wpe_task(int task, GT* dwpe32, const T* dx0, int N, int Tctx, int D) {
-  for (int pp = 0; pp < WPE_ROWS; pp++) {
-    const int p = task * WPE_ROWS + pp;
+  const int per_row = D / 4;
+  for (int i = threadIdx.x; i < WPE_ROWS * per_row; i += NTHR) {
+    const int p = task * WPE_ROWS + i / per_row, c = (i % per_row) * 4;
     if (p >= Tctx) break;
-    for (int c = threadIdx.x; c < D; c += NTHR) {
-      float s = 0.f;
-      for (int n = p; n < N; n += Tctx) s += to_f(dx0[(size_t)n * D + c]);
-      dwpe32[(size_t)p * D + c] = from_f<GT>(s);
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    int n = p;
+    for (; n + 3 * Tctx < N; n += 4 * Tctx) {
+      float f[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) ld4(dx0 + (size_t)(n + u * Tctx) * D + c, f[u]);
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) s[k] += f[u][k];
     }
+    for (; n < N; n += Tctx) {
+      float f[4]; ld4(dx0 + (size_t)n * D + c, f);
+#pragma unroll
+      for (int k = 0; k < 4; k++) s[k] += f[k];
+    }
+    st4(dwpe32 + (size_t)p * D + c, s);
   }
 }
 
@@ -593,7 +640,7 @@ __device__ __forceinline__ AdamHP adam_hp(const AdamConst& h, int step) {
 //   p -= lr/(1 - b1^t) * m / (sqrt(v)/sqrt(1 - b2^t) + eps)          (bias corrections in double)
 // then the working copy Wact (type T) that forward, backward and the decoder read is refreshed. The gradient is read as GT
 // (fp32 single-GPU buffer, or the all-reduced bf16 bucket) and multiplied by grad_scale (1/world size).
-// nodecay: sorted disjoint [start,end) element ranges relative to W. Task = 65,536 elements; n and ranges multiples of 4.
+// nodecay: sorted disjoint [start,end) element ranges relative to W. Task = `chunk` elements (see opt_chunk); n and ranges multiples of 4.
 struct AdamMath {                     // the per-task constants and the four-element update shared by both task bodies
   float step_size, inv_sqrt_bc2, decay_mul, one_minus_b1, one_minus_b2, b2, eps, gscale;
   const int2* nd; int n_nd, first_nd; bool any_nd;
@@ -639,10 +686,10 @@ __device__ __forceinline__ void adamw_span_direct(const AdamMath& A, size_t begi
 }
 template <class T, class GT>
 __device__ __forceinline__ void adamw_task(int task, float* W, const GT* G, float* M, float* Vv, T* Wact, size_t n, AdamHP hp,
-                                           const int2* nodecay, int n_nodecay) {
-  const size_t cs = (size_t)task * OPT_CHUNK;
+                                           const int2* nodecay, int n_nodecay, int chunk) {
+  const size_t cs = (size_t)task * chunk;
   if (cs >= n) return;
-  const size_t ce = cs + OPT_CHUNK < n ? cs + OPT_CHUNK : n;
+  const size_t ce = cs + chunk < n ? cs + chunk : n;
   AdamMath A; A.init(hp, nodecay, n_nodecay, cs, ce);
   adamw_span_direct<T, GT>(A, cs, ce, W, G, M, Vv, Wact);
 }
@@ -657,11 +704,11 @@ __device__ __forceinline__ void adamw_task(int task, float* W, const GT* G, floa
 constexpr int ADAM_TILE = 2048, ADAM_STAGES = 3, ADAM_STAGE_BYTES = 32768;
 template <class T, class GT>
 __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, float* M, float* Vv, T* Wact, size_t n, AdamHP hp,
-                                                const int2* nodecay, int n_nodecay, unsigned char* smem, uint32_t bar0, uint32_t& tiles,
+                                                const int2* nodecay, int n_nodecay, int chunk, unsigned char* smem, uint32_t bar0, uint32_t& tiles,
                                                 const DevStatus* st) {
-  const size_t cs = (size_t)task * OPT_CHUNK;
+  const size_t cs = (size_t)task * chunk;
   if (cs >= n) return;
-  const size_t ce = cs + OPT_CHUNK < n ? cs + OPT_CHUNK : n;
+  const size_t ce = cs + chunk < n ? cs + chunk : n;
   AdamMath A; A.init(hp, nodecay, n_nodecay, cs, ce);
   const int tid = threadIdx.x;
   const bool aligned = ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(M) | reinterpret_cast<uintptr_t>(Vv) | reinterpret_cast<uintptr_t>(G)) & 15) == 0;

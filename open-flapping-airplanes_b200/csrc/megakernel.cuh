@@ -95,6 +95,9 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
           break;
         }
       }
+      if constexpr (!IsBf16<T>::value) {
+        if (md.V <= ew::CE_WARP_MAX_V) { ew::ce_task_warp(local, (float*)d.p[0], (const int*)d.p[1], (float*)d.p[2], md.N, md.V, 1.0f / (float)md.N); break; }
+      }
       ew::ce_task<T>(local, (T*)d.p[0], (const int*)d.p[1], (float*)d.p[2], md.N, md.V, 1.0f / (float)md.N, smem, d.i0);
       break;
     case TK_CE_MEAN: {
@@ -111,8 +114,8 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
       else ew::ln_dgamma_reduce_task<float>(local, (float*)d.p[0], (const float*)d.p[1], (md.N + ew::ROWS_PER_TASK - 1) / ew::ROWS_PER_TASK, D, d.i0);
       break;
     case TK_EMB_WTE:
-      if (d.i1) ew::embed_bwd_wte_task<T, D, bf16>(local, (bf16*)d.p[0], (const T*)d.p[1], (const int*)d.p[2], md.N, md.V, d.i0, smem);
-      else ew::embed_bwd_wte_task<T, D, float>(local, (float*)d.p[0], (const T*)d.p[1], (const int*)d.p[2], md.N, md.V, d.i0, smem);
+      if (d.i1) ew::embed_bwd_wte_task<T, D, bf16>(local, (bf16*)d.p[0], (const T*)d.p[1], (const int*)d.p[2], md.N, md.V, d.tiles_m, d.i0, smem);
+      else ew::embed_bwd_wte_task<T, D, float>(local, (float*)d.p[0], (const T*)d.p[1], (const int*)d.p[2], md.N, md.V, d.tiles_m, d.i0, smem);
       break;
     case TK_EMB_WPE:
       if (d.i1) ew::embed_bwd_wpe_task<T, bf16>(local, (bf16*)d.p[0], (const T*)d.p[1], md.N, md.T, D);
@@ -123,13 +126,13 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
       if constexpr (IsBf16<T>::value) {               // inputs staged by the copy engine (the fp32 preset's blocks have no room for the stages)
         const uint32_t bar0 = smem_u32(smem + C.smem_bytes - CTRL_BYTES + 224);
         if (d.i2 == 0) {
-          if (d.i1) ew::adamw_task_bulk<T, bf16>(local, (float*)d.p[0], (const bf16*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, smem, bar0, adam_tiles, C.status);
-          else ew::adamw_task_bulk<T, float>(local, (float*)d.p[0], (const float*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, smem, bar0, adam_tiles, C.status);
+          if (d.i1) ew::adamw_task_bulk<T, bf16>(local, (float*)d.p[0], (const bf16*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m, smem, bar0, adam_tiles, C.status);
+          else ew::adamw_task_bulk<T, float>(local, (float*)d.p[0], (const float*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m, smem, bar0, adam_tiles, C.status);
           break;
         }
       }
-      if (d.i1) ew::adamw_task<T, bf16>(local, (float*)d.p[0], (const bf16*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0);
-      else ew::adamw_task<T, float>(local, (float*)d.p[0], (const float*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0);
+      if (d.i1) ew::adamw_task<T, bf16>(local, (float*)d.p[0], (const bf16*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m);
+      else ew::adamw_task<T, float>(local, (float*)d.p[0], (const float*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m);
       break;
     }
     case TK_SUMCAST:

@@ -200,8 +200,9 @@ bool prepare_gemm_bf16(PhaseDesc& d, MapSink& sink, int nsub_cfg, int nblocks, s
   return true;
 }
 void prepare_gemm_f32(PhaseDesc& d) {
-  d.tiles_m = (d.g.M + f32::GT - 1) / f32::GT;
-  d.ntasks = d.tiles_m * ((d.g.N + f32::GT - 1) / f32::GT);
+  const int t = f32::gemm_tile(d.layout);
+  d.tiles_m = (d.g.M + t - 1) / t;
+  d.ntasks = d.tiles_m * ((d.g.N + t - 1) / t);
   d.g.nsub = 1;
 }
 
@@ -449,6 +450,7 @@ bool build_train_graph(ofa_ctx* c) {
   };
   const bool train = cfg.mode == OFA_MODE_TRAIN, fwd_only = cfg.mode == OFA_MODE_FORWARD;
   const bool gbf = cfg.grad_bf16 != 0;
+  const int train_blocks = c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, opt_chunk = ew::opt_chunk(lay.total, train_blocks);
   auto G = [&](size_t off) -> void* { return gbf ? (void*)(c->Gbf + off) : (void*)(c->G32 + off); };
   const int wepi = gbf ? GE_STORE : GE_F32;
   const int rows16 = (int)((N + 15) / 16);
@@ -570,7 +572,8 @@ bool build_train_graph(ofa_ctx* c) {
       return deps;
     };
     auto mkadam = [&](size_t off, size_t n, const std::vector<Span>& nodecay) {
-      PhaseDesc d = mk(TK_ADAMW, (int)((n + ew::OPT_CHUNK - 1) / ew::OPT_CHUNK));
+      PhaseDesc d = mk(TK_ADAMW, (int)((n + opt_chunk - 1) / opt_chunk));
+      d.tiles_m = opt_chunk;
       d.p[0] = c->W32 + off; d.p[1] = G(off); d.p[2] = c->M32 + off; d.p[3] = c->V32 + off; d.p[4] = Wact + off;
       d.n = n; d.i0 = (int)nodecay.size(); d.i1 = gbf ? 1 : 0;
       d.i2 = getenv("OFA_B200_ADAM_DIRECT") ? 1 : 0;     // A/B switch for measurements: 1 = the loop of direct loads instead of the staged inputs
@@ -616,11 +619,11 @@ bool build_train_graph(ofa_ctx* c) {
       long budget = flush ? (1L << 40) : trickle_n;
       while (budget > 0 && adam_q_head < adam_q.size()) {
         AdamItem& it = adam_q[adam_q_head];
-        const int total = (int)((it.n + ew::OPT_CHUNK - 1) / ew::OPT_CHUNK);
+        const int total = (int)((it.n + opt_chunk - 1) / opt_chunk);
         int cnt = (int)std::min<long>(budget, total - it.next_task);
         if (total - it.next_task - cnt < trickle_n / 2) cnt = total - it.next_task;        // no tiny remainder
         const bool last = it.next_task + cnt == total;
-        const size_t o = it.off + (size_t)it.next_task * ew::OPT_CHUNK, nn = std::min((size_t)cnt * ew::OPT_CHUNK, it.off + it.n - o);
+        const size_t o = it.off + (size_t)it.next_task * opt_chunk, nn = std::min((size_t)cnt * opt_chunk, it.off + it.n - o);
         if (last && it.chunks == 0) {                    // the whole group in one piece: an ordinary optimizer phase
           addp(it.name, mkadam_range(o, nn, it.nd), it.deps, {});
         } else {
@@ -716,7 +719,8 @@ bool build_train_graph(ofa_ctx* c) {
         if (b.last_layer == l) signal(bucket_of_layer[l]);
       }
     }
-    { PhaseDesc d = mk(TK_EMB_WTE, (int)((V + ew::EMB_VCHUNK - 1) / ew::EMB_VCHUNK)); d.p[0] = G(lay.wte); d.p[1] = dxs[0]; d.p[2] = c->C.tok_in; d.i0 = lay.tied ? 1 : 0; d.i1 = gbf ? 1 : 0;
+    const int vchunk = ew::emb_vchunk((int)V, train_blocks);
+    { PhaseDesc d = mk(TK_EMB_WTE, (int)((V + vchunk - 1) / vchunk)); d.tiles_m = vchunk; d.p[0] = G(lay.wte); d.p[1] = dxs[0]; d.p[2] = c->C.tok_in; d.i0 = lay.tied ? 1 : 0; d.i1 = gbf ? 1 : 0;
       addp("embed bwd wte", d, {"L0 ln1 bwd", lay.tied ? "head dW" : ""}, {}); }
     { PhaseDesc d = mk(TK_EMB_WPE, (m.T + ew::WPE_ROWS - 1) / ew::WPE_ROWS); d.p[0] = G(lay.wpe); d.p[1] = dxs[0]; d.i1 = gbf ? 1 : 0; addp("embed bwd wpe", d, {"L0 ln1 bwd"}, {}); }
     if (ext) signal((int)buckets.size() - 1);
@@ -1552,9 +1556,9 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
         d.i0 = (int)(std::min<size_t>((size_t)((bf ? gemm_tc::BAR_OFFSET : smem - CTRL_BYTES) - 64), (size_t)m.V * (bf ? 2 : 4)) / 16 * 16); break;
       case TK_CE_MEAN: d.ntasks = 1; break;
       case TK_BARRIER: d.ntasks = s.n > 0 ? (int)std::min<size_t>(s.n, 1u << 24) : 1; break;     // n empty tasks: what a task costs the scheduler alone
-      case TK_EMB_WTE: d.ntasks = (m.V + ew::EMB_VCHUNK - 1) / ew::EMB_VCHUNK; break;
+      case TK_EMB_WTE: d.tiles_m = ew::emb_vchunk(m.V, nblocks); d.ntasks = (m.V + d.tiles_m - 1) / d.tiles_m; break;
       case TK_EMB_WPE: d.ntasks = (m.T + ew::WPE_ROWS - 1) / ew::WPE_ROWS; break;
-      case TK_ADAMW: d.ntasks = (int)((s.n + ew::OPT_CHUNK - 1) / ew::OPT_CHUNK); if (s.n == 0 || s.n % 4) { return fail(nullptr, OFA_BAD_ARGUMENT, "AdamW n must be a positive multiple of 4"); } break;
+      case TK_ADAMW: d.tiles_m = ew::opt_chunk(s.n, nblocks); d.ntasks = (int)((s.n + d.tiles_m - 1) / d.tiles_m); if (s.n == 0 || s.n % 4) { return fail(nullptr, OFA_BAD_ARGUMENT, "AdamW n must be a positive multiple of 4"); } break;
       default: return fail(nullptr, OFA_BAD_ARGUMENT, "task kind not available at task level");
     }
     if (bf && (s.kind == TK_ATT_FWD || s.kind == TK_ATT_BWD || s.kind == TK_ATT_PREP) && m.T % attn::QTILE) { return fail(nullptr, OFA_BAD_ARGUMENT, "ctx_len must be a multiple of 128"); }
