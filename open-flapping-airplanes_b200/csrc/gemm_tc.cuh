@@ -99,6 +99,22 @@ __device__ __forceinline__ void block_exit(GemmPipe& gp, unsigned char* smem, De
   if (threadIdx.x < 32) tmem_dealloc(gp.tmem_base, TMEM_COLS);
 }
 
+// Asks for the B operand of a task whose B is a weight matrix (PhaseDesc::i1) to be brought to L2, while the block waits for the tasks
+// that produce A. With few tokens every weight tile comes from HBM and the three-stage pipeline sees its latency on every third
+// k-step. One of the tasks that share a strip of B does it; at most 64 boxes (1 MB of K-major, 0.5 MB of MN-major tiles).
+__device__ __forceinline__ void l2_prefetch_box(const void* tmap, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void prefetch_weights(const PhaseDesc& d, int task) {
+  const GemmArgs& g = d.g;
+  if (task % d.tiles_m != 0) return;
+  const int n0 = (task / d.tiles_m) * g.nsub * g.bn, n1 = min(g.N, n0 + g.nsub * g.bn);
+  const bool kmajor = d.layout == GL_NT;
+  int left = 64;
+  for (int n = n0; n < n1 && left > 0; n += kmajor ? 128 : 64)
+    for (int k = 0; k < g.K && left > 0; k += BK, left--) { if (kmajor) l2_prefetch_box(g.tmB, k, n); else l2_prefetch_box(g.tmB, n, k); }
+}
+
 // ---------------------------------------------------------------------------------------------- epilogue math
 // The epilogues that meet their second operand in fp32 before the one rounding (and the fp32 result): eight consecutive
 // columns of one row, after the fp32 transpose. Everything else is stored from the bf16-staged pass of the task itself.

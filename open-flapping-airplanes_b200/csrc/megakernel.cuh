@@ -209,8 +209,8 @@ __device__ __forceinline__ int wait_deps(const Ctx& C, const Job& J, int job_id,
   const u64 limit = C.dep_timeout_ns + (C.dep_timeout_ns >> 1);
   unsigned spins = 0;
   if (cnt >= 0) {
-    // up to four dependencies from the phase's scheduling record: their counters are read with relaxed loads that are all in
-    // flight together, and one acquire fence after the last successful check orders the task's reads behind them
+    // up to four dependencies from the phase's scheduling record: their counters are read with acquire loads that are all in flight
+    // together (a load costs 303 cycles either way; relaxed loads and a fence behind the last one cost 310 more per wait)
     int need[4]; const int* ctr[4]; int span[4];
     int prod = 0, clo = 0, chi = 0;
     if (R.any_rb) rb_of_task(R.rb_map, C.md, local, prod, clo, chi);
@@ -218,7 +218,7 @@ __device__ __forceinline__ int wait_deps(const Ctx& C, const Job& J, int job_id,
     for (int k = 0; k < 4; k++) {
       const int p = k < cnt ? R.ph[k] : 0, dl = k < cnt ? R.dl[k] : 0, nt = k < cnt ? R.nt[k] : 0;
       const bool g = k < cnt && R.gr[k];
-      ctr[k] = g ? J.done_rb + prod_rb_off[k] + clo : J.done + p;
+      ctr[k] = g ? J.done_rb + (prod_rb_off[k] + clo) * RB_STRIDE : J.done + p * DONE_STRIDE;
       span[k] = g ? chi - clo + 1 : 1;
       need[k] = k < cnt ? nt * (step + 1 + dl) : 0;
     }
@@ -227,29 +227,38 @@ __device__ __forceinline__ int wait_deps(const Ctx& C, const Job& J, int job_id,
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (need[k] > 0) {
-          int v = ld_relaxed(ctr[k]);
-          for (int q = 1; q < span[k]; q++) v = min(v, ld_relaxed(ctr[k] + q));
+          int v = ld_acquire(ctr[k]);
+          for (int q = 1; q < span[k]; q++) v = min(v, ld_acquire(ctr[k] + q * RB_STRIDE));
           ready = ready && v >= need[k];
         }
       }
-      if (ready) { fence_acquire(); return 0; }
+      if (ready) return 0;
       if (job_id == 1 && C.use_train && ld_relaxed(C.finished)) return -2;
       if ((++spins & 63u) == 0) {
         if (aborted(C.status)) return -2;
         if (gtimer() - t0 > limit) { raise_abort(C.status, ST_DEP_TIMEOUT, ph, local, step); return -2; }
       }
-      __nanosleep(job_id == 1 ? 20 : 80);
+      if (spins > 32u) __nanosleep(job_id == 1 ? 20 : 80);       // a short wait, the rule along a chain of small phases, is polled without a pause
     }
   }
   const int off = __ldg(J.dep_off + ph), n = __ldg(J.dep_cnt + ph);
+  // more than four (AdamW, the end of a step): eight counters at a time are in flight, and those already seen complete are not read again
+  int seen = 0;
   for (;;) {
-    bool ready = true;
-    for (int k = 0; k < n && ready; k++) {
-      const Dep e = J.deps[off + k];
-      const int need = __ldg(J.ntasks + e.phase) * (step + 1 + e.delta);
-      if (need > 0 && ld_acquire(J.done + e.phase) < need) ready = false;
+    while (seen < n) {
+      bool ready = true;
+      const int m = min(8, n - seen);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        if (k < m) {
+          const Dep e = J.deps[off + seen + k];
+          ready = ready && ld_relaxed(J.done + e.phase * DONE_STRIDE) >= __ldg(J.ntasks + e.phase) * (step + 1 + e.delta);
+        }
+      }
+      if (!ready) break;
+      seen += m;
     }
-    if (ready) return 0;
+    if (seen >= n) { fence_acquire(); return 0; }
     if (job_id == 1 && C.use_train && ld_relaxed(C.finished)) return -2;
     if ((++spins & 63u) == 0) {
       if (aborted(C.status)) return -2;
@@ -352,23 +361,7 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
           // must not change any result - the reference's shuffled-order check (llm/gemm/test_gemm.cu:20-49)
           if (c_mul) local = (int)(((long long)local * c_mul + (c_mul >> 1)) % (long long)(c_hi - c_lo));
           // a phase whose dependencies are all phase-level stays ready once it has been seen ready; row-block dependencies are per task
-          if (job_id == 0 && (!(step == rstep && ph == rph) || c_any_rb)) {
-            const u64 w0 = prof ? gtimer() : 0;
-            DepSet ds; int pro[4] = {0, 0, 0, 0};
-            if (ptab) load_deps(ds, reinterpret_cast<const int*>(prec + ph)); else { need_rec(ph); load_deps(ds, s_rec); }
-            if (ds.any_rb) {
-#pragma unroll
-              for (int k = 0; k < 4; k++) if (k < ds.cnt && ds.gr[k]) pro[k] = ptab ? prec[ds.ph[k]].rb_off : __ldg(&J.rec[ds.ph[k]].rb_off);
-            }
-            res = wait_deps(C, J, job_id, step, ph, local, ds, pro);
-            c_any_rb = ds.any_rb;
-            if (prof) {
-              const u64 w = gtimer() - w0;
-              waited += w;
-              if (C.phase_busy && w > 200) atomicAdd(C.phase_busy + J.nph + ph, w);
-            }
-            if (res == 0) { rstep = step; rph = ph; }
-          }
+          if (job_id == 0 && (!(step == rstep && ph == rph) || c_any_rb)) res = 1;      // the dependencies have to be waited for
         }
       }
       s_sel[0] = res; s_sel[1] = step; s_sel[2] = ph; s_sel[3] = local; s_sel[5] = c_rb_off; s_sel[6] = c_rb_map;
@@ -385,15 +378,44 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
     // longer holds it, and the chain of dependent global loads that decoding it would take was a measurable part of the
     // per-task overhead. Two slots: the next phase's descriptor is requested at the end of a task (below), so a block that
     // moves on by one phase - the common case when phases have about as many tasks as there are blocks - finds it here.
+    bool settle = res == 1;                          // a second barrier is due before the task starts
     if (ph != cached_ph) {
       if (ph == ahead_ph) { slot ^= 1; ahead_ph = cached_ph; cached_ph = ph; }      // already there: no second barrier (-0.9 % per step)
       else {
-        if (tid < (int)(sizeof(PhaseDesc) / 4)) reinterpret_cast<uint32_t*>(ctrl + 256 + 256 * slot)[tid] = __ldg(reinterpret_cast<const uint32_t*>(J.ph + ph) + tid);
+        const int q = tid - 64;
+        if (q >= 0 && q < (int)(sizeof(PhaseDesc) / 4)) reinterpret_cast<uint32_t*>(ctrl + 256 + 256 * slot)[q] = __ldg(reinterpret_cast<const uint32_t*>(J.ph + ph) + q);
         cached_ph = ph;
-        __syncthreads();
+        settle = true;
       }
     }
     const PhaseDesc& d = *reinterpret_cast<const PhaseDesc*>(ctrl + 256 + 256 * slot);
+    // Thread 0 waits for the dependencies while other threads fetch the descriptor: behind the wait, a descriptor that was not
+    // fetched ahead cost its round trip on the critical path of every phase change.
+    if (settle) {
+      if (tid == 0 && res == 1) {
+        const u64 w0 = prof ? gtimer() : 0;
+        DepSet ds; int pro[4] = {0, 0, 0, 0};
+        if (ptab) load_deps(ds, reinterpret_cast<const int*>(prec + ph)); else { need_rec(ph); load_deps(ds, s_rec); }
+        if (ds.any_rb) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) if (k < ds.cnt && ds.gr[k]) pro[k] = ptab ? prec[ds.ph[k]].rb_off : __ldg(&J.rec[ds.ph[k]].rb_off);
+        }
+        const int r2 = wait_deps(C, J, job_id, step, ph, local, ds, pro);
+        c_any_rb = ds.any_rb;
+        if (prof) {
+          const u64 w = gtimer() - w0;
+          waited += w;
+          if (C.phase_busy && w > 200) atomicAdd(C.phase_busy + J.nph + ph, w);
+        }
+        if (r2 == 0) { rstep = step; rph = ph; }
+        s_sel[4] = r2;
+        if (prof) tl1 = gtimer();
+      }
+      // meanwhile the weights of the task, which no task of this step writes, start on their way to L2
+      if constexpr (IsBf16<T>::value) if (tid == 32 && res == 1 && J.ph[ph].kind == TK_GEMM && J.ph[ph].i1) gemm_tc::prefetch_weights(J.ph[ph], local);
+      __syncthreads();
+      if (res == 1 && s_sel[4] < 0) break;
+    }
     bool filled = false;
     if (job_id == 1) {                               // ---- serving: start the weight prefetch, THEN wait for the dependencies
       filled = dec::prefetch<T, D, DH>(C.dp, C.md, d.kind, d.i0, local, smem, fill_bar);
@@ -461,15 +483,15 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
         if (job_id == 1 && C.dec_phase_busy) atomicAdd(C.dec_phase_busy + ph, t1 - t0);
       }
     } else if (tid == 32) {
-      __threadfence();
+      fence_acq_rel();
       const int rb_off = t_rb_off, rb_map = t_rb_map;
       if (rb_off >= 0) {                               // completions per row block first: their waiters are the ones on the critical chain
         int prod, clo, chi; rb_of_task(rb_map, C.md, local, prod, clo, chi);
-        red_relaxed_add(J.done_rb + rb_off + prod, 1);
+        red_relaxed_add(J.done_rb + (rb_off + prod) * RB_STRIDE, 1);
       }
-      if (ph != J.last_phase) red_relaxed_add(J.done + ph, 1);
+      if (ph != J.last_phase) red_relaxed_add(J.done + ph * DONE_STRIDE, 1);
       else {                                           // the step's last phase needs the old value
-        const int old = atomicAdd(J.done + ph, 1);
+        const int old = atomicAdd(J.done + ph * DONE_STRIDE, 1);
         if (job_id == 0 && old == __ldg(J.ntasks + ph) * (step + 1) - 1) {     // last task of the step
           const u64 t1 = gtimer();
           C.step_done[step] = t1;

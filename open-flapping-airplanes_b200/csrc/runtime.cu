@@ -258,7 +258,7 @@ constexpr size_t up64(size_t n) { return (n + 63) / 64 * 64; }
 size_t job_table_bytes(const HostJob& h) {
   return up64(sizeof(PhaseDesc) * h.nph) + up64(sizeof(SchedRec) * h.nph) + up64(4 * ((size_t)h.nph + 1)) + 3 * up64(4 * (size_t)h.nph) + up64(sizeof(Dep) * h.deps.size());
 }
-size_t job_counter_bytes(const HostJob& h) { return 64 + up64(4 * (size_t)h.nph) + up64(4 * (size_t)std::max(1, h.rb_total)); }
+size_t job_counter_bytes(const HostJob& h) { return 128 + 4 * (size_t)(DONE_STRIDE * h.nph + RB_STRIDE * std::max(1, h.rb_total)); }
 // writes the tables to `host` (an image of `dev`) and fills the job's pointers; `cnt` = its counters, to be zero before a launch
 Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* dev, unsigned char* cnt) {
   Job j{};
@@ -271,7 +271,7 @@ Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* 
   j.dep_off = reinterpret_cast<const int*>(put(h.doff.data(), 4 * (size_t)h.nph));
   j.dep_cnt = reinterpret_cast<const int*>(put(h.dcnt.data(), 4 * (size_t)h.nph));
   j.deps = reinterpret_cast<const Dep*>(put(h.deps.data(), sizeof(Dep) * h.deps.size()));
-  j.ticket = reinterpret_cast<unsigned*>(cnt); j.done = reinterpret_cast<int*>(cnt + 64); j.done_rb = reinterpret_cast<int*>(cnt + 64 + up64(4 * (size_t)h.nph));
+  j.ticket = reinterpret_cast<unsigned*>(cnt); j.done = reinterpret_cast<int*>(cnt + 128); j.done_rb = j.done + (size_t)DONE_STRIDE * h.nph;
   j.nph = h.nph; j.tasks_per_step = h.prefix[h.nph]; j.nsteps = nsteps; j.last_phase = h.last_phase;
   return j;
 }
@@ -435,6 +435,7 @@ bool build_train_graph(ofa_ctx* c) {
   };
   MapSink sink; sink.ar = &c->ar;
   auto mk = [&](int kind, int ntasks) { PhaseDesc d; memset(&d, 0, sizeof d); d.kind = kind; d.ntasks = ntasks; return d; };
+  auto is_weight = [&](const void* p) { const T* w = reinterpret_cast<const T*>(p); return w >= Wact && w < Wact + lay.total; };   // read by the step, written only by its optimizer
   // wide = 1: 128 x 256 tiles where the width allows (a long K and more tiles than blocks: only the LM head's weight gradient)
   auto mkgemm = [&](int layout, int epi, const void* A, int lda, const void* B, int ldb, void* Cc, int ldc, void* aux, int ldaux,
                     int M, int Nn, int K, int accumulate, int wide = 0) {
@@ -446,6 +447,7 @@ bool build_train_graph(ofa_ctx* c) {
     const int nsub_cfg = (wide && cfg.gemm_nsub == 0 && !getenv("OFA_B200_HEAD_DW_128")) ? (getenv("OFA_B200_HEAD_DW_STRIPS") ? 2000 : 4001) : cfg.gemm_nsub;
     if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, nsub_cfg, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }   // waves are counted over the blocks that train
     else prepare_gemm_f32(d);
+    d.i1 = is_weight(B) ? 1 : 0;
     return d;
   };
   const bool train = cfg.mode == OFA_MODE_TRAIN, fwd_only = cfg.mode == OFA_MODE_FORWARD;
@@ -523,6 +525,7 @@ bool build_train_graph(ofa_ctx* c) {
     d.g.dr = reinterpret_cast<float*>(lse_part);
     if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, cfg.gemm_nsub, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }
     else prepare_gemm_f32(d);
+    d.i1 = 1;
     addp("logits", d, {"lnf"}, {opt_head}, {"lnf"});
   }
   std::vector<std::string> end_deps;
@@ -1515,7 +1518,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   // per phase (two for the first), at most four TMA descriptors per phase, counters, and what the kernel reports per repeat
   const size_t map_cap = (size_t)nph * sizeof(attn_tc::Maps), tab_cap = (size_t)nph * (sizeof(PhaseDesc) + sizeof(SchedRec) + 24 + sizeof(Dep)) + 1024;
   const size_t rep_bytes = up64(sizeof(unsigned long long) * (size_t)repeats) + up64(sizeof(float) * (size_t)repeats);
-  const size_t cnt_cap = 64 + up64(4 * (size_t)nph) + 64;
+  const size_t cnt_cap = 128 + 4 * (size_t)(DONE_STRIDE * nph + RB_STRIDE);
   WorkspaceLease ws(dev, map_cap + tab_cap + 192 + cnt_cap, rep_bytes);
   if (!ws.w) return fail(nullptr, OFA_CUDA_ERROR, "out of memory (workspace)");
   MapSink sink; sink.host = ws.w->host; sink.dev = ws.w->dev; sink.cap = map_cap;
@@ -1529,6 +1532,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
     const int BH = m.B * m.H, rows16 = (m.N + 15) / 16;
     switch (s.kind) {
       case TK_GEMM:
+        d.i1 = 0;                // nothing is known about who writes B
         d.g.A = s.p[0]; d.g.B = s.p[1]; d.g.C = s.p[2]; d.g.aux = s.p[3]; d.g.M = s.M; d.g.N = s.N; d.g.K = s.K; d.g.lda = s.lda; d.g.ldb = s.ldb; d.g.ldc = s.ldc; d.g.ldaux = s.ldaux;
         d.g.accumulate = s.accumulate;
         if (s.epi == GE_LSE) {  // p[4] = softmax partials [M, N / 128] float2

@@ -102,6 +102,9 @@ struct alignas(16) SchedRec {
   int pad[2];
 };
 constexpr int DEP_PREV = 1 << 16, DEP_RB = 1 << 17;
+// Completion counters sit in lines (phases) and sectors (row blocks) of their own: every block of the GPU polls the counter of the phase
+// it waits for while others add to it, and 32 phases in one line would put all of that on one L2 slice.
+constexpr int DONE_STRIDE = 32, RB_STRIDE = 8;
 constexpr int CTRL_BYTES = 1024;   // control area at the end of every block's dynamic shared memory
 // The scheduling records of both jobs travel with the launch as part of the kernel parameter (constant bank): a block that
 // claims a ticket finds the phase and its dependencies without a single round trip to global memory. Jobs with more phases than
@@ -117,8 +120,8 @@ struct Job {
   const int* dep_cnt;       // [nph]
   const Dep* deps;
   const SchedRec* rec;      // [nph]
-  int* done;                // [nph] monotonically increasing over steps
-  int* done_rb;             // completions per (phase that publishes them, row block of 128 tokens), monotonically increasing; see SchedRec
+  int* done;                // [nph] monotonically increasing over steps, DONE_STRIDE words apart
+  int* done_rb;             // completions per (phase that publishes them, row block of 128 tokens), monotonically increasing, RB_STRIDE words apart; see SchedRec
   unsigned* ticket;         // next (step * tasks_per_step + task) to hand out
 };
 
