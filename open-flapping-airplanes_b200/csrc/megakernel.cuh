@@ -159,12 +159,12 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
 }
 
 template <class T, int D, int DH>
-__device__ __forceinline__ void run_decode_task(const Ctx& C, const PhaseDesc& d, int local, unsigned char* smem, uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ void run_decode_task(const Ctx& C, const PhaseDesc& d, int local, int step, unsigned char* smem, uint32_t bar, uint32_t parity) {
   switch (d.kind) {
-    case TK_DEC_QKV: dec::task_qkv<T, D, DH>(C.dp, C.md, d.i0, local, smem, bar, parity, C.status); break;
-    case TK_DEC_ATTWO: dec::task_attwo<T, D, DH>(C.dp, C.md, d.i0, local, smem, bar, parity, C.status); break;
+    case TK_DEC_QKV: dec::task_qkv<T, D, DH>(C.dp, C.md, d.i0, local, step, smem, bar, parity, C.status); break;
+    case TK_DEC_ATTWO: dec::task_attwo<T, D, DH>(C.dp, C.md, d.i0, local, step, smem, bar, parity, C.status); break;
     case TK_DEC_UPDN: dec::task_updn<T, D, DH>(C.dp, C.md, d.i0, local, smem, bar, parity, C.status); break;
-    case TK_DEC_HEAD: dec::task_head<T, D, DH>(C.dp, C.md, local, smem, bar, parity, C.status); break;
+    case TK_DEC_HEAD: dec::task_head<T, D, DH>(C.dp, C.md, local, step, smem, bar, parity, C.status); break;
     case TK_DEC_SAMPLE: dec::task_sample<T, D, DH>(C.dp, C.md, C.live, smem); break;
     default: break;
   }
@@ -418,7 +418,7 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
     }
     bool filled = false;
     if (job_id == 1) {                               // ---- serving: start the weight prefetch, THEN wait for the dependencies
-      filled = dec::prefetch<T, D, DH>(C.dp, C.md, d.kind, d.i0, local, smem, fill_bar);
+      filled = dec::prefetch<T, D, DH>(C.dp, C.md, d.kind, d.i0, local, step, smem, fill_bar);
       if (tid == 0) {
         int r2 = 0;
         if (!(step == rstep && ph == rph)) {
@@ -447,7 +447,7 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
       if (tid == 0) s_sel[7] = 0;
       run_train_task<T, D, DH>(C, d, ph, local, step, smem, gp, ap, bulk_uses, adam_tiles, ce_chunks, et);
     }
-    else run_decode_task<T, D, DH>(C, d, local, smem, fill_bar, fills & 1u);
+    else run_decode_task<T, D, DH>(C, d, local, step, smem, fill_bar, fills & 1u);
     if (filled) fills++;
     __syncthreads();
     {                                                // ask for the next phase's descriptor and scheduling record now

@@ -191,3 +191,34 @@ def test_tiny_fp32_decode_resumes_exactly_across_launches_beside_training(ofa, o
     want, _ = oracle.greedy_decode(ocfg, w0, prompt, len(got))
     assert got == want
     mk.close()
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f32"])
+def test_decode_attention_at_the_edges_of_its_rounds(ofa, oracle, kind):
+    """Positions around the edges of the attention task's split: its first row, a round of 32 (fp32: 64) keys and one more, four rounds, the
+    rows that fit in shared memory (256) and the ones read from global memory behind them. Launches end at these positions, so the block
+    has prefetched all, some or none of the rows; logits against one full-sequence forward. bf16: the module's bound. fp32: ten products
+    deep, each within k * 2^-24 of its exact value (k <= 256)."""
+    if kind == "bf16":
+        ocfg = oracle.OracleConfig(V=512, D=768, L=2, H=12, T=384, B=1, tied=False)
+        ends, bound = [1, 2, 32, 33, 34, 128, 129, 256, 257, 258, 290, 300], 3e-2
+    else:
+        ocfg = oracle.OracleConfig(V=80, D=64, L=2, H=4, T=96, B=1, tied=False)
+        ends, bound = [1, 2, 63, 64, 65, 66, 96], 10 * 256 * 2.0 ** -24
+    w = oracle.decode_test_weights(ocfg)
+    prompt = [int(t) for t in np.random.default_rng(11).integers(0, ocfg.V - 3, size=5)]
+    cfg = ofa.default_config("gpt_s" if kind == "bf16" else "tiny")
+    cfg.vocab, cfg.valid_vocab, cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode = ocfg.V, ocfg.V - 3, ocfg.L, ocfg.T, 1, ofa.capi.MODE_DECODE_ONLY
+    cfg.use_decode, cfg.n_prompt, cfg.answer_len, cfg.temperature, cfg.decode_out_cap = 1, len(prompt), 0, 0.0, 4096
+    for i, t in enumerate(prompt):
+        cfg.prompt[i] = t
+    mk = ofa.Megakernel(cfg)
+    mk.load_weights(oracle.flatten(ocfg, w))
+    got, done = [], 0
+    for e in ends:
+        mk.run(e - done, timeout_ms=60000); done = e
+        got.append(mk.decode_logits())
+    ref, _ = oracle.forward_with_kv(ocfg, w, fed_tokens(prompt, mk.decode_tokens(done), done), weights_bf16=kind == "bf16")
+    mk.close()
+    for e, lg in zip(ends, got):
+        assert relmax(lg, ref[e - 1].numpy()) <= bound, (e, relmax(lg, ref[e - 1].numpy()))
