@@ -226,29 +226,31 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
     uint32_t tc = gp.tile_count[W];
     bool ok = true;
     const int cg = lane & 3;
+    // An epilogue's code runs once per tile and has left the instruction caches by the block's next task of the kind (a step runs through
+    // hundreds of KB of task code), so straight-line code pays a fetch from L2 for every line of it: the passes over the columns are loops.
+    // One-tile tasks of K = 768, 128 columns unrolled -> loops: GELU' 25 -> 14 us, softmax partials 19 -> 11, row term 15 -> 11.5. `aux` is
+    // fetched a pass at a time; fetching it one pass ahead as well spilled, and with next to no L1 a spill goes to L2 (residual 9 -> 14 us).
     for (int t = 0; t < nt && ok; t++, tc++) {
       const int b = tc % CF::NBUF; const uint32_t use = tc / CF::NBUF;
       const int n0 = (tn0 + t) * BN;
-#pragma unroll
+#pragma unroll 1
       for (int half = 0; half < BN / 128; half++) {          // 128 columns at a time
-        // Epilogues that read `aux` (residual, pre-activation) fetch this thread's 16 row segments of the 128 columns BEFORE
-        // waiting for the accumulator, so the loads travel while the MMAs run instead of being 16 dependent round trips.
-        uint4 auxr[HAS_AUX_IN ? 16 : 1];
-        if constexpr (EPI == GE_DR) {                    // layout of the bf16-staged pass below: row = it*4 + lane/8, 8 columns at (lane%8)*8
-          const bf16* aux = reinterpret_cast<const bf16*>(g.aux);
+        const uint32_t tacc = gp.tmem_base + ((uint32_t)(e * 32) << 16) + (uint32_t)(b * BN + half * 128);
+        const int nh = n0 + half * 128;
+        // Epilogues that read `aux` (residual, pre-activation) fetch this thread's row segments of the first pass BEFORE waiting for the
+        // accumulator, so the loads travel while the MMAs run.
+        constexpr int NAUX = EPI == GE_DR ? 8 : 4;             // row segments of 8 columns per pass (64 columns for the staged pass, 32 otherwise)
+        uint4 auxr[HAS_AUX_IN ? NAUX : 1];
+        const bf16* auxp = nullptr;
+        if constexpr (EPI == GE_DR) auxp = reinterpret_cast<const bf16*>(g.aux) + (size_t)(m0 + e * 32 + (lane >> 3)) * g.ldaux + nh + (lane & 7) * 8;   // row = it*4 + lane/8
+        else if constexpr (HAS_AUX_IN) auxp = reinterpret_cast<const bf16*>(g.aux) + (size_t)(m0 + e * 32 + (lane >> 2)) * g.ldaux + nh + cg * 8;       // row = it*8 + lane/4
+        auto fetch_aux = [&](uint4 (&dst)[HAS_AUX_IN ? NAUX : 1], int col) {
+          if constexpr (HAS_AUX_IN) {
 #pragma unroll
-          for (int cp = 0; cp < 2; cp++)
-#pragma unroll
-            for (int it = 0; it < 8; it++)
-              auxr[cp * 8 + it] = *reinterpret_cast<const uint4*>(aux + (size_t)(m0 + e * 32 + it * 4 + (lane >> 3)) * g.ldaux + n0 + half * 128 + cp * 64 + (lane & 7) * 8);
-        } else if constexpr (HAS_AUX_IN) {
-          const bf16* aux = reinterpret_cast<const bf16*>(g.aux);
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int it = 0; it < 4; it++)
-              auxr[c * 4 + it] = *reinterpret_cast<const uint4*>(aux + (size_t)(m0 + e * 32 + it * 8 + (lane >> 2)) * g.ldaux + n0 + half * 128 + c * 32 + cg * 8);
-        }
+            for (int it = 0; it < NAUX; it++) dst[it] = *reinterpret_cast<const uint4*>(auxp + (size_t)(it * (32 / NAUX)) * g.ldaux + col);
+          }
+        };
+        fetch_aux(auxr, 0);
         if (half == 0) {
           if (!mbar_wait(bar_accf<BN>(base, b), use & 1, st)) { if (lane == 0 && !aborted(st)) raise_abort(st, ST_MBAR_ACC_TIMEOUT, phase_id, task, t); ok = false; }
           ok = __all_sync(0xffffffffu, ok);
@@ -262,131 +264,109 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
           // stores, half the shared-memory traffic of an fp32 transpose (the pipeline's own traffic nearly saturates it).
           unsigned char* sb = reinterpret_cast<unsigned char*>(stg);
           const int sub = lane >> 3, ch = lane & 7;
-          float lm[EPI == GE_LSE ? 8 : 1], ls[EPI == GE_LSE ? 8 : 1];   // GE_LSE: running maximum (log2 domain) and sum of 2^(x - max) per row slot
-#pragma unroll
-          for (int i = 0; i < (EPI == GE_LSE ? 8 : 1); i++) { lm[i] = -INFINITY; ls[i] = 0.f; }
-#pragma unroll
+          float lm = -INFINITY, ls = 0.f;                  // GE_LSE: maximum (log2 domain) and sum of 2^(x - max) of this thread's row so far
+#pragma unroll 1
           for (int cp = 0; cp < 2; cp++) {                 // 64 columns at a time
-#pragma unroll
+            if (EPI == GE_DR && cp == 1) fetch_aux(auxr, 64);
+#pragma unroll(EPI == GE_LSE ? 1 : 2)
             for (int hc = 0; hc < 2; hc++) {
-              uint32_t r[32];
-              tmem_ld32(gp.tmem_base + ((uint32_t)(e * 32) << 16) + (uint32_t)(b * BN + half * 128 + cp * 64 + hc * 32), r);
+              uint32_t r[32], pk[16];
+              tmem_ld32(tacc + (uint32_t)(cp * 64 + hc * 32), r);
               if (half == BN / 128 - 1 && cp == 1 && hc == 1) {    // all TMEM reads of this accumulator are done: hand it back early
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_acce<BN>(base, b));
               }
 #pragma unroll
-              for (int q = 0; q < 4; q++) {
-                uint4 v;
-                v.x = pack2f(__uint_as_float(r[8 * q]), __uint_as_float(r[8 * q + 1])); v.y = pack2f(__uint_as_float(r[8 * q + 2]), __uint_as_float(r[8 * q + 3]));
-                v.z = pack2f(__uint_as_float(r[8 * q + 4]), __uint_as_float(r[8 * q + 5])); v.w = pack2f(__uint_as_float(r[8 * q + 6]), __uint_as_float(r[8 * q + 7]));
-                *reinterpret_cast<uint4*>(sb + lane * 128 + (((hc * 4 + q) ^ (lane & 7)) << 4)) = v;
+              for (int q = 0; q < 16; q++) pk[q] = pack2f(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1]));
+#pragma unroll
+              for (int q = 0; q < 4; q++)
+                *reinterpret_cast<uint4*>(sb + lane * 128 + (((hc * 4 + q) ^ (lane & 7)) << 4)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+              if constexpr (EPI == GE_LSE) {               // over the STORED values, which are what cross-entropy will read
+                float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int q = 0; q < 16; q++) gm[q & 3] = fmaxf(gm[q & 3], fmaxf(__uint_as_float(pk[q] << 16), __uint_as_float(pk[q] & 0xffff0000u)));
+                const float cm = fmaxf(fmaxf(gm[0], gm[1]), fmaxf(gm[2], gm[3])) * 1.4426950408889634f;
+                if (cm > lm) { ls *= ex2_approx(lm - cm); lm = cm; }
+#pragma unroll
+                for (int q = 0; q < 16; q++)
+                  s4[q & 3] += ex2_approx(fmaf(__uint_as_float(pk[q] << 16), 1.4426950408889634f, -lm)) + ex2_approx(fmaf(__uint_as_float(pk[q] & 0xffff0000u), 1.4426950408889634f, -lm));
+                ls += (s4[0] + s4[1]) + (s4[2] + s4[3]);
               }
             }
             __syncwarp();
-            float drs[EPI == GE_DR ? 8 : 1];
-            // all eight reads first: a global store between two shared-memory reads keeps the compiler from moving the second
-            // read up (it cannot rule out aliasing), and the pass would pay eight shared-memory latencies in a row
-            uint4 ov[8];
-#pragma unroll
-            for (int it = 0; it < 8; it++) { const int rr = it * 4 + sub; ov[it] = *reinterpret_cast<const uint4*>(sb + rr * 128 + ((ch ^ (rr & 7)) << 4)); }
-#pragma unroll
-            for (int it = 0; it < 8; it++) {
-              const int rr = it * 4 + sub;
-              const uint4 out = ov[it];
-              const size_t row = (size_t)(m0 + e * 32 + rr);
-              const int col = n0 + half * 128 + cp * 64 + ch * 8;
-              if constexpr (EPI == GE_GELU) {
-                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.aux) + row * g.ldaux + col) = out;   // bf16-rounded pre-activation is what backward sees
+            const size_t row0 = (size_t)(m0 + e * 32 + sub);
+            const int col = nh + cp * 64 + ch * 8;
+            if constexpr (EPI == GE_GELU) {
+#pragma unroll 2
+              for (int it = 0; it < 8; it++) {
+                const int rr = it * 4 + sub;
+                const uint4 out = *reinterpret_cast<const uint4*>(sb + rr * 128 + ((ch ^ (rr & 7)) << 4));
+                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.aux) + (row0 + it * 4) * g.ldaux + col) = out;   // bf16-rounded pre-activation is what backward sees
                 float pv[8]; unpack8(out, pv);
 #pragma unroll
                 for (int i = 0; i < 8; i++) pv[i] = gelu_fwd<true>(pv[i]);
-                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.C) + row * g.ldc + col) = pack8(pv);
-              } else {
-                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.C) + row * g.ldc + col) = out;
+                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.C) + (row0 + it * 4) * g.ldc + col) = pack8(pv);
               }
-              if constexpr (EPI == GE_LSE) {
-                float y[8]; unpack8(out, y);               // the STORED values: the partials describe exactly what cross-entropy will read
-                float gm = y[0];
+            } else {
+              // all eight reads first: a global store between two shared-memory reads keeps the compiler from moving the second
+              // read up (it cannot rule out aliasing), and the pass would pay eight shared-memory latencies in a row
+              uint4 ov[8];
 #pragma unroll
-                for (int i = 1; i < 8; i++) gm = fmaxf(gm, y[i]);
-                gm *= 1.4426950408889634f;
-                if (gm > lm[it]) { ls[it] *= ex2_approx(lm[it] - gm); lm[it] = gm; }
-                float s2 = 0.f;
+              for (int it = 0; it < 8; it++) { const int rr = it * 4 + sub; ov[it] = *reinterpret_cast<const uint4*>(sb + rr * 128 + ((ch ^ (rr & 7)) << 4)); }
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) { ls[it] += ex2_approx(fmaf(y[i], 1.4426950408889634f, -lm[it])); s2 += ex2_approx(fmaf(y[i + 1], 1.4426950408889634f, -lm[it])); }
-                ls[it] += s2;
-              }
-              if constexpr (EPI == GE_DR) {
-                float c8[8], o8[8]; unpack8(out, c8); unpack8(auxr[cp * 8 + it], o8);
-                float sdot = 0.f;
+              for (int it = 0; it < 8; it++) *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(g.C) + (row0 + it * 4) * g.ldc + col) = ov[it];
+              if constexpr (EPI == GE_DR) {                // one pass = the 64 columns of one head; a row's share sits in 8 lanes
+                // the 128 rows of a tile belong to one sequence (the context length is a multiple of 128): one division per tile
+                const int bseq = m0 / g.dr_T, t0 = m0 - bseq * g.dr_T + e * 32 + sub;
+                float* drow = g.dr + ((size_t)bseq * g.dr_H + nh / 64 + cp) * g.dr_T + t0;
 #pragma unroll
-                for (int i = 0; i < 8; i++) sdot = fmaf(c8[i], o8[i], sdot);
-                drs[it] = sdot;
-              }
-            }
-            if constexpr (EPI == GE_DR) {                  // one pass = the 64 columns of one head; a row's share sits in 8 lanes
-              // the 128 rows of a tile belong to one sequence (the context length is a multiple of 128): one division per tile
-              const int bseq = m0 / g.dr_T, t0 = m0 - bseq * g.dr_T + e * 32 + sub;
-              float* drow = g.dr + ((size_t)bseq * g.dr_H + (n0 + half * 128) / 64 + cp) * g.dr_T + t0;
+                for (int it = 0; it < 8; it++) {
+                  float c8[8], o8[8]; unpack8(ov[it], c8); unpack8(auxr[it], o8);
+                  float v = 0.f;
 #pragma unroll
-              for (int it = 0; it < 8; it++) {
-                float v = drs[it];
-                v += __shfl_xor_sync(0xffffffffu, v, 1); v += __shfl_xor_sync(0xffffffffu, v, 2); v += __shfl_xor_sync(0xffffffffu, v, 4);
-                if (ch == 0) drow[it * 4] = v;
+                  for (int i = 0; i < 8; i++) v = fmaf(c8[i], o8[i], v);
+                  v += __shfl_xor_sync(0xffffffffu, v, 1); v += __shfl_xor_sync(0xffffffffu, v, 2); v += __shfl_xor_sync(0xffffffffu, v, 4);
+                  if (ch == 0) drow[it * 4] = v;
+                }
               }
             }
             __syncwarp();
           }
-          if constexpr (EPI == GE_LSE) {                   // a row's 128 columns sit in 8 lanes: merge their (max, sum) pairs, same result in all eight
-            float2* part = reinterpret_cast<float2*>(g.dr) + (size_t)(m0 + e * 32 + sub) * (g.N / 128) + (n0 + half * 128) / 128;
-#pragma unroll
-            for (int it = 0; it < 8; it++) {
-              float m_ = lm[it], s_ = ls[it];
-#pragma unroll
-              for (int o = 1; o <= 4; o <<= 1) {
-                const float mo = __shfl_xor_sync(0xffffffffu, m_, o), so = __shfl_xor_sync(0xffffffffu, s_, o);
-                const float mn = fmaxf(m_, mo);
-                s_ = s_ * ex2_approx(m_ - mn) + so * ex2_approx(mo - mn);
-                m_ = mn;
-              }
-              if (ch == 0) part[(size_t)it * 4 * (g.N / 128)] = make_float2(m_, s_);
-            }
-          }
+          if constexpr (EPI == GE_LSE) reinterpret_cast<float2*>(g.dr)[(size_t)(m0 + e * 32 + lane) * (g.N / 128) + nh / 128] = make_float2(lm, ls);
         } else {
+#pragma unroll 1
+          for (int c = 0; c < 4; c++) {
+            if (c > 0) fetch_aux(auxr, c * 32);
+            uint32_t r[32];
+            tmem_ld32(tacc + (uint32_t)(c * 32), r);
+            if (half == BN / 128 - 1 && c == 3) {    // all TMEM reads of this accumulator are done: hand it back early
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar_acce<BN>(base, b));
+            }
+            // thread = row `lane` of the 32x32 block; 16-byte chunk j goes to position j ^ (lane & 7)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-          uint32_t r[32];
-          tmem_ld32(gp.tmem_base + ((uint32_t)(e * 32) << 16) + (uint32_t)(b * BN + half * 128 + c * 32), r);
-          if (half == BN / 128 - 1 && c == 3) {    // all TMEM reads of this accumulator are done: hand it back early
-            tc_fence_before();
+            for (int j = 0; j < 8; j++)
+              *reinterpret_cast<float4*>(stg + lane * 32 + ((j ^ (lane & 7)) << 2)) =
+                  make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_acce<BN>(base, b));
-          }
-          // thread = row `lane` of the 32x32 block; 16-byte chunk j goes to position j ^ (lane & 7)
+            // 8 rows per instruction: lane -> (row = it*8 + lane/4, 8 consecutive columns (lane%4)*8..)
+            float4 av[8];                            // all reads before the first global store (see the bf16-staged pass)
 #pragma unroll
-          for (int j = 0; j < 8; j++)
-            *reinterpret_cast<float4*>(stg + lane * 32 + ((j ^ (lane & 7)) << 2)) =
-                make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-          __syncwarp();
-          // 8 rows per instruction: lane -> (row = it*8 + lane/4, 8 consecutive columns (lane%4)*8..)
-          float4 av[8];                            // all reads before the first global store (see the bf16-staged pass)
+            for (int it = 0; it < 4; it++) {
+              const int rr = it * 8 + (lane >> 2);
+              av[2 * it] = *reinterpret_cast<const float4*>(stg + rr * 32 + (((2 * cg) ^ (rr & 7)) << 2));
+              av[2 * it + 1] = *reinterpret_cast<const float4*>(stg + rr * 32 + (((2 * cg + 1) ^ (rr & 7)) << 2));
+            }
 #pragma unroll
-          for (int it = 0; it < 4; it++) {
-            const int rr = it * 8 + (lane >> 2);
-            av[2 * it] = *reinterpret_cast<const float4*>(stg + rr * 32 + (((2 * cg) ^ (rr & 7)) << 2));
-            av[2 * it + 1] = *reinterpret_cast<const float4*>(stg + rr * 32 + (((2 * cg + 1) ^ (rr & 7)) << 2));
+            for (int it = 0; it < 4; it++) {
+              const float4 a0 = av[2 * it], a1 = av[2 * it + 1];
+              const float acc[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+              epi_store8<EPI>(g, (size_t)(m0 + e * 32 + it * 8 + (lane >> 2)), nh + c * 32 + cg * 8, acc, auxr[HAS_AUX_IN ? it : 0]);
+            }
+            __syncwarp();
           }
-#pragma unroll
-          for (int it = 0; it < 4; it++) {
-            const int rr = it * 8 + (lane >> 2);
-            const float4 a0 = av[2 * it], a1 = av[2 * it + 1];
-            const float acc[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            epi_store8<EPI>(g, (size_t)(m0 + e * 32 + rr), n0 + half * 128 + c * 32 + cg * 8, acc, auxr[HAS_AUX_IN ? c * 4 + it : 0]);
-          }
-          __syncwarp();
-        }
         }
       }
     }
