@@ -110,8 +110,8 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
                             (const float*)d.p[5], (const T*)d.p[6], (const T*)d.p[7], md.N, smem);
       break;
     case TK_LN_DG:
-      if (d.i1) ew::ln_dgamma_reduce_task<bf16>(local, (bf16*)d.p[0], (const float*)d.p[1], (md.N + ew::ROWS_PER_TASK - 1) / ew::ROWS_PER_TASK, D, d.i0);
-      else ew::ln_dgamma_reduce_task<float>(local, (float*)d.p[0], (const float*)d.p[1], (md.N + ew::ROWS_PER_TASK - 1) / ew::ROWS_PER_TASK, D, d.i0);
+      if (d.i1) ew::ln_dgamma_reduce_task<bf16>(local, (bf16*)d.p[0], (const float*)d.p[1], (md.N + ew::ROWS_PER_TASK - 1) / ew::ROWS_PER_TASK, D, d.i0, smem);
+      else ew::ln_dgamma_reduce_task<float>(local, (float*)d.p[0], (const float*)d.p[1], (md.N + ew::ROWS_PER_TASK - 1) / ew::ROWS_PER_TASK, D, d.i0, smem);
       break;
     case TK_EMB_WTE:
       if (d.i1) ew::embed_bwd_wte_task<T, D, bf16>(local, (bf16*)d.p[0], (const T*)d.p[1], (const int*)d.p[2], md.N, md.V, d.tiles_m, d.i0, smem);

