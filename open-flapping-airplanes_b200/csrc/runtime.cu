@@ -1180,6 +1180,13 @@ extern "C" int ofa_load_adam_state(ofa_ctx* c, const float* mm, const float* vv,
   return OFA_OK;
 }
 
+// The source has been read when this returns: from page-locked memory the copy runs beside the host, and a caller that refills its
+// buffer would hand the device words that were never checked.
+static int upload(ofa_ctx* c, void* dst, const void* src, size_t bytes) {
+  if (cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
+    return fail(c, OFA_CUDA_ERROR, std::string("H2D failed: ") + cudaGetErrorString(cudaGetLastError()));
+  return OFA_OK;
+}
 extern "C" int ofa_set_tokens(ofa_ctx* c, const uint32_t* tokens, size_t n) {
   if (c && c->dry) return fail(c, OFA_BAD_ARGUMENT, "planning context (device < 0) has no device memory");
   if (!c || !tokens || n < (size_t)c->md.T + 2) return fail(c, OFA_BAD_ARGUMENT, "need more than ctx_len + 1 tokens");
@@ -1194,7 +1201,7 @@ extern "C" int ofa_set_tokens(ofa_ctx* c, const uint32_t* tokens, size_t n) {
   }
   c->ntok = n;
   c->nstarts = 0;                                   // a starts table was validated against the old stream: it has to be set again
-  return cudaMemcpyAsync(c->d_tokens, tokens, n * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
+  return upload(c, c->d_tokens, tokens, n * 4);
 }
 extern "C" int ofa_set_starts(ofa_ctx* c, const uint32_t* starts, size_t nsteps) {
   if (!c) return OFA_BAD_ARGUMENT;
@@ -1211,7 +1218,7 @@ extern "C" int ofa_set_starts(ofa_ctx* c, const uint32_t* starts, size_t nsteps)
     c->starts_cap = n;
   }
   c->nstarts = (int)nsteps;
-  return cudaMemcpyAsync(c->d_starts, starts, n * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, "H2D failed");
+  return upload(c, c->d_starts, starts, n * 4);
 }
 
 extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
