@@ -366,6 +366,7 @@ struct ofa_ctx {
   int* d_ext_ready = nullptr; int* d_ext_done = nullptr;   // device flags [32] each: gradients of bucket b ready / all-reduce of bucket b done
   std::vector<Span> buckets;
   cudaStream_t stream = nullptr, abort_stream = nullptr; cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;   // start, end of the kernel, results copied back
+  cudaEvent_t ev_host = nullptr;     // what the caller has queued on the default stream
   bool dry = false;
   int step_done_cap = 0; size_t starts_cap = 0, tokens_cap = 0;
   bool abort_requested = false;      // ofa_abort was called for the launch in flight (also honoured if the device word was cleared by a launch that had not started yet)
@@ -940,11 +941,24 @@ cudaError_t read_back(int device, cudaStream_t stream, const void* src, void* ou
   return (cudaError_t)err.load();
 }
 
+// The context's stream does not wait for the default stream by itself, but hosts reach the gradients through ofa_grad_buffer and
+// work on them there: what they have queued before a call comes before what the call does.
+cudaError_t follow_default_stream(ofa_ctx* c) {
+  cudaError_t e = cudaSetDevice(c->device);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev_host, cudaStreamLegacy);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_host, 0);
+  return e;
+}
+cudaError_t read_ctx(ofa_ctx* c, const void* src, void* out, size_t bytes, bool widen) {
+  const cudaError_t e = follow_default_stream(c);
+  return e == cudaSuccess ? read_back(c->device, c->stream, src, out, bytes, widen) : e;
+}
+
 int read_f32(ofa_ctx* c, const float* src, float* out, size_t n) {
   if (c && c->dry) return fail(c, OFA_BAD_ARGUMENT, "planning context (device < 0) has no device memory");
   if (!c || !out || n > c->lay.total) return fail(c, OFA_BAD_ARGUMENT, "bad size");
   if (c->in_flight) return fail(c, OFA_BAD_ARGUMENT, "launch in flight: call ofa_wait first");
-  const cudaError_t e = read_back(c->device, c->stream, src, out, n * sizeof(float), false);
+  const cudaError_t e = read_ctx(c, src, out, n * sizeof(float), false);
   return e == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, cudaGetErrorString(e));
 }
 
@@ -1011,6 +1025,7 @@ extern "C" void ofa_destroy(ofa_ctx* c) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->ev2) cudaEventDestroy(c->ev2);
+  if (c->ev_host) cudaEventDestroy(c->ev_host);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->abort_stream) cudaStreamDestroy(c->abort_stream);
   delete c;
@@ -1062,7 +1077,7 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   }
   if (!dry) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(OFA_CUDA_ERROR, "stream");
-    cudaEventCreate(&c->ev0); cudaEventCreate(&c->ev1); cudaEventCreateWithFlags(&c->ev2, cudaEventDisableTiming);
+    cudaEventCreate(&c->ev0); cudaEventCreate(&c->ev1); cudaEventCreateWithFlags(&c->ev2, cudaEventDisableTiming); cudaEventCreateWithFlags(&c->ev_host, cudaEventDisableTiming);
     c->ar.stream = c->stream;
   }
   // SM split
@@ -1165,7 +1180,7 @@ extern "C" int ofa_read_grads(ofa_ctx* c, float* out, size_t n) {
   if (c->dry) return fail(c, OFA_BAD_ARGUMENT, "planning context (device < 0) has no device memory");
   if (!out || n > c->lay.total) return fail(c, OFA_BAD_ARGUMENT, "bad size");
   if (c->in_flight) return fail(c, OFA_BAD_ARGUMENT, "launch in flight: call ofa_wait first");
-  const cudaError_t e = read_back(c->device, c->stream, c->Gbf, out, n * sizeof(bf16), true);
+  const cudaError_t e = read_ctx(c, c->Gbf, out, n * sizeof(bf16), true);
   return e == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, cudaGetErrorString(e));
 }
 extern "C" int ofa_load_adam_state(ofa_ctx* c, const float* mm, const float* vv, size_t n, int step_base) {
@@ -1426,7 +1441,7 @@ static int read_named(ofa_ctx* c, const char* name, void* out, size_t bytes, boo
   if (it == c->bufs.end()) return fail(c, OFA_BAD_ARGUMENT, std::string("no buffer named ") + name);
   if (bytes > it->second.second) return fail(c, OFA_BAD_ARGUMENT, "buffer is smaller than requested");
   if (c->dry) return fail(c, OFA_CUDA_ERROR, "planning context (device < 0) has no device memory");
-  const cudaError_t e = read_back(c->device, c->stream, it->second.first, out, bytes, widen);
+  const cudaError_t e = read_ctx(c, it->second.first, out, bytes, widen);
   return e == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, std::string("D2H failed: ") + cudaGetErrorString(e));
 }
 extern "C" int ofa_read_buffer(ofa_ctx* c, const char* name, void* out, size_t bytes) { return read_named(c, name, out, bytes, false); }

@@ -1,4 +1,5 @@
-"""What the host calls promise beside their results, on the GPU through the C ABI: a call has read its host buffers when it returns."""
+"""What the host calls promise beside their results, on the GPU through the C ABI: a call has read its host buffers when it returns, and
+comes behind work that the caller queued on the default stream."""
 import numpy as np
 import pytest
 import torch
@@ -60,4 +61,39 @@ def test_starts_have_been_read_when_the_call_returns(ofa):
     st[-1] = 7 + np.arange(B) * 300
     mk.run(1)
     np.testing.assert_array_equal(mk.read_buffer("logits", (N, 65), np.float32), ref)
+    mk.close()
+
+
+class _View:
+    def __init__(self, ptr, n, typestr):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": typestr, "data": (int(ptr), False), "version": 2}
+
+
+def grads_of(mk, bf16):
+    v = torch.as_tensor(_View(mk.grad_buffer_ptr(), mk.num_params, "<i2" if bf16 else "<f4"), device="cuda")
+    return v.view(torch.bfloat16) if bf16 else v
+
+
+def small_bf16(ofa, mode, grad_bf16=0):
+    cfg = ofa.default_config("gpt_s")
+    cfg.vocab = cfg.valid_vocab = 512
+    cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode, cfg.grad_bf16 = 1, 128, 1, mode, grad_bf16
+    mk = ofa.Megakernel(cfg)
+    g = torch.Generator().manual_seed(8)
+    mk.load_weights(torch.randn(mk.num_params, generator=g).mul_(0.02).numpy())
+    return mk
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_reads_are_ordered_behind_the_default_stream(ofa, bf16):
+    """A host that scales the gradients through ofa_grad_buffer on the default stream reads the scaled ones."""
+    mk = small_bf16(ofa, ofa.capi.MODE_NO_OPT, 1) if bf16 else tiny(ofa, ofa.capi.MODE_NO_OPT)
+    mk.set_tokens(np.random.default_rng(3).integers(0, 65, 1 << 13, dtype=np.uint32))
+    mk.run(1)
+    before = mk.read_grads()
+    g = grads_of(mk, bf16)
+    torch.cuda._sleep(1000); g.mul_(1.0); torch.cuda.synchronize()       # both kernels are loaded: neither call below waits for the device
+    torch.cuda._sleep(200_000_000)                   # about 0.1 s on the default stream
+    g.mul_(2.0)
+    np.testing.assert_array_equal(mk.read_grads(), 2.0 * before)
     mk.close()
