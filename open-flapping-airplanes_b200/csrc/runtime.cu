@@ -1242,7 +1242,10 @@ extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
   if (c->in_flight) return fail(c, OFA_BAD_ARGUMENT, "previous launch still in flight: call ofa_wait");
   const bool train_on = c->C.train_sms > 0;
   if (train_on && (!c->d_tokens || c->ntok < (size_t)c->md.T + 2)) return fail(c, OFA_BAD_ARGUMENT, "no tokens set");
-  cudaSetDevice(c->device);
+  {  // a gradient buffer cleared or read on the default stream is not overwritten under it
+    const cudaError_t e = follow_default_stream(c);
+    if (e != cudaSuccess) return fail(c, OFA_CUDA_ERROR, std::string("default stream: ") + cudaGetErrorString(e));
+  }
   if (c->jobs_seed != g_task_shuffle_seed && !place_jobs(c)) return fail(c, OFA_BAD_CONFIG, c->err);
   Ctx& C = c->C;
   if (train_on) {

@@ -97,3 +97,20 @@ def test_reads_are_ordered_behind_the_default_stream(ofa, bf16):
     g.mul_(2.0)
     np.testing.assert_array_equal(mk.read_grads(), 2.0 * before)
     mk.close()
+
+
+def test_launches_are_ordered_behind_the_default_stream(ofa):
+    """Gradients cleared on the default stream before a launch are cleared before it, not after its backward pass."""
+    mk = tiny(ofa, ofa.capi.MODE_NO_OPT)
+    mk.set_tokens(np.random.default_rng(4).integers(0, 65, 1 << 13, dtype=np.uint32))
+    mk.set_starts(np.arange(mk.cfg.batch, dtype=np.uint32)[None, :] * 100)
+    mk.run(1)
+    before = mk.read_grads()
+    g = grads_of(mk, False)
+    torch.cuda._sleep(1000); g.zero_(); torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)
+    g.zero_()
+    mk.run(1)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(mk.read_grads(), before)
+    mk.close()
