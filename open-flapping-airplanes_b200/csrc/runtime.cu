@@ -888,41 +888,57 @@ bool probe_smids(ofa_ctx* c) {
 
 // Device -> pageable host memory, optionally widening bf16 to fp32 on the way. The copy engine fills pinned slots and host threads
 // move (and widen) them into the caller's buffer, whose pages they usually touch for the first time: one thread alone spends longer on
-// those page faults than the copy takes (12.9M logits of an evaluation: 20 ms with a pageable copy and a conversion by the caller,
-// 1.5 ms here). Slots and threads: 2 MB each, at most eight, and never more than there are pieces of 2 MB. The slots are shared by all
-// contexts of the process; a second caller waits for the first.
-constexpr size_t READ_SLOT = 2u << 20; constexpr int READ_SLOTS = 8;
+// those page faults than the copy takes (12.9M logits of an evaluation: 19 ms with a pageable copy and a conversion by the caller,
+// 2.5 ms here). Slots and threads: 2 MB each, at most eight, and never more than there are pieces of 2 MB. The slots of a device are shared by
+// its contexts; a second caller waits for the first. They are made one at a time and kept: growing one allocation would free the old
+// one, and that can wait for a launch of another context. Where a slot or a thread cannot be had, the read goes on with those there are.
+constexpr size_t READ_SLOT = 2u << 20; constexpr int READ_SLOTS = 8, READ_DEVICES = 64;
 struct ReadSlots {
-  std::mutex mu; unsigned char* p = nullptr; int n = 0;
-  bool need(int k) {                     // with mu held
-    if (n >= k) return true;
-    if (p) cudaFreeHost(p);
-    p = nullptr; n = 0;
-    if (cudaHostAlloc(&p, READ_SLOT * k, cudaHostAllocPortable) != cudaSuccess) { p = nullptr; return false; }
-    n = k;
-    return true;
+  std::mutex mu; unsigned char* p[READ_SLOTS] = {};
+  int have(int want) {                   // with mu held: the number of slots there are, at most `want`
+    int n = 0;
+    while (n < want && (p[n] || cudaHostAlloc(&p[n], READ_SLOT, cudaHostAllocPortable) == cudaSuccess)) n++;
+    if (n < want) { p[n] = nullptr; cudaGetLastError(); }
+    return n;
   }
-  ~ReadSlots() { if (p) cudaFreeHost(p); }
 };
-ReadSlots g_read_slots;
+ReadSlots* read_slots() { static ReadSlots* const s = new ReadSlots[READ_DEVICES]; return s; }      // never destroyed: the driver may be gone before a destructor runs
 void widen_bf16(const uint16_t* src, float* dst, size_t n) {
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
   for (size_t i = 0; i < n; i++) d[i] = (uint32_t)src[i] << 16;
 }
+// without pinned memory: bf16 words land in the upper half of the caller's buffer and are widened from its start, a block at a time
+cudaError_t read_pageable(cudaStream_t stream, const void* src, void* out, size_t bytes, bool widen) {
+  char* raw = static_cast<char*>(out) + (widen ? bytes : 0);
+  cudaError_t e = cudaMemcpyAsync(raw, src, bytes, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess || !widen) return e;
+  uint16_t block[1024];
+  for (size_t i = 0, n = bytes / 2; i < n; i += 1024) {
+    const size_t m = std::min<size_t>(1024, n - i);
+    memcpy(block, raw + 2 * i, 2 * m);
+    widen_bf16(block, static_cast<float*>(out) + i, m);
+  }
+  return e;
+}
+// the caller has made `device` current
 cudaError_t read_back(int device, cudaStream_t stream, const void* src, void* out, size_t bytes, bool widen) {
   if (bytes == 0) return cudaSuccess;
+  if (device >= READ_DEVICES) return read_pageable(stream, src, out, bytes, widen);
   const size_t pieces = (bytes + READ_SLOT - 1) / READ_SLOT;
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
-  const int nt = (int)std::min<size_t>(pieces, (size_t)std::min(READ_SLOTS, std::max(1, cores / 2)));
-  std::lock_guard<std::mutex> lk(g_read_slots.mu);
-  if (!g_read_slots.need(nt)) return cudaErrorMemoryAllocation;
+  ReadSlots& slots = read_slots()[device];
+  std::lock_guard<std::mutex> lk(slots.mu);
+  const int nt = slots.have((int)std::min<size_t>(pieces, (size_t)std::min(READ_SLOTS, std::max(1, cores / 2))));
+  if (nt == 0) return read_pageable(stream, src, out, bytes, widen);
+  std::atomic<size_t> next{0};
   std::atomic<int> err{(int)cudaSuccess};
   auto work = [&](int t) {
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    unsigned char* slot = g_read_slots.p + READ_SLOT * t;
-    for (size_t k = t; k < pieces && e == cudaSuccess; k += nt) {
+    unsigned char* slot = slots.p[t];
+    for (size_t k; e == cudaSuccess && (k = next.fetch_add(1)) < pieces;) {
       const size_t off = k * READ_SLOT, nb = std::min(READ_SLOT, bytes - off);
       e = cudaMemcpyAsync(slot, static_cast<const char*>(src) + off, nb, cudaMemcpyDeviceToHost, stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev, stream);
@@ -934,10 +950,12 @@ cudaError_t read_back(int device, cudaStream_t stream, const void* src, void* ou
     if (ev) cudaEventDestroy(ev);
     if (e != cudaSuccess) err.store((int)e);
   };
-  std::vector<std::thread> th;
-  for (int t = 1; t < nt; t++) th.emplace_back(work, t);
+  std::thread th[READ_SLOTS];
+  for (int t = 1; t < nt; t++) {
+    try { th[t] = std::thread(work, t); } catch (...) { break; }        // no exception leaves a C entry
+  }
   work(0);
-  for (std::thread& x : th) x.join();
+  for (std::thread& x : th) if (x.joinable()) x.join();
   return (cudaError_t)err.load();
 }
 
@@ -1448,7 +1466,10 @@ static int read_named(ofa_ctx* c, const char* name, void* out, size_t bytes, boo
   return e == cudaSuccess ? OFA_OK : fail(c, OFA_CUDA_ERROR, std::string("D2H failed: ") + cudaGetErrorString(e));
 }
 extern "C" int ofa_read_buffer(ofa_ctx* c, const char* name, void* out, size_t bytes) { return read_named(c, name, out, bytes, false); }
-extern "C" int ofa_read_buffer_bf16(ofa_ctx* c, const char* name, float* out, size_t n) { return read_named(c, name, out, n * sizeof(bf16), true); }
+extern "C" int ofa_read_buffer_bf16(ofa_ctx* c, const char* name, float* out, size_t n) {
+  if (n > SIZE_MAX / sizeof(bf16)) return c ? fail(c, OFA_BAD_ARGUMENT, "buffer is smaller than requested") : OFA_BAD_ARGUMENT;
+  return read_named(c, name, out, n * sizeof(bf16), true);
+}
 
 // ================================================================================================ C ABI: task level
 extern "C" int ofa_dev_alloc(void** p, size_t bytes) {

@@ -1,10 +1,18 @@
 """What the host calls promise beside their results, on the GPU through the C ABI: a call has read its host buffers when it returns, and
-comes behind work that the caller queued on the default stream."""
+comes behind work that the caller queued on the default stream; reads work from several threads and where no thread can be started."""
+import ctypes as C
+import os
+import subprocess
+import sys
+import threading
+
 import numpy as np
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def pinned(n):
@@ -114,3 +122,87 @@ def test_launches_are_ordered_behind_the_default_stream(ofa):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(mk.read_grads(), before)
     mk.close()
+
+
+def test_read_buffers_of_any_length_from_two_threads(ofa):
+    """Lengths around the pieces a read is cut into (2 MB), odd counts among them, two contexts read at the same time."""
+    SLOT = 2 << 20
+    cases = []
+    for seed in (1, 2):
+        cfg = ofa.default_config("gpt_s")
+        cfg.vocab = cfg.valid_vocab = 50304
+        cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode = 1, 128, 2, ofa.capi.MODE_FORWARD
+        mk = ofa.Megakernel(cfg)
+        g = torch.Generator().manual_seed(seed)
+        w = torch.randn(mk.num_params, generator=g).mul_(0.02).numpy()
+        mk.load_weights(w)
+        mk.set_tokens(np.random.default_rng(seed).integers(0, 50304, 1 << 13, dtype=np.uint32))
+        mk.run(1)
+        cases.append((mk, w, mk.read_buffer("logits", (256 * 50304,), np.uint16)))
+    errors = []
+
+    def check(mk, w, bits):
+        try:
+            for n in (1, 3, SLOT // 2 - 1, SLOT // 2, SLOT // 2 + 1, 8 * SLOT // 2 + 5, 256 * 50304 - 1, 256 * 50304):
+                wide = mk.read_buffer("logits", (n,), "bf16")
+                np.testing.assert_array_equal(wide.view(np.uint32), bits[:n].astype(np.uint32) << 16)
+                np.testing.assert_array_equal(mk.read_buffer("logits", (n,), np.uint16), bits[:n])
+            for n in (1, SLOT // 4 + 1, mk.num_params - 3, mk.num_params):
+                np.testing.assert_array_equal(mk._read(mk.lib.ofa_read_weights, n), w[:n])
+        except BaseException as e:                   # shown by the test's own thread below
+            errors.append(e)
+
+    ts = [threading.Thread(target=check, args=c) for c in cases]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors[0]
+    out = np.empty(4, np.float32)
+    assert cases[0][0].lib.ofa_read_buffer_bf16(cases[0][0].h, b"logits", out.ctypes.data_as(C.c_void_p), (1 << 63) + 2) == ofa.capi.BAD_ARGUMENT
+    for mk, _, _ in cases:
+        mk.close()
+
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
+int refuse_threads = 0;
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) {
+  static int (*real)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*) = 0;
+  if (refuse_threads) return EAGAIN;
+  if (!real) real = (int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*))dlsym(RTLD_NEXT, "pthread_create");
+  return real(t, a, f, x);
+}
+"""
+
+
+NO_THREADS = r"""
+import ctypes, importlib, sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+ofa = importlib.import_module("open-flapping-airplanes_b200")
+cfg = ofa.default_config("gpt_s")
+cfg.vocab = cfg.valid_vocab = 8192
+cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode = 1, 128, 1, ofa.capi.MODE_FORWARD
+mk = ofa.Megakernel(cfg)
+w = torch.randn(mk.num_params, generator=torch.Generator().manual_seed(1)).mul_(0.02).numpy()
+mk.load_weights(w)
+flag = ctypes.c_int.in_dll(ctypes.CDLL(None), "refuse_threads")
+flag.value = 1
+got = mk.read_weights()
+flag.value = 0
+assert np.array_equal(got, w)
+print("READ")
+"""
+
+
+def test_reads_work_where_no_thread_can_be_started(ofa, tmp_path):
+    """pthread_create is replaced by one that fails, in a process of its own: no exception leaves the C entry, the weights arrive."""
+    src, so, prog = tmp_path / "shim.c", tmp_path / "shim.so", tmp_path / "prog.py"
+    src.write_text(SHIM); prog.write_text(NO_THREADS)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(so), str(src), "-ldl"], check=True)
+    r = subprocess.run([sys.executable, str(prog), ROOT], env=dict(os.environ, LD_PRELOAD=str(so)), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "READ" in r.stdout, (r.returncode, r.stdout[-500:], r.stderr[-2000:])
