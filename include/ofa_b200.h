@@ -195,6 +195,9 @@ int ofa_d2h(void* dst, const void* src, size_t bytes);
  * = {lr, beta1, beta2, eps, wd, grad_scale} with optimizer step r+1. */
 int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* phases, int nph, int repeats, const float* adam,
                    float* ms, ofa_status_t* status);
+/* What calls keep between them is bounded - per GPU four workspaces of ofa_run_phases of at most 4 MB each, and 16 MB of pinned memory through
+ * which buffers are read - and given back here. Other threads may be inside calls meanwhile; what they use stays. */
+int ofa_release_caches(void);
 /* Test hook: with seed != 0 every phase uploaded afterwards (by ofa_launch or ofa_run_phases, training and serving graphs) hands
  * its tasks out in a pseudo-randomly permuted order; 0 restores the natural order. Every result must be bit-identical either
  * way: the reference checks its task libraries the same way (llm/gemm/test_gemm.cu:20-49, llm/attention/test_attention.cu:45-77,

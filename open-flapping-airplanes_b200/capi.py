@@ -101,6 +101,7 @@ PROTOTYPES = {
     "ofa_noalloc_max_rows": (C.c_int, []),
     "ofa_noalloc_last_error": (C.c_char_p, []),
     "ofa_debug_set_task_shuffle": (None, [C.c_uint]),
+    "ofa_release_caches": (C.c_int, []),
     "ofa_run_phases": (C.c_int, [C.c_int, C.POINTER(Dims), C.POINTER(Phase), C.c_int, C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(Status)]),
 }
 

@@ -84,6 +84,21 @@ EncodeFn get_encode() {
   }
   return enc;
 }
+// Identity of the current CUDA context, 0 if the driver cannot tell. What is kept between calls is only good in the context it was made in:
+// a device reset ends it and frees everything in it.
+unsigned long long context_id() {
+  typedef CUresult (*IdFn)(CUcontext, unsigned long long*);
+  static const IdFn fn = [] {
+    void* f = nullptr; cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess ? (IdFn)f : (IdFn) nullptr;
+  }();
+  unsigned long long id = 0;
+  cudaFree(nullptr);                     // the context exists now
+  return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+constexpr int MAX_SMEM = 227 * 1024;     // dynamic shared memory of a block, largest opt-in size of sm_100
+constexpr int KEPT_DEVICES = 64;         // devices for which memory is kept between calls
+
 // 2-D tensor map: `inner` contiguous elements, `outer` rows of `ld` elements, box {box_inner, box_outer}. GEMM operands are
 // bf16 with SWIZZLE_128B; the serving job's weight prefetch uses plain (unswizzled) views in the activation type.
 bool encode_map(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer,
@@ -285,21 +300,14 @@ void fill_param_records(Ctx& C, const HostJob* train, const HostJob* dec) {
   if (dec && dec->nph > 0 && dec->nph <= PARAM_DEC_PH) { memcpy(C.dec_rec, dec->rec.data(), sizeof(SchedRec) * dec->nph); C.dec_rec_n = dec->nph; }
 }
 
-template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nblocks, int smem, int device, cudaStream_t s) {
-  static std::atomic<int> allowed[64];     // per device: the largest dynamic shared memory the kernel has been allowed so far
-  std::atomic<int>* a = device >= 0 && device < 64 ? &allowed[device] : nullptr;
-  if (!a || a->load(std::memory_order_acquire) < smem) {
-    static std::mutex mu;                  // two threads must not lower the limit below what the other just raised it to
-    std::lock_guard<std::mutex> lk(mu);
-    if (!a || a->load(std::memory_order_relaxed) < smem) {
-      cudaError_t e = cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
-      // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
-      cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      if (a) a->store(smem, std::memory_order_release);
-    }
-  }
+// The limit is always the device's (227 KB), whatever this launch needs: two threads cannot lower it under each other, and nothing has to
+// be remembered between launches (a device reset would make it untrue). The two calls take 0.2 us together.
+template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nblocks, int smem, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+  if (e != cudaSuccess) return e;
+  // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
+  // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
+  cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   ofa_kernel<T, D, DH><<<nblocks, NTHR, smem, s>>>(C);
   return cudaGetLastError();
 }
@@ -317,7 +325,7 @@ std::string smem_fit_error(bool bf, int Tctx, int N, bool emb_wte, bool decode, 
       return "ctx_len " + std::to_string(Tctx) + ": the serving tasks need " + std::to_string(dec::smem_bytes<bf16, 768, 64>(Tctx)) + " B of shared memory, the block has " + std::to_string(room);
     return "";
   }
-  if (smem > 227 * 1024) return "the fp32 path would need " + std::to_string(smem) + " B of shared memory per block (limit 232,448)";
+  if (smem > MAX_SMEM) return "the fp32 path would need " + std::to_string(smem) + " B of shared memory per block (limit 232,448)";
   return "";
 }
 
@@ -892,17 +900,23 @@ bool probe_smids(ofa_ctx* c) {
 // 2.5 ms here). Slots and threads: 2 MB each, at most eight, and never more than there are pieces of 2 MB. The slots of a device are shared by
 // its contexts; a second caller waits for the first. They are made one at a time and kept: growing one allocation would free the old
 // one, and that can wait for a launch of another context. Where a slot or a thread cannot be had, the read goes on with those there are.
-constexpr size_t READ_SLOT = 2u << 20; constexpr int READ_SLOTS = 8, READ_DEVICES = 64;
+constexpr size_t READ_SLOT = 2u << 20; constexpr int READ_SLOTS = 8;
 struct ReadSlots {
-  std::mutex mu; unsigned char* p[READ_SLOTS] = {};
-  int have(int want) {                   // with mu held: the number of slots there are, at most `want`
+  std::mutex mu; unsigned char* p[READ_SLOTS] = {}; unsigned long long ctx = 0;
+  int have(int want) {                   // with mu held, the device current: the number of slots there are, at most `want`
+    const unsigned long long now = context_id();
+    if (ctx != now) { memset(p, 0, sizeof p); ctx = now; }
     int n = 0;
     while (n < want && (p[n] || cudaHostAlloc(&p[n], READ_SLOT, cudaHostAllocPortable) == cudaSuccess)) n++;
     if (n < want) { p[n] = nullptr; cudaGetLastError(); }
     return n;
   }
+  void release() {                       // with mu held, the device current
+    if (ctx == context_id()) for (unsigned char* q : p) if (q) cudaFreeHost(q);
+    memset(p, 0, sizeof p);
+  }
 };
-ReadSlots* read_slots() { static ReadSlots* const s = new ReadSlots[READ_DEVICES]; return s; }      // never destroyed: the driver may be gone before a destructor runs
+ReadSlots* read_slots() { static ReadSlots* const s = new ReadSlots[KEPT_DEVICES]; return s; }      // never destroyed: the driver may be gone before a destructor runs
 void widen_bf16(const uint16_t* src, float* dst, size_t n) {
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
   for (size_t i = 0; i < n; i++) d[i] = (uint32_t)src[i] << 16;
@@ -924,7 +938,7 @@ cudaError_t read_pageable(cudaStream_t stream, const void* src, void* out, size_
 // the caller has made `device` current
 cudaError_t read_back(int device, cudaStream_t stream, const void* src, void* out, size_t bytes, bool widen) {
   if (bytes == 0) return cudaSuccess;
-  if (device >= READ_DEVICES) return read_pageable(stream, src, out, bytes, widen);
+  if (device >= KEPT_DEVICES) return read_pageable(stream, src, out, bytes, widen);
   const size_t pieces = (bytes + READ_SLOT - 1) / READ_SLOT;
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
   ReadSlots& slots = read_slots()[device];
@@ -1311,7 +1325,7 @@ extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
     cudaMemsetAsync(c->d_phase_last, 0, sizeof(unsigned long long) * nph, c->stream);
   }
   cudaEventRecord(c->ev0, c->stream);
-  cudaError_t e = c->bf ? launch_kernel<bf16, 768, 64>(C, c->nblocks, c->smem, c->device, c->stream) : launch_kernel<float, 64, 16>(C, c->nblocks, c->smem, c->device, c->stream);
+  cudaError_t e = c->bf ? launch_kernel<bf16, 768, 64>(C, c->nblocks, c->smem, c->stream) : launch_kernel<float, 64, 16>(C, c->nblocks, c->smem, c->stream);
   cudaEventRecord(c->ev1, c->stream);
   if (e != cudaSuccess) return fail(c, OFA_CUDA_ERROR, std::string("kernel launch failed: ") + cudaGetErrorString(e));
   // what ofa_wait looks at comes back behind the kernel: the decoder's scalars and the device status, 128 adjacent bytes
@@ -1487,50 +1501,60 @@ namespace {
 // Memory and events of one ofa_run_phases call, kept between calls: allocating and freeing them on each call (some twenty
 // cudaMalloc / cudaFree, every one a device-wide wait, and a query of all device properties) cost 3 ms beside a kernel of 0.1 to
 // 1 ms. A call takes a workspace of its device from the pool or makes one, and hands it back when its kernel has finished, so
-// threads and streams never share one. The pool keeps at most four, none above 4 MB; the rest are freed.
+// threads and streams never share one. A device's pool keeps the four used last, none above 4 MB; the rest are freed, all of them by
+// ofa_release_caches; those of a context that a device reset has ended are never used again.
 struct Workspace {
-  int device = -1;
+  unsigned long long ctx = 0;
   unsigned char *dev = nullptr, *host = nullptr, *rep = nullptr, *back = nullptr;   // tables on the device, their pinned image, per-repeat words on the device, pinned status
   size_t bytes = 0, rep_bytes = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
-  bool make(int d, size_t n, size_t nrep) {
-    device = d; bytes = up64(std::max<size_t>(n, 64 << 10)); rep_bytes = std::max<size_t>(nrep, 4096);
+  bool make(size_t n, size_t nrep) {
+    bytes = up64(std::max<size_t>(n, 64 << 10)); rep_bytes = std::max<size_t>(nrep, 4096);
     return cudaMalloc(&dev, bytes) == cudaSuccess && cudaMalloc(&rep, rep_bytes) == cudaSuccess && cudaHostAlloc(&host, bytes, cudaHostAllocDefault) == cudaSuccess &&
            cudaHostAlloc(&back, 64, cudaHostAllocDefault) == cudaSuccess && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess &&
            cudaEventCreateWithFlags(&e2, cudaEventDisableTiming) == cudaSuccess;
   }
-  ~Workspace() {
+  void free_all() {                      // its context is current
     if (dev) cudaFree(dev);
     if (rep) cudaFree(rep);
     if (host) cudaFreeHost(host);
     if (back) cudaFreeHost(back);
     for (cudaEvent_t e : {e0, e1, e2}) if (e) cudaEventDestroy(e);
+    *this = Workspace();
   }
 };
-struct WorkspacePool {
-  std::mutex mu; std::vector<Workspace*> idle;
-  ~WorkspacePool() { for (Workspace* w : idle) delete w; }
+struct WorkspacePool {                   // of one device; the used last at the end
+  static constexpr int KEEP = 4;
+  std::mutex mu; Workspace idle[KEEP]; int n = 0;
+  Workspace take(int i) { Workspace w = idle[i]; for (n--; i < n; i++) idle[i] = idle[i + 1]; return w; }
 };
-WorkspacePool g_workspaces;
+WorkspacePool* workspaces() { static WorkspacePool* const p = new WorkspacePool[KEPT_DEVICES]; return p; }
 struct WorkspaceLease {
-  Workspace* w = nullptr;
-  WorkspaceLease(int dev, size_t bytes, size_t rep_bytes) {
-    {
-      std::lock_guard<std::mutex> lk(g_workspaces.mu);
-      for (size_t i = 0; i < g_workspaces.idle.size() && !w; i++) {
-        Workspace* c = g_workspaces.idle[i];
-        if (c->device == dev && c->bytes >= bytes && c->rep_bytes >= rep_bytes) { w = c; g_workspaces.idle.erase(g_workspaces.idle.begin() + i); }
-      }
+  WorkspacePool* pool; Workspace w; bool ok = false;
+  WorkspaceLease(int device, size_t bytes, size_t rep_bytes) : pool(device < KEPT_DEVICES ? workspaces() + device : nullptr) {
+    const unsigned long long now = context_id();
+    if (pool) {
+      std::lock_guard<std::mutex> lk(pool->mu);
+      for (int i = pool->n - 1; i >= 0 && !ok; i--)
+        if (pool->idle[i].ctx == now && pool->idle[i].bytes >= bytes && pool->idle[i].rep_bytes >= rep_bytes) { w = pool->take(i); ok = true; }
     }
-    if (!w) { w = new Workspace(); if (!w->make(dev, bytes, rep_bytes)) { cudaGetLastError(); delete w; w = nullptr; } }
+    if (ok) return;
+    ok = w.make(bytes, rep_bytes); w.ctx = now;
+    if (!ok) { cudaGetLastError(); w.free_all(); }
   }
   ~WorkspaceLease() {
-    if (!w) return;
-    if (w->bytes + w->rep_bytes <= (4u << 20)) {
-      std::lock_guard<std::mutex> lk(g_workspaces.mu);
-      if (g_workspaces.idle.size() < 4) { g_workspaces.idle.push_back(w); return; }
+    if (ok && pool && w.bytes + w.rep_bytes <= (4u << 20)) {
+      std::lock_guard<std::mutex> lk(pool->mu);
+      Workspace oldest;                  // of this context; if there is none, one of a context that has ended makes room
+      if (pool->n == WorkspacePool::KEEP) {
+        int i = 0;
+        while (i < pool->n && pool->idle[i].ctx != w.ctx) i++;
+        if (i < pool->n) oldest = pool->take(i); else pool->take(0);
+      }
+      pool->idle[pool->n++] = w;
+      w = oldest;
     }
-    delete w;
+    w.free_all();
   }
   WorkspaceLease(const WorkspaceLease&) = delete; WorkspaceLease& operator=(const WorkspaceLease&) = delete;
 };
@@ -1566,8 +1590,8 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   const size_t rep_bytes = up64(sizeof(unsigned long long) * (size_t)repeats) + up64(sizeof(float) * (size_t)repeats);
   const size_t cnt_cap = 128 + 4 * (size_t)(DONE_STRIDE * nph + RB_STRIDE);
   WorkspaceLease ws(dev, map_cap + tab_cap + 192 + cnt_cap, rep_bytes);
-  if (!ws.w) return fail(nullptr, OFA_CUDA_ERROR, "out of memory (workspace)");
-  MapSink sink; sink.host = ws.w->host; sink.dev = ws.w->dev; sink.cap = map_cap;
+  if (!ws.ok) return fail(nullptr, OFA_CUDA_ERROR, "out of memory (workspace)");
+  MapSink sink; sink.host = ws.w.host; sink.dev = ws.w.dev; sink.cap = map_cap;
   std::vector<HostPhase> P(nph);
   for (int i = 0; i < nph; i++) {
     const ofa_phase& s = phases[i];
@@ -1620,35 +1644,56 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   // one image of everything the launch needs: TMA descriptors | tables | status, finished word, end time | counters (zero), uploaded
   // in one copy behind the caller's earlier work on the default stream
   const size_t o_tab = map_cap, o_st = o_tab + job_table_bytes(hj), o_cnt = o_st + 192, total = o_cnt + job_counter_bytes(hj);
-  if (total > ws.w->bytes) return fail(nullptr, OFA_CUDA_ERROR, "workspace too small");
-  memset(ws.w->host + o_st, 0, total - o_st);
+  if (total > ws.w.bytes) return fail(nullptr, OFA_CUDA_ERROR, "workspace too small");
+  memset(ws.w.host + o_st, 0, total - o_st);
   static thread_local Ctx C;      // 31 KB: not on the stack
   memset(&C, 0, offsetof(Ctx, train_rec));
-  C.train = place_job(hj, repeats, ws.w->host + o_tab, ws.w->dev + o_tab, ws.w->dev + o_cnt); C.md = m;
+  C.train = place_job(hj, repeats, ws.w.host + o_tab, ws.w.dev + o_tab, ws.w.dev + o_cnt); C.md = m;
   fill_param_records(C, &hj, nullptr);
   if (adam) { C.hp.lr_max = adam[0]; C.hp.lr_min = adam[0]; C.hp.beta1 = adam[1]; C.hp.beta2 = adam[2]; C.hp.eps = adam[3]; C.hp.wd = adam[4]; C.hp.grad_scale = adam[5]; C.hp.constant_lr = 1; }
   C.train_sms = num_sms; C.use_train = 1;
-  C.status = reinterpret_cast<DevStatus*>(ws.w->dev + o_st); C.finished = reinterpret_cast<int*>(ws.w->dev + o_st + 64); C.t_end = reinterpret_cast<unsigned long long*>(ws.w->dev + o_st + 128);
-  C.step_done = reinterpret_cast<unsigned long long*>(ws.w->rep); C.loss_hist = reinterpret_cast<float*>(ws.w->rep + up64(sizeof(unsigned long long) * (size_t)repeats));
+  C.status = reinterpret_cast<DevStatus*>(ws.w.dev + o_st); C.finished = reinterpret_cast<int*>(ws.w.dev + o_st + 64); C.t_end = reinterpret_cast<unsigned long long*>(ws.w.dev + o_st + 128);
+  C.step_done = reinterpret_cast<unsigned long long*>(ws.w.rep); C.loss_hist = reinterpret_cast<float*>(ws.w.rep + up64(sizeof(unsigned long long) * (size_t)repeats));
   C.dep_timeout_ns = 20000000000ull;
   C.smem_bytes = smem;
   C.prof_step = -1;
-  cudaError_t e = cudaMemcpyAsync(ws.w->dev, ws.w->host, total, cudaMemcpyHostToDevice, 0);
+  cudaError_t e = cudaMemcpyAsync(ws.w.dev, ws.w.host, total, cudaMemcpyHostToDevice, 0);
   if (e == cudaSuccess) {
-    cudaEventRecord(ws.w->e0, 0);
-    e = bf ? launch_kernel<bf16, 768, 64>(C, nblocks, smem, dev, 0) : launch_kernel<float, 64, 16>(C, nblocks, smem, dev, 0);
-    cudaEventRecord(ws.w->e1, 0);
+    cudaEventRecord(ws.w.e0, 0);
+    e = bf ? launch_kernel<bf16, 768, 64>(C, nblocks, smem, 0) : launch_kernel<float, 64, 16>(C, nblocks, smem, 0);
+    cudaEventRecord(ws.w.e1, 0);
   }
   if (e != cudaSuccess) { cudaStreamSynchronize(0); return fail(nullptr, OFA_CUDA_ERROR, std::string("launch failed: ") + cudaGetErrorString(e)); }
-  DevStatus& ds = *reinterpret_cast<DevStatus*>(ws.w->back);
+  DevStatus& ds = *reinterpret_cast<DevStatus*>(ws.w.back);
   cudaMemcpyAsync(&ds, C.status, sizeof ds, cudaMemcpyDeviceToHost, 0);
-  cudaEventRecord(ws.w->e2, 0);
-  if ((e = cudaEventSynchronize(ws.w->e2)) != cudaSuccess) return fail(nullptr, OFA_CUDA_ERROR, std::string("kernel failed: ") + cudaGetErrorString(e));
-  float t = 0.f; cudaEventElapsedTime(&t, ws.w->e0, ws.w->e1); if (ms) *ms = t;
+  cudaEventRecord(ws.w.e2, 0);
+  if ((e = cudaEventSynchronize(ws.w.e2)) != cudaSuccess) return fail(nullptr, OFA_CUDA_ERROR, std::string("kernel failed: ") + cudaGetErrorString(e));
+  float t = 0.f; cudaEventElapsedTime(&t, ws.w.e0, ws.w.e1); if (ms) *ms = t;
   if (ds.code || ds.abort) {
     if (status) { status->code = OFA_DEVICE_ABORT; status->dev_code = ds.code; status->phase = ds.phase; status->task = ds.task; status->block = ds.block; status->aux = ds.aux; }
     return fail(nullptr, OFA_DEVICE_ABORT, "device-side bounded wait expired: code " + std::to_string(ds.code) + " phase " + std::to_string(ds.phase) + " task " + std::to_string(ds.task) + " aux " + std::to_string(ds.aux));
   }
+  return OFA_OK;
+}
+
+extern "C" int ofa_release_caches(void) {
+  int before = 0, count = 0;
+  if (cudaGetDevice(&before) != cudaSuccess || cudaGetDeviceCount(&count) != cudaSuccess) { cudaGetLastError(); return OFA_CUDA_ERROR; }
+  for (int d = 0; d < std::min(count, KEPT_DEVICES); d++) {
+    ReadSlots& slots = read_slots()[d]; WorkspacePool& pool = workspaces()[d];
+    Workspace give_back[WorkspacePool::KEEP]; int n = 0;
+    {
+      std::lock_guard<std::mutex> lk(pool.mu);
+      while (pool.n > 0) give_back[n++] = pool.take(pool.n - 1);
+    }
+    std::lock_guard<std::mutex> lk(slots.mu);
+    if (n == 0 && slots.ctx == 0) continue;            // nothing was kept there: no context is made for it
+    cudaSetDevice(d);
+    const unsigned long long now = context_id();
+    for (int i = 0; i < n; i++) if (give_back[i].ctx == now) give_back[i].free_all();
+    slots.release();
+  }
+  cudaSetDevice(before);
   return OFA_OK;
 }
 

@@ -1,5 +1,6 @@
 """What the host calls promise beside their results, on the GPU through the C ABI: a call has read its host buffers when it returns, and
-comes behind work that the caller queued on the default stream; reads work from several threads and where no thread can be started."""
+comes behind work that the caller queued on the default stream; reads work from several threads and where no thread can be started; launches
+work again after a device reset, and what is kept between calls can be given back."""
 import ctypes as C
 import os
 import subprocess
@@ -206,3 +207,68 @@ def test_reads_work_where_no_thread_can_be_started(ofa, tmp_path):
     subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(so), str(src), "-ldl"], check=True)
     r = subprocess.run([sys.executable, str(prog), ROOT], env=dict(os.environ, LD_PRELOAD=str(so)), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "READ" in r.stdout, (r.returncode, r.stdout[-500:], r.stderr[-2000:])
+
+
+RESET = r"""
+import ctypes, glob, importlib, os, sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+ofa = importlib.import_module("open-flapping-airplanes_b200")
+K = ofa.capi
+cands = glob.glob(os.path.join(os.path.dirname(os.path.dirname(torch.__file__)), "nvidia", "cuda_runtime", "lib", "libcudart.so*")) + ["libcudart.so.12", "/usr/local/cuda/lib64/libcudart.so"]
+rt = None
+for c in cands:
+    try:
+        rt = ctypes.CDLL(c); break
+    except OSError:
+        pass
+w = np.random.default_rng(0).normal(0, 0.02, 1 << 20).astype(np.float32)
+def once():
+    for preset, V in (("tiny", 65), ("gpt_s", 512)):
+        cfg = ofa.default_config(preset)
+        cfg.vocab = cfg.valid_vocab = V
+        if preset == "gpt_s": cfg.n_layer, cfg.ctx_len, cfg.batch = 1, 128, 1
+        mk = ofa.Megakernel(cfg)
+        mk.load_weights(np.resize(w, mk.num_params))
+        mk.set_tokens(np.arange(4096, dtype=np.uint32) % V)
+        mk.run(2)
+        out = mk.losses(), mk.read_weights()
+        mk.close()
+        yield out
+    dims = dict(vocab=65, d_model=64, n_layer=1, n_head=4, ctx_len=64, batch=4)
+    a = ofa.DeviceBuffer.from_host(w[:4096].reshape(64, 64)); b = ofa.DeviceBuffer((64, 64), np.float32)
+    ofa.run_phases(K.DTYPE_F32, dims, [ofa.gemm_phase(0, 0, 64, 64, 64, a, 64, a, 64, b, 64)])
+    out = (b.download(),)
+    a.free(); b.free()
+    yield out
+first = list(once())
+rc = rt.cudaDeviceReset()
+assert rc == 0, rc
+second = list(once())
+for x, y in zip(first, second):
+    for p, q in zip(x, y):
+        assert np.array_equal(p, q)
+print("SAME")
+"""
+
+
+def test_everything_works_again_after_a_device_reset(ofa, tmp_path):
+    prog = tmp_path / "prog.py"
+    prog.write_text(RESET)
+    r = subprocess.run([sys.executable, str(prog), ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "SAME" in r.stdout, (r.returncode, r.stdout[-500:], r.stderr[-2000:])
+
+
+def test_what_calls_keep_is_bounded_and_can_be_given_back(ofa):
+    """Ever larger phase lists push the smaller workspaces out; afterwards nothing of them is left."""
+    lib, K = ofa.capi.load(), ofa.capi
+    dims = dict(vocab=65, d_model=64, n_layer=1, n_head=4, ctx_len=64, batch=4)
+    assert lib.ofa_release_caches() == K.OK
+    free = torch.cuda.mem_get_info()[0]
+    for n in (1, 40, 200, 500, 1000, 1500, 2000, 2500, 3, 3000):
+        ofa.run_phases(K.DTYPE_F32, dims, [ofa.phase(K.TK_BARRIER)] * n)
+        assert free - torch.cuda.mem_get_info()[0] <= 4 * (4 << 20) + (4 << 20)      # four of 4 MB, in granules of 2 MB
+    assert lib.ofa_release_caches() == K.OK
+    assert free - torch.cuda.mem_get_info()[0] <= 2 << 20
+    assert ofa.run_phases(K.DTYPE_F32, dims, [ofa.phase(K.TK_BARRIER)] * 3) > 0
+    assert lib.ofa_release_caches() == K.OK and lib.ofa_release_caches() == K.OK
