@@ -546,7 +546,7 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
 #pragma unroll 4
   for (int n = p0 + lane; n < p0 + per; n += 32) {
     const int v = n < p1 ? tok[n] - lo : -1;
-    const bool hit = (unsigned)v < (unsigned)EMB_VCHUNK;
+    const bool hit = (unsigned)v < (unsigned)vchunk;
     mine_cnt += __popc(__ballot_sync(0xffffffffu, hit));
     if (hit) atomicAdd(&rowcnt[v], 1);
   }
@@ -557,7 +557,7 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
   for (int w = 0; w < NTHR / 32; w++) { const int c = wcnt[w]; total += c; if (w < warp) slot += c; }
   for (int n = p0 + lane; n < p0 + per && mine_cnt > 0; n += 32) {      // second look at the same positions (now in L1): place the matches
     const int v = n < p1 ? tok[n] - lo : -1;
-    const bool hit = (unsigned)v < (unsigned)EMB_VCHUNK;
+    const bool hit = (unsigned)v < (unsigned)vchunk;
     const unsigned b = __ballot_sync(0xffffffffu, hit);
     if (hit) { const int at = slot + __popc(b & ((1u << lane) - 1u)); list[at] = n; rowof[at] = (unsigned char)v; }
     slot += __popc(b);

@@ -1,0 +1,31 @@
+"""Tasks at the sizes where their tiles, panels, rounds and task sizes end, on the GPU through the C ABI, against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K(ofa):
+    return ofa.capi
+
+
+@pytest.mark.parametrize("bf,V", [(True, 128), (True, 2432), (True, 4864), (True, 9600), (False, 1), (False, 7), (False, 65), (False, 1183), (False, 2400)])
+def test_embedding_gradient_with_each_task_size(ofa, K, bf, V):
+    """A task covers 8 to 128 rows of the vocabulary, by its size; ids at the edges of the tasks, repeated and absent ones."""
+    D, T, B = (768, 128, 2) if bf else (64, 64, 4)
+    N = T * B
+    dims = dict(vocab=V, d_model=D, n_layer=1, n_head=12 if bf else 4, ctx_len=T, batch=B)
+    g = torch.Generator().manual_seed(V)
+    tok = torch.randint(0, V, (N,), generator=g, dtype=torch.int32)
+    edge = [v for c in (8, 16, 32, 64, 128) for v in (c - 1, c, c + 1, 2 * c) if v < V] + [0, V - 1]
+    tok[:len(edge)] = torch.tensor(edge, dtype=torch.int32); tok[N - len(edge):] = tok[:len(edge)]
+    dx = torch.randn(N, D, generator=g)
+    dx = dx.bfloat16().float() if bf else dx
+    d_dx, d_tok, out = ofa.DeviceBuffer.from_host(dx.numpy(), "bf16" if bf else np.float32), ofa.DeviceBuffer.from_host(tok.numpy()), ofa.DeviceBuffer.from_host(np.full((V, D), 9.0, np.float32))
+    ofa.run_phases(K.DTYPE_BF16 if bf else K.DTYPE_F32, dims, [ofa.phase(K.TK_EMB_WTE, [out, d_dx, d_tok])])
+    ref = np.zeros((V, D), np.float32)
+    for n in range(N):                                   # the order of the task: increasing position
+        ref[tok[n]] += dx[n].numpy()
+    np.testing.assert_array_equal(out.download(), ref)
