@@ -419,7 +419,9 @@ bool build_train_graph(ofa_ctx* c) {
   auto rbmap = [&](const PhaseDesc& d) -> int {
     if (!rb_ok) return 0;
     switch (d.kind) {
-      case TK_GEMM: return (d.layout != GL_TN && d.g.M == (int)N && d.tiles_m == (int)N / 128) ? (RB_MOD | d.tiles_m << 8) : 0;
+      case TK_GEMM:                                    // d.i0: tasks walk along N first, a row block's strips are consecutive
+        if (d.layout == GL_TN || d.g.M != (int)N || d.tiles_m != (int)N / 128) return 0;
+        return d.i0 ? (RB_DIV | (d.ntasks / d.tiles_m) << 8) : (RB_MOD | d.tiles_m << 8);
       case TK_LN_FWD: case TK_LN_BWD: case TK_EMBED: return RB_DIV | (128 / ew::ROWS_PER_TASK) << 8;
       case TK_CE: return RB_DIV | (128 / ew::CE_ROWS) << 8;
       case TK_ATT_FWD: return RB_ATT_FWD;

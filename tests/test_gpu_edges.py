@@ -29,3 +29,23 @@ def test_embedding_gradient_with_each_task_size(ofa, K, bf, V):
     for n in range(N):                                   # the order of the task: increasing position
         ref[tok[n]] += dx[n].numpy()
     np.testing.assert_array_equal(out.download(), ref)
+
+
+@pytest.mark.parametrize("nsub", [0, 1, 4001, 4002, 4003])
+def test_training_step_with_tasks_ordered_along_n(ofa, nsub):
+    """A task waits for the producers of its rows and asks for its weights ahead, whatever the order of a phase's tasks: the gradients do not change."""
+    cfg = ofa.default_config("gpt_s")
+    cfg.vocab = cfg.valid_vocab = 640
+    cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode, cfg.gemm_nsub = 1, 256, 1, ofa.capi.MODE_NO_OPT, nsub
+    mk = ofa.Megakernel(cfg)
+    w = torch.randn(mk.num_params, generator=torch.Generator().manual_seed(3)).mul_(0.02).numpy()
+    mk.load_weights(w); mk.set_tokens(np.random.default_rng(1).integers(0, 640, 1 << 13, dtype=np.uint32)); mk.set_starts(np.array([[17]], np.uint32))
+    mk.run(1)
+    got = mk.read_grads()
+    mk.close()
+    cfg.gemm_nsub = 2
+    mk = ofa.Megakernel(cfg)
+    mk.load_weights(w); mk.set_tokens(np.random.default_rng(1).integers(0, 640, 1 << 13, dtype=np.uint32)); mk.set_starts(np.array([[17]], np.uint32))
+    mk.run(1)
+    np.testing.assert_array_equal(got, mk.read_grads())
+    mk.close()
