@@ -187,6 +187,9 @@ struct EarlyTicket { unsigned* counter; volatile int* slot; };
 __device__ __forceinline__ void take_early_ticket(const EarlyTicket& e) { if (e.counter) *e.slot = (int)(atomicAdd(e.counter, 1u) + 1u); }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+// a descriptor in global memory that the host has written: needed once per block and launch before its first use, else the descriptor
+// that an earlier launch found at the address may be used
+__device__ __forceinline__ void tmap_fence(const void* tmap) { asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(tmap) : "memory"); }
 // 2-D tiled TMA load (no multicast), completion counted in bytes on `bar`. c0 = innermost coordinate (elements).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -299,6 +299,7 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
   const unsigned total = (unsigned)J.nsteps * (unsigned)J.tasks_per_step;
   gemm_tc::GemmPipe gp; gp.stage_count[0] = gp.stage_count[1] = gp.tile_count[0] = gp.tile_count[1] = gp.tmem_base = 0;
   const bool use_tc = IsBf16<T>::value && job_id == 0;
+  for (int q = tid; q < C.nmaps; q += NTHR) tmap_fence(C.maps + 128 * (size_t)q);      // the barriers below come before the first use of any
   attn_tc::AttnPipe ap; ap.tasks = ap.stages = ap.stages2 = ap.a = ap.b = ap.done = 0;
   uint32_t bulk_uses = 0;                            // uses of the block's bulk-copy barrier (control area byte 104)
   uint32_t adam_tiles = 0;                           // tiles the block's AdamW tasks have staged (three barriers at control area byte 224)

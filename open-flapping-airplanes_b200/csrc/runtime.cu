@@ -130,23 +130,18 @@ struct Arena {   // device allocations owned by one context / one ofa_run_phases
   void free_all() { for (void* p : ptrs) cudaFree(p); ptrs.clear(); }
 };
 
-// Where the TMA descriptors of phases go: one by one into a context's arena, or (ofa_run_phases) into the call's packed tables, which
-// are uploaded in one copy.
+// Where the TMA descriptors of a launch go: side by side in one piece of device memory (a context's, or the head of an ofa_run_phases
+// workspace), written to its host image and uploaded in one copy. Every block of a launch fences them all before it uses the first
+// (Ctx::maps): the same addresses may have held other descriptors in an earlier launch.
 struct MapSink {
-  Arena* ar = nullptr;
   unsigned char *host = nullptr, *dev = nullptr; size_t used = 0, cap = 0;
-  bool dry() const { return ar && ar->dry; }
-  // device address of n descriptors with the given contents, 64-byte aligned
+  bool dry = false;
+  // device address of consecutive descriptors with the given contents, 128-byte aligned
   const void* put(const void* maps, size_t bytes) {
-    if (ar) {
-      unsigned char* d = ar->alloc<unsigned char>(bytes, false);
-      if (d && !ar->dry) ar->h2d(d, maps, bytes);
-      return d;
-    }
     if (used + bytes > cap) return nullptr;
     memcpy(host + used, maps, bytes);
     const void* d = dev + used;
-    used += (bytes + 63) / 64 * 64;
+    used += (bytes + 127) / 128 * 128;
     return d;
   }
 };
@@ -154,7 +149,7 @@ struct MapSink {
 // TMA descriptors of one layer's attention operands (qkv [N, 3D] and, for the backward tasks, dO [N, D]) in device memory
 const void* make_attn_maps(MapSink& sink, const void* qkv, const void* dO, int N, int D, std::string& err) {
   attn_tc::Maps hm; memset(&hm, 0, sizeof hm);
-  if (!sink.dry()) {
+  if (!sink.dry) {
     bool ok = encode_map(&hm.qkv128, qkv, 3 * D, N, 3 * D, 64, 128) && encode_map(&hm.qkv64, qkv, 3 * D, N, 3 * D, 64, 64);
     if (dO) ok = ok && encode_map(&hm.dO128, dO, D, N, D, 64, 128) && encode_map(&hm.dO64, dO, D, N, D, 64, 64);
     if (!ok) { err = "cuTensorMapEncodeTiled failed (attention)"; return nullptr; }
@@ -203,7 +198,7 @@ bool prepare_gemm_bf16(PhaseDesc& d, MapSink& sink, int nsub_cfg, int nblocks, s
   d.tiles_m = tm;
   d.ntasks = tm * ((tn + nsub - 1) / nsub);
   CUtensorMap hm[2]; memset(hm, 0, sizeof hm);
-  if (!sink.dry()) {
+  if (!sink.dry) {
     const bool a_kmajor = d.layout != GL_TN, b_kmajor = d.layout == GL_NT;
     bool ok = a_kmajor ? encode_map(&hm[0], g.A, g.K, g.M, g.lda, 64, 128) : encode_map(&hm[0], g.A, g.M, g.K, g.lda, 64, 64);
     ok = ok && (b_kmajor ? encode_map(&hm[1], g.B, g.K, g.N, g.ldb, 64, 128) : encode_map(&hm[1], g.B, g.N, g.K, g.ldb, 64, 64));
@@ -359,7 +354,8 @@ struct ofa_ctx {
   std::vector<HostPhase> train_ph, dec_ph; int train_last = 0, dec_last = 0;
   HostJob train_job, dec_job;        // the uploaded jobs
   unsigned char* d_jobs = nullptr; size_t jobs_cnt_off = 0, jobs_cnt_bytes = 0;   // tables of both jobs, then everything a launch starts from zero: counters, status, finished words
-  bool jobs_ready = false; unsigned jobs_seed = 0;
+  unsigned jobs_seed = 0;
+  MapSink maps; std::vector<unsigned char> maps_img;   // TMA descriptors of both graphs and their host image
   unsigned char* h_back = nullptr;   // pinned: what every launch copies back (device status, then the decoder's scalars)
   Ctx C{};
   DevStatus* d_status = nullptr;
@@ -444,7 +440,7 @@ bool build_train_graph(ofa_ctx* c) {
     std::vector<std::string> pv; for (auto& e : deps_prev) if (!e.empty()) pv.push_back(e);
     prevdeps.push_back(pv);
   };
-  MapSink sink; sink.ar = &c->ar;
+  MapSink& sink = c->maps;
   auto mk = [&](int kind, int ntasks) { PhaseDesc d; memset(&d, 0, sizeof d); d.kind = kind; d.ntasks = ntasks; return d; };
   auto is_weight = [&](const void* p) { const T* w = reinterpret_cast<const T*>(p); return w >= Wact && w < Wact + lay.total; };   // read by the step, written only by its optimizer
   // wide = 1: 128 x 256 tiles where the width allows (a long K and more tiles than blocks: only the LM head's weight gradient)
@@ -794,9 +790,8 @@ bool build_decode_graph(ofa_ctx* c) {
             encode_map(&mo[l], ho[l], D, D, D, cbw, m.DH, f32w, false);
     }
     if (!okm) { c->err = "cuTensorMapEncodeTiled failed (decode prefetch views)"; return false; }
-    CUtensorMap* dq = c->ar.alloc<CUtensorMap>(L, false); CUtensorMap* du = c->ar.alloc<CUtensorMap>(L, false); CUtensorMap* dw = c->ar.alloc<CUtensorMap>(L, false);
-    if (dq && du && dw) { c->ar.h2d(dq, mq.data(), L * sizeof(CUtensorMap)); c->ar.h2d(du, mu.data(), L * sizeof(CUtensorMap)); c->ar.h2d(dw, mo.data(), L * sizeof(CUtensorMap)); }
-    dp.tm_qkv = dq; dp.tm_up = du; dp.tm_wo = dw;
+    dp.tm_qkv = c->maps.put(mq.data(), L * sizeof(CUtensorMap)); dp.tm_up = c->maps.put(mu.data(), L * sizeof(CUtensorMap)); dp.tm_wo = c->maps.put(mo.data(), L * sizeof(CUtensorMap));
+    if (!dp.tm_qkv || !dp.tm_up || !dp.tm_wo) { c->err = "out of device memory (decode prefetch views)"; return false; }
   }
   DecodeState& st = dp.st;
   st.xw = c->ar.alloc<unsigned long long>(D); st.xr = c->ar.alloc<unsigned long long>(D);
@@ -1149,12 +1144,19 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
   C.smid_rank = c->d_smid_rank; C.live = c->d_live; C.t_end = c->d_t_end;
   C.dep_timeout_ns = (unsigned long long)((cfg->timeout_s > 0 ? cfg->timeout_s : 20.0) * 1e9);
   C.prof_step = -1;
+  // a layer has 12 products of two descriptors, attention forward and backward of four, three views for the decoder; the head and its split form
+  c->maps.cap = 128 * (size_t)(35 * m.L + 32); c->maps.dry = dry;
+  c->maps_img.resize(c->maps.cap); c->maps.host = c->maps_img.data();
+  c->maps.dev = c->ar.alloc<unsigned char>(c->maps.cap, false);
+  if (!c->maps.dev) return bail(OFA_CUDA_ERROR, "out of device memory (TMA descriptors)");
   bool ok = decode_only ? true : (c->bf ? build_train_graph<bf16>(c) : build_train_graph<float>(c));
   if (!ok) return bail(OFA_BAD_CONFIG, "training graph: " + c->err);
   if (cfg->use_decode) {
     ok = c->bf ? build_decode_graph<bf16>(c) : build_decode_graph<float>(c);
     if (!ok) return bail(OFA_BAD_CONFIG, "decode graph: " + c->err);
   }
+  c->ar.h2d(c->maps.dev, c->maps.host, c->maps.used);
+  C.maps = c->maps.dev; C.nmaps = (int)(c->maps.used / 128);
   const int nph = std::max<int>(1, (int)c->train_ph.size());
   c->d_phase_busy = c->ar.alloc<unsigned long long>(2 * nph);   /* busy, then dependency wait */ c->d_phase_first = c->ar.alloc<unsigned long long>(nph); c->d_phase_last = c->ar.alloc<unsigned long long>(nph);
   c->d_blk_busy = c->ar.alloc<unsigned long long>(6 * c->nblocks);
@@ -1658,6 +1660,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   C.step_done = reinterpret_cast<unsigned long long*>(ws.w.rep); C.loss_hist = reinterpret_cast<float*>(ws.w.rep + up64(sizeof(unsigned long long) * (size_t)repeats));
   C.dep_timeout_ns = 20000000000ull;
   C.smem_bytes = smem;
+  C.maps = ws.w.dev; C.nmaps = (int)(sink.used / 128);
   C.prof_step = -1;
   cudaError_t e = cudaMemcpyAsync(ws.w.dev, ws.w.host, total, cudaMemcpyHostToDevice, 0);
   if (e == cudaSuccess) {

@@ -272,3 +272,43 @@ def test_what_calls_keep_is_bounded_and_can_be_given_back(ofa):
     assert free - torch.cuda.mem_get_info()[0] <= 2 << 20
     assert ofa.run_phases(K.DTYPE_F32, dims, [ofa.phase(K.TK_BARRIER)] * 3) > 0
     assert lib.ofa_release_caches() == K.OK and lib.ofa_release_caches() == K.OK
+
+
+def _gemm_case(ofa, K, N, Kd, seed):
+    g = torch.Generator().manual_seed(seed)
+    A, B = (torch.randn(256, Kd, generator=g) * 0.3).bfloat16(), (torch.randn(Kd, N, generator=g) * 0.3).bfloat16()
+    bufs = [ofa.DeviceBuffer.from_host(A.float().numpy(), "bf16"), ofa.DeviceBuffer.from_host(B.float().numpy(), "bf16"), ofa.DeviceBuffer((256, N), "bf16")]
+    return bufs, ofa.gemm_phase(0, 0, 256, N, Kd, bufs[0], Kd, bufs[1], N, bufs[2], N), (A.double() @ B.double()).numpy()
+
+
+DIMS = dict(vocab=1024, d_model=768, n_layer=1, n_head=12, ctx_len=256, batch=2)
+
+
+def test_a_workspace_is_reused_with_other_operands_shapes_sizes_and_threads(ofa):
+    """Call after call through ofa_run_phases: other operands and shapes at the same place of the tables, phase lists and repeat counts
+    that grow and shrink, from two threads. 256 x N x K products, bf16 results: half a unit in the last place of 8 bits, 2^-8 of the value."""
+    K = ofa.capi
+    errors = []
+
+    def check(bufs, ref):
+        got = bufs[2].download()
+        assert np.abs(got - ref).max() <= 2.0 ** -8 * np.abs(ref).max() + 1e-3
+
+    def work(base):
+        try:
+            torch.cuda.set_device(0)
+            for i in range(24):
+                cases = [_gemm_case(ofa, K, (128, 256, 384)[(i + j) % 3], (64, 192, 768)[(i + 2 * j) % 3], base + 100 * i + j) for j in range(1 + i % 5)]
+                empty = [ofa.phase(K.TK_BARRIER)] * ((0, 3, 400, 7)[i % 4])
+                ofa.run_phases(K.DTYPE_BF16, DIMS, [c[1] for c in cases] + empty, repeats=(1, 3, 600)[i % 3] if not empty else 1)
+                for bufs, _, ref in cases:
+                    check(bufs, ref)
+        except BaseException as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(b,)) for b in (1, 50000)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors[0]
