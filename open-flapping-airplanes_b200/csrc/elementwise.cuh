@@ -612,6 +612,13 @@ __device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0
 template <class T, class GT>
 __device__ __forceinline__ void embed_bwd_wpe_task(int task, GT* dwpe32, const T* dx0, int N, int Tctx, int D) {
   const int per_row = D / 4;
+  // the buffers of an explicit phase list may begin at any element: four columns then travel one by one
+  const bool vin = (reinterpret_cast<uintptr_t>(dx0) & (4 * sizeof(T) - 1)) == 0, vout = (reinterpret_cast<uintptr_t>(dwpe32) & (4 * sizeof(GT) - 1)) == 0;
+  auto in4 = [vin](const T* p, float* f) {
+    if (vin) { ld4(p, f); return; }
+#pragma unroll
+    for (int k = 0; k < 4; k++) f[k] = to_f(p[k]);
+  };
   for (int i = threadIdx.x; i < WPE_ROWS * per_row; i += NTHR) {
     const int p = task * WPE_ROWS + i / per_row, c = (i % per_row) * 4;
     if (p >= Tctx) break;
@@ -620,18 +627,23 @@ __device__ __forceinline__ void embed_bwd_wpe_task(int task, GT* dwpe32, const T
     for (; n + 3 * Tctx < N; n += 4 * Tctx) {
       float f[4][4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) ld4(dx0 + (size_t)(n + u * Tctx) * D + c, f[u]);
+      for (int u = 0; u < 4; u++) in4(dx0 + (size_t)(n + u * Tctx) * D + c, f[u]);
 #pragma unroll
       for (int u = 0; u < 4; u++)
 #pragma unroll
         for (int k = 0; k < 4; k++) s[k] += f[u][k];
     }
     for (; n < N; n += Tctx) {
-      float f[4]; ld4(dx0 + (size_t)n * D + c, f);
+      float f[4]; in4(dx0 + (size_t)n * D + c, f);
 #pragma unroll
       for (int k = 0; k < 4; k++) s[k] += f[k];
     }
-    st4(dwpe32 + (size_t)p * D + c, s);
+    GT* dst = dwpe32 + (size_t)p * D + c;
+    if (vout) st4(dst, s);
+    else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) dst[k] = from_f<GT>(s[k]);
+    }
   }
 }
 

@@ -49,3 +49,25 @@ def test_training_step_with_tasks_ordered_along_n(ofa, nsub):
     mk.run(1)
     np.testing.assert_array_equal(got, mk.read_grads())
     mk.close()
+
+
+@pytest.mark.parametrize("bf,gbf", [(False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("off_out,off_in", [(0, 0), (1, 0), (0, 1), (2, 2), (3, 1)])
+def test_position_gradient_at_any_element(ofa, K, bf, gbf, off_out, off_in):
+    """Result and operand begin at any element of a buffer, as the scalar form of the task allowed."""
+    D, T, B = (768, 128, 3) if bf else (64, 18, 5)
+    dims = dict(vocab=128, d_model=D, n_layer=1, n_head=12 if bf else 4, ctx_len=T, batch=B)
+    g = torch.Generator().manual_seed(1)
+    dx = torch.randn(B * T, D, generator=g)
+    dx = dx.bfloat16().float() if bf else dx
+    src = ofa.DeviceBuffer.from_host(np.concatenate([np.zeros(off_in, np.float32), dx.numpy().ravel(), np.zeros(4, np.float32)]), "bf16" if bf else np.float32)
+    out = ofa.DeviceBuffer.from_host(np.full(off_out + T * D + 4, 5.0, np.float32), "bf16" if gbf else np.float32)
+    ofa.run_phases(K.DTYPE_BF16 if bf else K.DTYPE_F32, dims, [ofa.phase(K.TK_EMB_WPE, [out.at(off_out), src.at(off_in)], i1=1 if gbf else 0)])
+    ref = np.zeros((T, D), np.float32)
+    for b in range(B):
+        ref += dx.numpy().reshape(B, T, D)[b]
+    got = out.download()
+    if gbf:
+        ref = torch.from_numpy(ref).bfloat16().float().numpy()
+    np.testing.assert_array_equal(got[off_out:off_out + T * D].reshape(T, D), ref)
+    assert np.all(got[:off_out] == 5.0) and np.all(got[off_out + T * D:] == 5.0)
