@@ -107,15 +107,8 @@ __device__ __forceinline__ void l2_prefetch_box(const void* tmap, int c0, int c1
 }
 __device__ __forceinline__ void prefetch_weights(const PhaseDesc& d, int task) {
   const GemmArgs& g = d.g;
-  int strip;
-  if (d.i0) {                                          // tasks walk along N first (see gemm_tc_task): those of the first rows ask
-    strip = task;
-    if (task * g.nsub * g.bn >= g.N) return;
-  } else {
-    if (task % d.tiles_m != 0) return;
-    strip = task / d.tiles_m;
-  }
-  const int n0 = strip * g.nsub * g.bn, n1 = min(g.N, n0 + g.nsub * g.bn);
+  if (task % d.tiles_m != 0) return;
+  const int n0 = (task / d.tiles_m) * g.nsub * g.bn, n1 = min(g.N, n0 + g.nsub * g.bn);
   const bool kmajor = d.layout == GL_NT;
   int left = 64;
   for (int n = n0; n < n1 && left > 0; n += kmajor ? 128 : 64)

@@ -454,7 +454,7 @@ bool build_train_graph(ofa_ctx* c) {
     const int nsub_cfg = (wide && cfg.gemm_nsub == 0 && !getenv("OFA_B200_HEAD_DW_128")) ? (getenv("OFA_B200_HEAD_DW_STRIPS") ? 2000 : 4001) : cfg.gemm_nsub;
     if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, nsub_cfg, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }   // waves are counted over the blocks that train
     else prepare_gemm_f32(d);
-    d.i1 = is_weight(B) ? 1 : 0;
+    d.i1 = is_weight(B) && !d.i0 ? 1 : 0;     // asked for ahead (prefetch_weights), where tasks walk down M first
     return d;
   };
   const bool train = cfg.mode == OFA_MODE_TRAIN, fwd_only = cfg.mode == OFA_MODE_FORWARD;
@@ -532,7 +532,7 @@ bool build_train_graph(ofa_ctx* c) {
     d.g.dr = reinterpret_cast<float*>(lse_part);
     if (bf) { std::string e; if (!prepare_gemm_bf16(d, sink, cfg.gemm_nsub, c->C.train_sms > 0 ? 2 * c->C.train_sms : c->nblocks, e)) { ok = false; err = e; } }
     else prepare_gemm_f32(d);
-    d.i1 = 1;
+    d.i1 = d.i0 ? 0 : 1;
     addp("logits", d, {"lnf"}, {opt_head}, {"lnf"});
   }
   std::vector<std::string> end_deps;
