@@ -131,8 +131,8 @@ struct Arena {   // device allocations owned by one context / one ofa_run_phases
 };
 
 // Where the TMA descriptors of a launch go: side by side in one piece of device memory (a context's, or the head of an ofa_run_phases
-// workspace), written to its host image and uploaded in one copy. Every block of a launch fences them all before it uses the first
-// (Ctx::maps): the same addresses may have held other descriptors in an earlier launch.
+// workspace), written to its host image and uploaded in one copy. Every block of the first launch that uses them, on every SM, fences them
+// all when it starts (Ctx::maps): the same addresses may have held other descriptors in an earlier launch.
 struct MapSink {
   unsigned char *host = nullptr, *dev = nullptr; size_t used = 0, cap = 0;
   bool dry = false;
@@ -1156,7 +1156,7 @@ extern "C" int ofa_create(const ofa_config* cfg, ofa_ctx** out) {
     if (!ok) return bail(OFA_BAD_CONFIG, "decode graph: " + c->err);
   }
   c->ar.h2d(c->maps.dev, c->maps.host, c->maps.used);
-  C.maps = c->maps.dev; C.nmaps = (int)(c->maps.used / 128);
+  C.maps = c->maps.dev; C.nmaps = (int)(c->maps.used / 128);      // until the first launch is under way
   const int nph = std::max<int>(1, (int)c->train_ph.size());
   c->d_phase_busy = c->ar.alloc<unsigned long long>(2 * nph);   /* busy, then dependency wait */ c->d_phase_first = c->ar.alloc<unsigned long long>(nph); c->d_phase_last = c->ar.alloc<unsigned long long>(nph);
   c->d_blk_busy = c->ar.alloc<unsigned long long>(6 * c->nblocks);
@@ -1336,6 +1336,7 @@ extern "C" int ofa_launch(ofa_ctx* c, int nsteps) {
   cudaMemcpyAsync(c->h_back, c->d_scal, 128, cudaMemcpyDeviceToHost, c->stream);
   cudaEventRecord(c->ev2, c->stream);
   c->in_flight = true; c->last_nsteps = nsteps;
+  C.nmaps = 0;                    // every SM has been told; a block of a later launch finds these descriptors and no older ones
   return OFA_OK;
 }
 

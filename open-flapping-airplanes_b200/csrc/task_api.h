@@ -188,11 +188,11 @@ struct Ctx {
   int* blk_info;            // per block: %smid | role << 16 (1 serve, 2 reserved-idle, 3 train, 4 idle)
   int* arrived;             // blocks of this launch that have started (idle partitions leave only when all have)
   int smem_bytes;           // dynamic shared memory per block; its last 1,024 bytes are the control area (barriers, hand-off words, descriptor slots)
-  const unsigned char* maps; int nmaps;     // all TMA descriptors the launch uses, 128 bytes each
   int sched_flags;                          // bit 1: keep the per-phase / per-block time tables
   int train_rec_n, dec_rec_n;               // phases whose records are held below (0: use Job::rec in global memory)
   SchedRec train_rec[PARAM_TRAIN_PH];
   SchedRec dec_rec[PARAM_DEC_PH];
+  const unsigned char* maps; int nmaps;     // TMA descriptors (128 bytes each) that the launch is the first to use
 };
 static_assert(sizeof(Ctx) <= 32764, "kernel parameter too large");
 
