@@ -144,10 +144,11 @@ __device__ __noinline__ void gemm_run(const PhaseDesc& d, int task, unsigned cha
 }
 
 // ---------------------------------------------------------------------------------------------- attention (one task per (b, h))
-// Four lanes share a row: lane l takes every fourth partner position, with the row's own vectors in registers; rows of scores are one
-// word longer than T so that the rows of a warp fall into different banks.
-__host__ __device__ constexpr size_t attn_fwd_smem(int T, int DH) { return (size_t)(3 * T * DH + T * (T + 1)) * 4; }
-__host__ __device__ constexpr size_t attn_bwd_smem(int T, int DH) { return (size_t)(5 * T * DH + 2 * T * (T + 1) + T) * 4; }
+// Four lanes share a row: lane l takes every fourth partner position, with the row's own vectors in registers; rows of scores have an odd
+// length so that the rows of a warp fall into different banks (an even T is padded by a word; T = 151, the longest that fits a block, is odd).
+__host__ __device__ constexpr int score_row(int T) { return T | 1; }
+__host__ __device__ constexpr size_t attn_fwd_smem(int T, int DH) { return (size_t)(3 * T * DH + T * score_row(T)) * 4; }
+__host__ __device__ constexpr size_t attn_bwd_smem(int T, int DH) { return (size_t)(5 * T * DH + 2 * T * score_row(T) + T) * 4; }
 
 template <int DH> __device__ __forceinline__ void ld_row(const float* p, float (&f)[DH]) {
 #pragma unroll
@@ -176,7 +177,7 @@ template <int DH> __device__ __forceinline__ void load_heads(float* dst, const f
 
 template <int DH>
 __device__ __forceinline__ void attn_fwd_task(const float* qkv, float* o, float* lse, int b, int h, int T, int H, unsigned char* smem) {
-  const int D = H * DH, ld = 3 * D, S = T + 1;
+  const int D = H * DH, ld = 3 * D, S = score_row(T);
   float* sq = reinterpret_cast<float*>(smem); float* sk = sq + T * DH; float* sv = sk + T * DH; float* sp = sv + T * DH;
   const float scale = rsqrtf((float)DH);
   const float* base = qkv + (size_t)b * T * ld + h * DH;
@@ -217,7 +218,7 @@ __device__ __forceinline__ void attn_fwd_task(const float* qkv, float* o, float*
 template <int DH>
 __device__ __forceinline__ void attn_bwd_task(const float* qkv, const float* o, const float* dO, const float* lse, float* dqkv,
                                               int b, int h, int T, int H, unsigned char* smem) {
-  const int D = H * DH, ld = 3 * D, S = T + 1;
+  const int D = H * DH, ld = 3 * D, S = score_row(T);
   float* sq = reinterpret_cast<float*>(smem); float* sk = sq + T * DH; float* sv = sk + T * DH; float* sdo = sv + T * DH; float* so = sdo + T * DH;
   float* sp = so + T * DH; float* sds = sp + T * S;
   const float scale = rsqrtf((float)DH);
