@@ -312,3 +312,31 @@ def test_a_workspace_is_reused_with_other_operands_shapes_sizes_and_threads(ofa)
     for t in ts:
         t.join()
     assert not errors, errors[0]
+
+
+def test_layernorm_backward_without_allocations_under_capture(ofa):
+    """Both launches, the second a programmatic dependent one, recorded into a graph and replayed: the same bits as a direct call."""
+    lib = ofa.capi.load()
+    n, D = 1003, 768
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, dy = (torch.randn(n, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    gamma = torch.randn(D, generator=g, device="cuda").bfloat16()
+    mean, rstd = x.float().mean(1), torch.rsqrt(x.float().var(1, unbiased=False) + 1e-5)
+
+    def call(dx, dg):
+        rc = lib.ofa_ln_bwd_noalloc(dx.data_ptr(), dg.data_ptr(), dy.data_ptr(), x.data_ptr(), mean.data_ptr(), rstd.data_ptr(), gamma.data_ptr(), None, n, D, 0,
+                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == ofa.capi.OK, lib.ofa_noalloc_last_error().decode()
+
+    want, wdg = torch.empty_like(x), torch.empty(D, device="cuda")
+    call(want, wdg)
+    torch.cuda.synchronize()
+    dx, dg = torch.zeros_like(x), torch.zeros(D, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(dx, dg)
+    for _ in range(3):
+        dx.zero_(); dg.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(dx, want) and torch.equal(dg, wdg)
