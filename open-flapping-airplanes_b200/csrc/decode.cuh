@@ -39,27 +39,12 @@ __device__ __forceinline__ uint4 ldw16(const void* p) {   // streaming 16-byte l
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
   return r;
 }
-__device__ __forceinline__ void ldwv(const bf16* p, float* f) { unpack8(ldw16(p), f); }
-__device__ __forceinline__ void ldwv(const float* p, float* f) {
-  const uint4 u = ldw16(p); f[0] = __uint_as_float(u.x); f[1] = __uint_as_float(u.y); f[2] = __uint_as_float(u.z); f[3] = __uint_as_float(u.w);
-}
 template <class T> __device__ __forceinline__ void cvt16(uint4 u, float* f);      // 16 raw bytes -> Vec<T>::N floats
 template <> __device__ __forceinline__ void cvt16<bf16>(uint4 u, float* f) { unpack8(u, f); }
 template <> __device__ __forceinline__ void cvt16<float>(uint4 u, float* f) { f[0] = __uint_as_float(u.x); f[1] = __uint_as_float(u.y); f[2] = __uint_as_float(u.z); f[3] = __uint_as_float(u.w); }
 template <class T> __device__ __forceinline__ float ldcg_f(const T* p);
 template <> __device__ __forceinline__ float ldcg_f<bf16>(const bf16* p) { return __bfloat162float(__ldcg(p)); }
 template <> __device__ __forceinline__ float ldcg_f<float>(const float* p) { return __ldcg(p); }
-
-// L2 prefetch of part `part` of `nparts` of a contiguous byte range (128-byte lines), spread over the 256 threads. Weights do
-// not depend on activations, so every decode task pulls a share of the NEXT phase's weights towards L2 before it starts its
-// own dependent work; the next phase then streams from L2 instead of DRAM. Hint only: it never changes results.
-__device__ __forceinline__ void l2_prefetch_share(const void* base, size_t bytes, int part, int nparts) {
-  const size_t lines = (bytes + 127) >> 7;
-  const size_t per = (lines + nparts - 1) / nparts;
-  const size_t lo = per * part, hi = lo + per < lines ? lo + per : lines;
-  const char* b = reinterpret_cast<const char*>(base);
-  for (size_t i = lo + threadIdx.x; i < hi; i += NTHR) asm volatile("prefetch.global.L2 [%0];" ::"l"(b + (i << 7)));
-}
 
 __device__ __forceinline__ bool better(float a, int ai, float b, int bi) {
   if (a != a) return false;
@@ -128,8 +113,6 @@ __device__ __forceinline__ void block_init(unsigned char* smem, int Tctx) {
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void ld2(const bf16* p, float& a, float& b) { const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); a = f.x; b = f.y; }
-__device__ __forceinline__ void ld2(const float* p, float& a, float& b) { const float2 f = *reinterpret_cast<const float2*>(p); a = f.x; b = f.y; }
 
 // ---------------------------------------------------------------------------------------------- prefetch (runs while the task's dependencies are still pending)
 // Starts the bulk copies of task (kind, layer, t) into the weight buffer; warp 0 only. Returns true (uniformly for the block)
