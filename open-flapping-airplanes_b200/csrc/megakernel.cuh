@@ -299,7 +299,7 @@ __device__ void job_loop(const Ctx& C, const Job& J, int job_id, unsigned char* 
   const unsigned total = (unsigned)J.nsteps * (unsigned)J.tasks_per_step;
   gemm_tc::GemmPipe gp; gp.stage_count[0] = gp.stage_count[1] = gp.tile_count[0] = gp.tile_count[1] = gp.tmem_base = 0;
   const bool use_tc = IsBf16<T>::value && job_id == 0;
-  attn_tc::AttnPipe ap; ap.tasks = ap.stages = ap.stages2 = ap.a = ap.b = ap.done = 0;
+  attn_tc::AttnPipe ap; ap.tasks = ap.ring = ap.stages2 = ap.a = ap.b = ap.done = 0;
   uint32_t bulk_uses = 0;                            // uses of the block's bulk-copy barrier (control area byte 104)
   uint32_t adam_tiles = 0;                           // tiles the block's AdamW tasks have staged (three barriers at control area byte 224)
   uint32_t ce_chunks = 0;                            // chunks the block's streamed cross-entropy tasks have staged (barriers at bytes 112, 120, 160, 168)
