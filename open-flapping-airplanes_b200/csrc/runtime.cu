@@ -573,9 +573,9 @@ bool build_train_graph(ofa_ctx* c) {
       addp("grads ready " + std::to_string(bi), d, buckets[bi].producers, {});
     };
 
-    // ---- optimizer helpers. Optionally (cfg.adam_interleave, and only without external gradient synchronisation) a layer's
-    // AdamW is placed INSIDE the backward pass, one layer below the one it updates, instead of after it. Off by default: on the
-    // full model it measured 0.5-0.9 % slower per step (the memory-bound tasks delay the chain of small backward phases).
+    // ---- optimizer helpers. cfg.adam_interleave = 1 (only without external gradient synchronisation) places a layer's AdamW INSIDE the
+    // backward pass, one layer below the one it updates, instead of after it. On the full model it measured 0.5-0.9 % slower per step (the
+    // memory-bound tasks delay the chain of small backward phases).
     auto gate = [&](const std::string& adam_name, std::vector<std::string> deps) {
       if (!ext) return deps;
       for (size_t bi = 0; bi < buckets.size(); bi++) for (const std::string& a : buckets[bi].adam_phases) if (a == adam_name) return std::vector<std::string>{"allreduce done " + std::to_string(bi)};
@@ -603,17 +603,20 @@ bool build_train_graph(ofa_ctx* c) {
       addp("adamw L" + std::to_string(l), mkadam(off, end - off, nd), gate("adamw L" + std::to_string(l), deps), {});
     };
     const bool interleave_adam = train && !ext && cfg.adam_interleave == 1;
-    // cfg.adam_interleave = n >= 2 (off by default: measured 0.9-1.5 % slower per step for n = 6..48, because an AdamW task is bound
-    // by what one block keeps in flight - 88 us beside GEMMs against 100 us beside 231 others like it - so moving it buys little and
-    // costs the chain its earliest blocks): AdamW trickles through the backward pass. As soon as a tensor group's gradient is final its
-    // update is queued, and after every backward phase up to n optimizer tasks are emitted as a small phase of their own. A
-    // backward phase of 192 strips leaves 40 of the 232 training blocks without a ticket; they take these tasks instead of
-    // waiting, and a memory-bound task that runs beside GEMMs instead of beside 231 others like it finishes several times
-    // sooner. The group's usual phase name goes to a 1-task phase behind its last chunk that waits for all of them, so the next
-    // step's forward pass still has one thing to wait for.
+    // n >= 2: AdamW trickles through the backward pass. As soon as a tensor group's gradient is final its update is queued, and after every
+    // backward phase up to n optimizer tasks are emitted as a small phase of their own, which blocks without a task of the chain take. The
+    // group's usual phase name goes to a 1-task phase behind its last chunk that waits for all of them, so the next step's forward pass
+    // still has one thing to wait for.
+    // n = 0, the default, chooses by how many blocks the chain's [tokens, d_model] products leave idle (us per step with 0 / 16 / 32 / 64 tasks, 296
+    // blocks): 384 tokens (18 tiles), 3 layers 871 / 858 / 846 / 833, 768 937 / 913 / 871 / 881, 1,024 1,370 / 1,301 / 1,303 / 1,337, 2,048 1,561 / 1,489 /
+    // 1,507 / 1,540; GPT-S with 512 tokens 3,867 / 3,691 / 3,707 / 3,735, 1,024 4,256 / 4,051 / 4,070 / 4,092, 3,072 (144 tiles) 5,616 / 5,606 / 5,651 /
+    // 5,713, 4,096 (192 tiles) 6,583 / 6,575 / 6,557 / 6,641 (0.9-1.5 % slower on 116 SMs: an AdamW task is bound by what one block keeps in flight, so
+    // moving it buys little there and costs the chain its earliest blocks). So 32 up to an eighth of the blocks, 16 up to half of them, else none.
+    const int chain_tiles = bf ? (int)(N / 128 * (D / 128)) : train_blocks;
+    const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : 8 * chain_tiles <= train_blocks ? 32 : 2 * chain_tiles <= train_blocks ? 16 : -1;
     struct AdamItem { std::string name; size_t off, n; std::vector<Span> nd; std::vector<std::string> deps, parts; int next_task = 0, chunks = 0; };
     std::vector<AdamItem> adam_q; size_t adam_q_head = 0;
-    const int trickle_n = (train && !ext && cfg.adam_interleave >= 2) ? cfg.adam_interleave : 0;
+    const int trickle_n = (train && !ext && interleave >= 2) ? interleave : 0;
     bool in_trickle = false;
     auto mkadam_range = [&](size_t off, size_t n, const std::vector<Span>& nodecay_abs) {
       std::vector<Span> clipped;

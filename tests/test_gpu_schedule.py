@@ -162,3 +162,23 @@ def test_abort_and_wait_timeout(ofa, oracle):
     assert mk.steps_done == done_before + 300
     assert live["steps"] >= 0
     mk.close()
+
+
+@pytest.mark.parametrize("ctx,layers,vocab", [(1024, 12, 50304), (384, 3, 1152)])
+def test_spread_adamw_gives_the_same_bits(ofa, ctx, layers, vocab):
+    """A short batch spreads AdamW through the backward pass: losses and weights after two steps are those of the optimizer behind it."""
+    out = []
+    for spread in (0, -1):
+        cfg = ofa.default_config("gpt_s")
+        cfg.vocab = cfg.valid_vocab = vocab
+        cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.adam_interleave = layers, ctx, 1, spread
+        mk = ofa.Megakernel(cfg)
+        g = np.random.default_rng(3)
+        mk.load_weights((g.standard_normal(mk.num_params, dtype=np.float32) * 0.02))
+        mk.set_tokens(g.integers(0, vocab, size=1 << 14, dtype=np.uint32))
+        mk.run(2)
+        out.append((len(mk.phases()), mk.losses()[-2:].copy(), mk.read_weights()))
+        mk.close()
+    assert out[0][0] > out[1][0]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_array_equal(out[0][2], out[1][2])

@@ -165,3 +165,17 @@ def test_row_block_dependencies_follow_the_layer_chain(ofa):
     tiny = plan(ofa, "tiny")
     assert all(not any(tiny.phase_dep_grain(i)[1]) for i in range(len(tiny.phases())))
     tiny.close()
+
+
+@pytest.mark.parametrize("ctx,batch,kw,most", [(128, 1, {}, 32), (768, 1, {}, 32), (896, 1, {}, 16), (1024, 3, {}, 16), (640, 5, {}, 0), (1024, 4, {}, 0), (768, 1, dict(adam_interleave=-1), 0),
+                                               (768, 1, dict(adam_interleave=8), 8), (1024, 1, dict(dp_world=2, grad_bf16=1, ext_sync=1), 0)])
+def test_adamw_is_spread_by_the_blocks_the_chain_leaves_idle(ofa, ctx, batch, kw, most):
+    """By default AdamW trickles through the backward pass while the chain's [tokens, d_model] products (128 x 128 tiles) fill at most half of
+    the 296 blocks, 32 tasks at a time up to an eighth of them (37 tiles), else 16."""
+    mk = plan(ofa, "gpt_s", ctx_len=ctx, batch=batch, **kw)
+    chunks = [p["ntasks"] for p in mk.phases() if p["kind"] == 13 and " ." in p["name"]]
+    if most == 0:
+        assert not chunks
+    else:
+        assert max(set(chunks), key=chunks.count) == most             # the last piece of a group may hold a rest, and what is left at the end goes out in one piece
+    mk.close()
