@@ -41,23 +41,31 @@ __device__ __forceinline__ void panel_kmajor(float* dst, const float* X, int ld,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool vec = aligned_rows(X, ld, K), in = r0 + lane < rows;
   const float* row = X + (size_t)(r0 + lane) * ld;
+  auto put = [&](int k, const float4 v) { dst[k * GS + lane] = v.x; dst[(k + 1) * GS + lane] = v.y; dst[(k + 2) * GS + lane] = v.z; dst[(k + 3) * GS + lane] = v.w; };
+  if (vec) {
 #pragma unroll 4
-  for (int k = warp * 4; k < kc; k += NTHR / 8) {
-    const float4 v = in ? row4(row, k0 + k, K, vec) : zero4();
-    dst[k * GS + lane] = v.x; dst[(k + 1) * GS + lane] = v.y; dst[(k + 2) * GS + lane] = v.z; dst[(k + 3) * GS + lane] = v.w;
+    for (int k = warp * 4; k < kc; k += NTHR / 8) put(k, in ? row4(row, k0 + k, K, true) : zero4());
+  } else {
+#pragma unroll 1
+    for (int k = warp * 4; k < kc; k += NTHR / 8) put(k, in ? row4(row, k0 + k, K, false) : zero4());
   }
 }
 // panel dst[k][GT] of an operand stored [K][cols]
 __device__ __forceinline__ void panel_nmajor(float* dst, const float* X, int ld, int c0, int cols, int k0, int kc, int K) {
   const int c = (threadIdx.x & 7) * 4;
   const bool vec = aligned_rows(X, ld, cols);
+  auto put = [&](int k, bool v4) { *reinterpret_cast<float4*>(dst + k * GS + c) = k0 + k < K ? row4(X + (size_t)(k0 + k) * ld, c0 + c, cols, v4) : zero4(); };
+  if (vec) {
 #pragma unroll 4
-  for (int k = threadIdx.x >> 3; k < kc; k += NTHR / 8) {
-    const float4 v = k0 + k < K ? row4(X + (size_t)(k0 + k) * ld, c0 + c, cols, vec) : zero4();
-    *reinterpret_cast<float4*>(dst + k * GS + c) = v;
+    for (int k = threadIdx.x >> 3; k < kc; k += NTHR / 8) put(k, true);
+  } else {
+#pragma unroll 1
+    for (int k = threadIdx.x >> 3; k < kc; k += NTHR / 8) put(k, false);
   }
 }
-__device__ __forceinline__ void epilogue1(const GemmArgs& g, int epi, int m, int n, float v) {
+// Out of line, like the unaligned forms of the loads above in loops of their own: a block runs through most of the library in a step, so what a task's code
+// occupies beyond what it executes often is fetched anew each time. The char model's step: 407 -> 376 us, a weight gradient of 64 x 256 13.1 -> 8.7 us.
+__device__ __noinline__ void epilogue1(const GemmArgs& g, int epi, int m, int n, float v) {
   float* C = reinterpret_cast<float*>(g.C); float* aux = reinterpret_cast<float*>(g.aux);
   const size_t ci = (size_t)m * g.ldc + n, ai = (size_t)m * g.ldaux + n;
   switch (epi) {
@@ -95,7 +103,7 @@ __device__ __forceinline__ void gemm_task(const GemmArgs& g, int epi, int tiles_
 #pragma unroll
   for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(red + kg * GT * GT + (ty * 4 + i) * GT + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   __syncthreads();
-#pragma unroll
+#pragma unroll 1
   for (int q = 0; q < 4; q++) {                         // a warp's 32 outputs are one row of the tile
     const int o = tid + q * NTHR, m = m0 + o / GT, n = n0 + o % GT;
     const float v = (red[o] + red[GT * GT + o]) + (red[2 * GT * GT + o] + red[3 * GT * GT + o]);
@@ -114,22 +122,34 @@ __device__ __forceinline__ void gemm_task_tn(const GemmArgs& g, int epi, int til
 #pragma unroll
   for (int i = 0; i < 4; i++) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
   int k = kg;
-  for (; k + 7 * 16 < g.K; k += 8 * 16) {
-    float4 a[8], b[8];
+  if (va && vb) {
+#pragma unroll 1
+    for (; k + 7 * 16 < g.K; k += 8 * 16) {
+      float4 a[8], b[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      a[u] = row4(A + (size_t)(k + u * 16) * g.lda, m0 + ty * 4, g.M, va);
-      b[u] = row4(B + (size_t)(k + u * 16) * g.ldb, n0 + tx * 4, g.N, vb);
+      for (int u = 0; u < 8; u++) {
+        a[u] = row4(A + (size_t)(k + u * 16) * g.lda, m0 + ty * 4, g.M, true);
+        b[u] = row4(B + (size_t)(k + u * 16) * g.ldb, n0 + tx * 4, g.N, true);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) fma16(acc, a[u], b[u]);
     }
-#pragma unroll
-    for (int u = 0; u < 8; u++) fma16(acc, a[u], b[u]);
   }
+#pragma unroll 1
+  for (; k + 3 * 16 < g.K; k += 4 * 16) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) { a[u] = row4(A + (size_t)(k + u * 16) * g.lda, m0 + ty * 4, g.M, va); b[u] = row4(B + (size_t)(k + u * 16) * g.ldb, n0 + tx * 4, g.N, vb); }
+#pragma unroll
+    for (int u = 0; u < 4; u++) fma16(acc, a[u], b[u]);
+  }
+#pragma unroll 1
   for (; k < g.K; k += 16) fma16(acc, row4(A + (size_t)k * g.lda, m0 + ty * 4, g.M, va), row4(B + (size_t)k * g.ldb, n0 + tx * 4, g.N, vb));
 #pragma unroll
   for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(red + kg * 256 + (ty * 4 + i) * GT_TN + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   __syncthreads();
   float v = 0.f;
-#pragma unroll
+#pragma unroll 4
   for (int q = 0; q < 16; q++) v += red[q * 256 + tid];
   const int m = m0 + tid / GT_TN, n = n0 + tid % GT_TN;
   if (m < g.M && n < g.N) epilogue1(g, epi, m, n, v);
