@@ -329,6 +329,24 @@ def test_attention_bf16_forward_with_growing_row_maxima(ofa, K, oracle):
     assert np.abs(d_lse.download() - lse_ref.numpy()).max() <= 2e-3 * max(1.0, float(lse_ref.abs().max()))
 
 
+def test_attention_bf16_row_sums_add_neighbours_first(ofa, K):
+    """A row's 64 exponentials per key tile are summed by neighbours (1 addition), in four chains of eight such pairs (7) and across the chains (2), then
+    the tiles are added up. With one probability of 1 and all others 0.98 * 2^-24, an order that adds them to the 1 one by one loses all of its chain.
+    Bound: every addition whose result lies near 1 rounds by at most 2^-24; ten of them lie on the way of the 1 within its tile, one more per further
+    tile. The error of the exponentials themselves (2^-22 of 127 * 2^-24) is nothing beside that, and so is logf's (1 ulp of 7e-6)."""
+    T, D = 128, 768
+    qkv = torch.zeros(T, 3, 12, 64)
+    qkv[:, 0, :, :2] = 1.0
+    qkv[1:, 1, :, 0], qkv[1:, 1, :, 1] = -133.0, -0.25                     # score -133.25 * 0.125 * log2(e) = -24.03
+    qkv[:, 2] = 1.0
+    d_qkv = ofa.DeviceBuffer.from_host(qkv.reshape(T, 3 * D).numpy(), "bf16")
+    d_o = ofa.DeviceBuffer((T, D), "bf16"); d_lse = ofa.DeviceBuffer((1, 12, T), np.float32)
+    ofa.run_phases(K.DTYPE_BF16, dict(DIMS_S, ctx_len=T, batch=1), [ofa.phase(K.TK_ATT_FWD, [d_qkv, d_o, d_lse])])
+    exact = np.log1p(np.arange(T) * np.exp(-133.25 * 0.125))
+    assert np.abs(d_lse.download() - exact).max() <= 11 * 2.0 ** -24
+    assert np.abs(d_o.download() - 1.0).max() <= 2.0 ** -8
+
+
 def test_attention_fp32_forward_backward(ofa, K, oracle):
     B, T, H, dh = 4, 64, 4, 16
     D = H * dh
