@@ -613,7 +613,10 @@ bool build_train_graph(ofa_ctx* c) {
     // 5,713, 4,096 (192 tiles) 6,583 / 6,575 / 6,557 / 6,641 (0.9-1.5 % slower on 116 SMs: an AdamW task is bound by what one block keeps in flight, so
     // moving it buys little there and costs the chain its earliest blocks). So 32 up to an eighth of the blocks, 16 up to half of them, else none.
     const int chain_tiles = bf ? (int)(N / 128 * (D / 128)) : train_blocks;
-    const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : 8 * chain_tiles <= train_blocks ? 32 : 2 * chain_tiles <= train_blocks ? 16 : -1;
+    // Not beside a serving job: its tokens/s fall by what the optimizer takes from it closer together (24 SMs, us per step and tokens/s without / with: 384
+    // tokens 4,272 and 2,286 / 3,972 and 2,216, 1,024 4,764 and 2,215 / 4,644 and 2,153, 1,536 4,817 and 2,182 / 4,717 and 2,117, 2,304 5,556 and
+    // 2,178 / 5,579 and 2,111). Which of the two counts more is the caller's to say.
+    const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : cfg.use_decode ? -1 : 8 * chain_tiles <= train_blocks ? 32 : 2 * chain_tiles <= train_blocks ? 16 : -1;
     struct AdamItem { std::string name; size_t off, n; std::vector<Span> nd; std::vector<std::string> deps, parts; int next_task = 0, chunks = 0; };
     std::vector<AdamItem> adam_q; size_t adam_q_head = 0;
     const int trickle_n = (train && !ext && interleave >= 2) ? interleave : 0;

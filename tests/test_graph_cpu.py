@@ -179,3 +179,15 @@ def test_adamw_is_spread_by_the_blocks_the_chain_leaves_idle(ofa, ctx, batch, kw
     else:
         assert max(set(chunks), key=chunks.count) == most             # the last piece of a group may hold a rest, and what is left at the end goes out in one piece
     mk.close()
+
+
+SPLIT = dict(infer_sms=24, reserved_sms=8, train_sms=116)
+
+
+@pytest.mark.parametrize("ctx,batch,kw,most", [(384, 1, dict(SPLIT, use_decode=1), 0), (1024, 1, dict(use_decode=1), 0), (384, 1, dict(SPLIT, use_decode=1, adam_interleave=16), 16)])
+def test_adamw_is_not_spread_by_default_beside_a_serving_job(ofa, ctx, batch, kw, most):
+    """The serving job's rate falls when the optimizer runs beside the backward pass: only on request."""
+    mk = plan(ofa, "gpt_s", ctx_len=ctx, batch=batch, **kw)
+    chunks = [p["ntasks"] for p in mk.phases() if p["kind"] == 13 and " ." in p["name"]]
+    assert max(set(chunks), key=chunks.count) == most if most else not chunks
+    mk.close()
