@@ -607,16 +607,23 @@ bool build_train_graph(ofa_ctx* c) {
     // backward phase up to n optimizer tasks are emitted as a small phase of their own, which blocks without a task of the chain take. The
     // group's usual phase name goes to a 1-task phase behind its last chunk that waits for all of them, so the next step's forward pass
     // still has one thing to wait for.
-    // n = 0, the default, chooses by how many blocks the chain's [tokens, d_model] products leave idle (us per step with 0 / 16 / 32 / 64 tasks, 296
-    // blocks): 384 tokens (18 tiles), 3 layers 871 / 858 / 846 / 833, 768 937 / 913 / 871 / 881, 1,024 1,370 / 1,301 / 1,303 / 1,337, 2,048 1,561 / 1,489 /
-    // 1,507 / 1,540; GPT-S with 512 tokens 3,867 / 3,691 / 3,707 / 3,735, 1,024 4,256 / 4,051 / 4,070 / 4,092, 3,072 (144 tiles) 5,616 / 5,606 / 5,651 /
-    // 5,713, 4,096 (192 tiles) 6,583 / 6,575 / 6,557 / 6,641 (0.9-1.5 % slower on 116 SMs: an AdamW task is bound by what one block keeps in flight, so
-    // moving it buys little there and costs the chain its earliest blocks). So 32 up to an eighth of the blocks, 16 up to half of them, else none.
-    const int chain_tiles = bf ? (int)(N / 128 * (D / 128)) : train_blocks;
+    // n = 0, the default, chooses by how many blocks the chain's [tokens, d_model] products (128 x 128 tiles) leave idle. us per step with none / 16 / 32 tasks after
+    // a phase, 12 layers and V = 50,304 (then 3 layers and V = 1,152 where measured):
+    //   whole GPU, 296 blocks    18 tiles  3,812 / 3,679 / 3,693 (840 / 836 / 806)    24 tiles  3,852 / 3,690 / 3,689    48 tiles  4,228 / 4,043 / 4,040
+    //                            96 tiles  4,834 / 4,683 / 4,703 (1,058 / 1,033 / 1,013)    108 tiles  4,868 / 4,781 / 4,833
+    //                            120 tiles 5,009 / 4,990 / 5,033 (1,072 / 1,074 / 1,068)    144 tiles  5,794 / 5,803 / 5,851 (1,232 / 1,234 / 1,215)
+    //   116 of 148 SMs, 232      18 tiles  3,915 / 3,676 / 3,692    48 tiles  4,506 / 4,389 / 4,407    72 tiles  4,611 / 4,514 / 4,566 (1,014 / 994 / 980)
+    //                            96 tiles  5,230 / 5,232 / 5,318 (1,144 / 1,143 / 1,132)    108 tiles  5,338 / 5,380 / 5,420
+    // So 32 up to an eighth of the blocks, where the smallest models gain most by it, and 16 above, up to half of them: from 0.4 of the blocks on there is next to
+    // nothing to gain. On a partition it costs there (an AdamW task is bound by what one block keeps in flight, and the chain loses its
+    // earliest blocks), so 16 only up to three eighths. How many phases come of it does not matter: scheduling records that no longer fit the kernel parameter are
+    // read from global memory at the same speed (14 layers, 48 tiles: 454 phases 4,557, 381 phases 4,557, not spread, 310 phases, 4,765; 12 layers, 396 phases 4,043 and 4,044).
     // Not beside a serving job: its tokens/s fall by what the optimizer takes from it closer together (24 SMs, us per step and tokens/s without / with: 384
     // tokens 4,272 and 2,286 / 3,972 and 2,216, 1,024 4,764 and 2,215 / 4,644 and 2,153, 1,536 4,817 and 2,182 / 4,717 and 2,117, 2,304 5,556 and
     // 2,178 / 5,579 and 2,111). Which of the two counts more is the caller's to say.
-    const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : cfg.use_decode ? -1 : 8 * chain_tiles <= train_blocks ? 32 : 2 * chain_tiles <= train_blocks ? 16 : -1;
+    const int chain_tiles = bf ? (int)(N / 128 * (D / 128)) : train_blocks;
+    const int most_tiles = train_blocks < c->nblocks ? train_blocks * 3 / 8 : train_blocks / 2;
+    const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : cfg.use_decode ? -1 : 8 * chain_tiles <= train_blocks ? 32 : chain_tiles <= most_tiles ? 16 : -1;
     struct AdamItem { std::string name; size_t off, n; std::vector<Span> nd; std::vector<std::string> deps, parts; int next_task = 0, chunks = 0; };
     std::vector<AdamItem> adam_q; size_t adam_q_head = 0;
     const int trickle_n = (train && !ext && interleave >= 2) ? interleave : 0;

@@ -191,3 +191,12 @@ def test_adamw_is_not_spread_by_default_beside_a_serving_job(ofa, ctx, batch, kw
     chunks = [p["ntasks"] for p in mk.phases() if p["kind"] == 13 and " ." in p["name"]]
     assert max(set(chunks), key=chunks.count) == most if most else not chunks
     mk.close()
+
+
+@pytest.mark.parametrize("ctx,batch,most", [(512, 1, 32), (640, 1, 16), (896, 2, 16), (1024, 2, 0), (768, 3, 0)])
+def test_adamw_is_spread_less_on_a_partition(ofa, ctx, batch, most):
+    """On 116 SMs (232 blocks) without a serving job: 32 tasks up to 29 tiles of the chain's products, 16 up to 87 (three eighths of the blocks)."""
+    mk = plan(ofa, "gpt_s", ctx_len=ctx, batch=batch, **dict(SPLIT, infer_sms=0))
+    chunks = [p["ntasks"] for p in mk.phases() if p["kind"] == 13 and " ." in p["name"]]
+    assert max(set(chunks), key=chunks.count) == most if most else not chunks
+    mk.close()
