@@ -182,3 +182,38 @@ def test_spread_adamw_gives_the_same_bits(ofa, ctx, layers, vocab):
     assert out[0][0] > out[1][0]
     np.testing.assert_array_equal(out[0][1], out[1][1])
     np.testing.assert_array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("layers,vocab,ctx,batch,kw,env,shuffle", [
+    (3, 8192, 384, 2, dict(tied_head=1, grad_bf16=1), None, 0),
+    (3, 8192, 384, 2, dict(), None, 31337),
+    (3, 1152, 384, 1, dict(), "OFA_B200_GLOBAL_RECS", 0),
+    (16, 1152, 384, 1, dict(), None, 0),                                                            # 412 phases: more records than fit the kernel parameter
+    (3, 1152, 384, 1, dict(infer_sms=24, reserved_sms=8, train_sms=116, use_decode=1, n_prompt=6, adam_interleave=16), None, 0)])
+def test_spread_adamw_gives_the_same_bits_in_every_form(ofa, monkeypatch, layers, vocab, ctx, batch, kw, env, shuffle):
+    """Tied head with bf16 gradients, permuted task order, scheduling records in global memory (asked for, or because they do not fit), live serving."""
+    lib = ofa.capi.load()
+    out = []
+    if env:
+        monkeypatch.setenv(env, "1")
+    try:
+        for spread in (kw.get("adam_interleave", 0), -1):
+            lib.ofa_debug_set_task_shuffle(shuffle if spread >= 0 else 0)
+            cfg = ofa.default_config("gpt_s")
+            cfg.vocab = cfg.valid_vocab = vocab
+            cfg.n_layer, cfg.ctx_len, cfg.batch = layers, ctx, batch
+            for k, v in kw.items():
+                setattr(cfg, k, v)
+            cfg.adam_interleave = spread
+            mk = ofa.Megakernel(cfg)
+            g = np.random.default_rng(3)
+            mk.load_weights(g.standard_normal(mk.num_params, dtype=np.float32) * 0.02)
+            mk.set_tokens(g.integers(0, vocab, size=1 << 14, dtype=np.uint32))
+            mk.run(3)
+            out.append((len(mk.phases()), mk.losses()[-3:].copy(), mk.read_weights()))
+            mk.close()
+    finally:
+        lib.ofa_debug_set_task_shuffle(0)
+    assert out[0][0] > out[1][0]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_array_equal(out[0][2], out[1][2])

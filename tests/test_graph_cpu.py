@@ -200,3 +200,35 @@ def test_adamw_is_spread_less_on_a_partition(ofa, ctx, batch, most):
     chunks = [p["ntasks"] for p in mk.phases() if p["kind"] == 13 and " ." in p["name"]]
     assert max(set(chunks), key=chunks.count) == most if most else not chunks
     mk.close()
+
+
+@pytest.mark.parametrize("kw", [dict(ctx_len=1024), dict(ctx_len=384), dict(ctx_len=384, tied_head=1, grad_bf16=1), dict(ctx_len=384, vocab=1152, valid_vocab=1152, n_layer=16), dict(SPLIT, use_decode=1, adam_interleave=16)])
+def test_spread_adamw_comes_after_every_reader_of_its_weights(ofa, kw):
+    """Each optimizer piece of a tensor group has all phases of its step that read the group's weights, or write its gradients, among its ancestors."""
+    mk = plan(ofa, "gpt_s", **{"batch": 1, **kw})
+    names = [p["name"] for p in mk.phases()]
+    deps = [[d for d, delta in mk.phase_deps(i) if delta == 0] for i in range(len(names))]
+    above = []
+    for i in range(len(names)):
+        above.append(set().union({names[d] for d in deps[i]}, *(above[d] for d in deps[i])) if deps[i] else set())
+    L, pieces = mk.cfg.n_layer, 0
+    for i, p in enumerate(mk.phases()):
+        if p["kind"] != 13:
+            continue
+        group = p["name"][len("adamw "):].split(" ")[0]
+        pieces += " ." in p["name"]
+        if group.startswith("L"):
+            need = {f"{group} {n}" for n in ("ln1", "qkv", "wo+res", "ln2", "up+gelu", "down+res", "dpre", "dWdown", "dln2", "dWup", "ln2 bwd", "dgamma2", "dO", "dWo", "dln1", "dWqkv", "ln1 bwd", "dgamma1")}
+            if group == f"L{L - 1}":
+                need |= {"lnf", "lnf bwd", "lnf dgamma"}
+        elif group == "head":
+            need = {"logits", "head dX", "head dW"}
+        elif group == "wte":
+            need = {"embed", "embed bwd wte"} | ({"logits", "head dX", "head dW"} if mk.cfg.tied_head else set())
+        else:
+            need = {"embed", "embed bwd wpe"}
+        assert need <= above[i], (p["name"], need - above[i])
+        if " ." in p["name"]:
+            assert p["name"] in above[names.index("step barrier")]
+    assert pieces > L
+    mk.close()
