@@ -335,7 +335,7 @@ def main():
             import re
             cat = {}
             for p in mk.phases():
-                key = re.sub(r"^L\d+ ", "L* ", p["name"]); key = re.sub(r"adamw L\d+", "adamw L*", key)
+                key = re.sub(r"^L\d+ ", "L* ", p["name"]); key = re.sub(r"adamw L\d+", "adamw L*", key); key = re.sub(r"^(adamw .*) (\.\d+|ready)$", r"\1", key)
                 c = cat.setdefault(key, [0, 0, 0]); c[0] += p["busy_ns"]; c[1] += p["ntasks"]; c[2] += p["wait_ns"]
             print("  per category (block-ms per step, share of busy, mean us per task, block-ms per step waiting for its dependencies):", file=sys.stderr)
             for k, (b, n, w) in sorted(cat.items(), key=lambda kv: -kv[1][0]):

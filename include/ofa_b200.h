@@ -62,7 +62,7 @@ typedef struct {
   int ext_sync;             /* 1: gradients are cut into buckets; the graph raises a "ready" flag per bucket and holds the bucket's AdamW until the matching "done" flag is raised from outside (the all-reduce) */
   int bucket_bytes;         /* target bucket size for ext_sync (0 = 25 MiB)                                       */
   int attn_legacy;          /* must be 0 (the field once selected mma.sync attention tasks kept for comparison; they are gone, the tensor-core tasks are checked against the oracle directly) */
-  int adam_interleave;      /* 0 (default): chosen by the number of tokens; 1 = each layer's AdamW phase inside the backward pass; n >= 2 = AdamW trickles through the backward pass, up to n tasks after every backward phase; -1 = after the backward pass */
+  int adam_interleave;      /* 0 (default): bf16 without ext_sync and without a serving job: n = 32 or 16 while the [tokens, d_model] products leave most of the training blocks idle, else -1; all others -1. 1 = each layer's AdamW phase inside the backward pass; n >= 2 = AdamW trickles through the backward pass, about n tasks after every backward phase (a group's last piece up to 1.5 n); -1 = after the backward pass */
   int head_dx_splitk;       /* 1: compute lm_head dX as K-split partial products + reduce (experimental, default 0)     */
   int gemm_nsub;            /* consecutive N tiles per GEMM task: n = strips of n 128-wide tiles; 0 = chosen per phase by waves over the blocks that train; 2000 + n = 256-wide tiles where N allows; 4000 + n = the same with a phase's tasks ordered along N first (also accepted as ofa_phase.nsub) */
   double timeout_s;         /* device-side bound for a wait on an external flag (0 = default 20 s); waits for dependencies inside the graph give up after 1.5 x this */

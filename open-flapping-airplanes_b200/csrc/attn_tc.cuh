@@ -10,7 +10,7 @@
 //   producer (warp 0, one thread)   TMA: the task's own 128-row tiles once, then per step two 64-row partner tiles
 //   issuers  (warps 1 and 2, one thread each)   warp 1, group A: scores (and dP) of the step into tensor memory, as far
 //                                   ahead of the softmax threads as the buffers allow;  warp 2, group B: the products that
-//                                   consume what the softmax threads wrote to shared memory. Two threads because one thread
+//                                   consume what the softmax threads wrote. Two threads because one thread
 //                                   issues a tcgen05.mma only every ~96 cycles (measured) and because the two groups wait
 //                                   for different things
 //   softmax  (warps 4-7)            thread = row = tensor-memory lane: reads group A's result with tcgen05.ld, writes bf16 operands for
@@ -229,7 +229,7 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
       tc_fence_after();
       // The row's 64 scores come to registers once, which frees their columns; half of them at a time becomes 16 packed pairs of probabilities,
       // which go back to tensor memory as the A operand of the product. Through shared memory each step paid a fence of the async
-      // proxy (200 clocks of a softmax thread's 2,100) and its 32 KB of tiles were missing in the ring. 4 x 12 x 1,024 rows: 30.8 -> 28.8 us.
+      // proxy (200 clocks of a softmax thread's 2,100); of its 32 KB of tiles 16 are the ring's fourth stage now, 16 are free. 4 x 12 x 1,024 rows: 30.8 -> 28.8 us.
       const uint32_t ts = tl + (c & 1) * 64;
       const bool need_mask = __any_sync(0xffffffffu, k0 + KTILE - 1 > qg);       // warp-uniform: only tiles on the diagonal
       uint32_t s0[32], s1[32];
