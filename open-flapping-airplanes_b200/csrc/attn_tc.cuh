@@ -41,7 +41,7 @@ enum { B_QFULL = 0, B_STFULL = 1, B_STEMPTY = 5, B_AFULL = 9, B_AFREE = 11, B_WF
 static_assert(BAR0 + 8 * NBAR <= CTRL_BYTES, "attention barriers do not fit the control area");
 __device__ __forceinline__ uint32_t bar(uint32_t base, int i) { return base + gemm_tc::BAR_OFFSET + BAR0 + 8u * (uint32_t)i; }
 
-// running state (identical in every thread): tasks, parity of the ring's next use per slot, stages loaded through the two-stage ring, steps
+// running state (in shared memory, read at the start of a task and advanced by thread 0 behind its closing barrier): tasks, parity of the ring's next use per slot, stages loaded through the two-stage ring, steps
 // (group A / softmax), forward PV tiles, backward tasks
 struct AttnPipe { uint32_t tasks, ring, stages2, a, b, done; };
 // A task's ring of NST stages begins at slot 0 whatever the task before used, so that tasks with different depths share the barriers: step i
@@ -54,8 +54,8 @@ template <int NST> __device__ __forceinline__ uint32_t ring_after(uint32_t ring,
 }
 
 __device__ __forceinline__ void block_init(AttnPipe& ap, unsigned char* smem) {
-  ap.tasks = ap.ring = ap.stages2 = ap.a = ap.b = ap.done = 0;
   if (threadIdx.x == 0) {
+    ap.tasks = ap.ring = ap.stages2 = ap.a = ap.b = ap.done = 0;
     const uint32_t base = smem_u32(smem);
     mbar_init(bar(base, B_QFULL), 1);
     for (int s = 0; s < 4; s++) { mbar_init(bar(base, B_STFULL + s), 1); mbar_init(bar(base, B_STEMPTY + s), 1); }
@@ -158,7 +158,8 @@ __device__ __forceinline__ void warp_arrive(uint32_t b) { __syncwarp(); if ((thr
 // same softmax; after the first tiles of a row the rescale is rare and the step is one pass over S.
 constexpr float RESCALE_LOG2 = 8.f;
 __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b, int h, int qt, int T, int H, unsigned char* smem,
-                                      AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, const EarlyTicket& et) {
+                                      AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
+  const AttnPipe a0 = ap;
   const int D = H * DH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = smem_u32(smem);
@@ -175,21 +176,21 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
       int j = 0;
       for (; j < n; j++) {
         const int s = j % NST;
-        if (!wait_or_abort(bar(base, B_STEMPTY + s), ring_parity<NST>(ap.ring, j) ^ 1, st, ST_MBAR_EMPTY_TIMEOUT, phase_id, task, j)) break;
+        if (!wait_or_abort(bar(base, B_STEMPTY + s), ring_parity<NST>(a0.ring, j) ^ 1, st, ST_MBAR_EMPTY_TIMEOUT, phase_id, task, j)) break;
         const uint32_t full = bar(base, B_STFULL + s);
         mbar_expect_tx(full, 16384);
         tma_load_2d(sSt + s * 16384, &mp->qkv64, full, D + h * DH, nrow0 + j * KTILE);
         tma_load_2d(sSt + s * 16384 + 8192, &mp->qkv64, full, 2 * D + h * DH, nrow0 + j * KTILE);
       }
       if (!aborted(st)) take_early_ticket(et);                               // the last copy of the task is on its way
-      if (aborted(st)) drain_ring<NST>(base, ap.ring, j);
+      if (aborted(st)) drain_ring<NST>(base, a0.ring, j);
     }
   } else if (warp == 1) {
     if (lane == 0) {                                                           // ---- issuer of the scores: up to two steps ahead of the softmax threads
-      bool ok = wait_or_abort(bar(base, B_QFULL), ap.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
+      bool ok = wait_or_abort(bar(base, B_QFULL), a0.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
       for (int j = 0; j < n && ok; j++) {
-        const uint32_t c = ap.a + j; const int s = j % NST;
-        ok = wait_or_abort(bar(base, B_STFULL + s), ring_parity<NST>(ap.ring, j), st, ST_MBAR_FULL_TIMEOUT, phase_id, task, j);
+        const uint32_t c = a0.a + j; const int s = j % NST;
+        ok = wait_or_abort(bar(base, B_STFULL + s), ring_parity<NST>(a0.ring, j), st, ST_MBAR_FULL_TIMEOUT, phase_id, task, j);
         if (ok && j >= 2) ok = wait_or_abort(bar(base, B_AFREE + (c & 1)), ((c - 2) >> 1) & 1, st, ST_MBAR_ACC_TIMEOUT, phase_id, task, j);
         if (!ok) break;
         tc_fence_after();
@@ -201,7 +202,7 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
     if (lane == 0) {                                                           // ---- issuer of the products: follows the softmax threads
       bool ok = true;
       for (int i = 0; i < n && ok; i++) {                                      // O += P_i V_i
-        const uint32_t c = ap.a + i, cb = ap.b + i; const int s = i % NST;
+        const uint32_t c = a0.a + i, cb = a0.b + i; const int s = i % NST;
         ok = wait_or_abort(bar(base, B_WFULL + (c & 1)), (c >> 1) & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 2000 + i);
         if (!ok) break;
         tc_fence_after();
@@ -216,12 +217,12 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     auto wait_pv = [&](int i) {                                               // product i has been added to the output rows
-      const uint32_t cb = ap.b + i;
+      const uint32_t cb = a0.b + i;
       ok = mbar_wait(bar(base, B_BFULL + (cb & 1)), (cb >> 1) & 1, st);
       ok = __all_sync(0xffffffffu, ok);
     };
     for (int j = 0; j < n && ok; j++) {
-      const uint32_t c = ap.a + j;
+      const uint32_t c = a0.a + j;
       const int k0 = j * KTILE;
       ok = mbar_wait(bar(base, B_AFULL + (c & 1)), (c >> 1) & 1, st);
       ok = __all_sync(0xffffffffu, ok);
@@ -316,16 +317,17 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
       lse[((size_t)b * H + h) * T + qg] = m * LN2 + logf(l);
     }
   }
-  ap.tasks += 1; ap.ring = ring_after<NST>(ap.ring, n); ap.a += (uint32_t)n; ap.b += (uint32_t)n;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (tid == 0) { ap.tasks = a0.tasks + 1; ap.ring = ring_after<NST>(a0.ring, n); ap.a = a0.a + (uint32_t)n; ap.b = a0.b + (uint32_t)n; }
 }
 
 // ---------------------------------------------------------------------------------------------- backward: dK, dV
 // Task (b, h, kt): 128 key rows k0 = kt*128; walks query blocks of 64 rows from the diagonal to the end of the sequence.
 __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int kt, int T, int H,
-                                           unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, const EarlyTicket& et) {
+                                           unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
+  const AttnPipe a0 = ap;
   const int D = H * DH, ld = 3 * D;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = smem_u32(smem);
@@ -334,7 +336,7 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
   const int k0 = kt * QTILE, nrow0 = b * T;
   const int i0 = k0 / KTILE, n = T / KTILE - i0;
   constexpr int NST = 2;
-  const uint32_t st0 = ap.stages2;                              // this task's ring has its own barriers and counter
+  const uint32_t st0 = a0.stages2;                              // this task's ring has its own barriers and counter
   if (warp == 0) {
     if (lane == 0) {                                                           // ---- producer
       fence_proxy_async();
@@ -358,9 +360,9 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
     }
   } else if (warp == 1) {
     if (lane == 0) {                                                           // ---- issuer of the scores: runs one step ahead of the softmax threads
-      bool ok = wait_or_abort(bar(base, B_QFULL), ap.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
+      bool ok = wait_or_abort(bar(base, B_QFULL), a0.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
       for (int i = 0; i < n && ok; i++) {
-        const uint32_t sc = st0 + i, c = ap.a + i; const int s = sc % NST;
+        const uint32_t sc = st0 + i, c = a0.a + i; const int s = sc % NST;
         ok = wait_or_abort(bar(base, B_ST2FULL + s), (sc / NST) & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, i);
         if (ok && i >= 1) ok = wait_or_abort(bar(base, B_AFREE + ((c - 1) & 1)), ((c - 1) >> 1) & 1, st, ST_MBAR_ACC_TIMEOUT, phase_id, task, i);
         if (!ok) break;
@@ -374,7 +376,7 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
     if (lane == 0) {                                                           // ---- issuer of the products: follows the softmax threads
       bool ok = true;
       for (int i = 0; i < n && ok; i++) {
-        const uint32_t sc = st0 + i, c = ap.a + i; const int s = sc % NST;
+        const uint32_t sc = st0 + i, c = a0.a + i; const int s = sc % NST;
         ok = wait_or_abort(bar(base, B_WFULL + (c & 1)), (c >> 1) & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 2000 + i);
         if (!ok) break;
         tc_fence_after();
@@ -389,7 +391,7 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
     const uint32_t tl = tmem + ((uint32_t)(e * 32) << 16);
     bool ok = true;
     for (int i = 0; i < n && ok; i++) {
-      const uint32_t sc = st0 + i, c = ap.a + i; const int s = sc % NST;
+      const uint32_t sc = st0 + i, c = a0.a + i; const int s = sc % NST;
       const int qi0 = (i0 + i) * KTILE;
       ok = mbar_wait(bar(base, B_ST2FULL + s), (sc / NST) & 1, st) && mbar_wait(bar(base, B_AFULL + (c & 1)), (c >> 1) & 1, st);   // lse, D of the stage; S^T, dP^T
       ok = __all_sync(0xffffffffu, ok);
@@ -434,7 +436,7 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
       fence_async_smem();
       warp_arrive(bar(base, B_WFULL + (c & 1)));
     }
-    if (ok) { ok = mbar_wait(bar(base, B_DONE), ap.done & 1, st); ok = __all_sync(0xffffffffu, ok); }
+    if (ok) { ok = mbar_wait(bar(base, B_DONE), a0.done & 1, st); ok = __all_sync(0xffffffffu, ok); }
     if (ok) {
       tc_fence_after();
 #pragma unroll
@@ -456,16 +458,17 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
       }
     }
   }
-  ap.tasks += 1; ap.stages2 += (uint32_t)n; ap.a += (uint32_t)n; ap.done += 1;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (tid == 0) { ap.tasks = a0.tasks + 1; ap.stages2 = a0.stages2 + (uint32_t)n; ap.a = a0.a + (uint32_t)n; ap.done = a0.done + 1; }
 }
 
 // ---------------------------------------------------------------------------------------------- backward: dQ
 // Task (b, h, qt): 128 query rows; walks key blocks of 64 rows from 0 to the diagonal.
 __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int qt, int T, int H,
-                                         unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, const EarlyTicket& et) {
+                                         unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
+  const AttnPipe a0 = ap;
   const int D = H * DH, ld = 3 * D;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = smem_u32(smem);
@@ -482,21 +485,21 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
       int j = 0;
       for (; j < n; j++) {
         const int s = j % NST;
-        if (!wait_or_abort(bar(base, B_STEMPTY + s), ring_parity<NST>(ap.ring, j) ^ 1, st, ST_MBAR_EMPTY_TIMEOUT, phase_id, task, j)) break;
+        if (!wait_or_abort(bar(base, B_STEMPTY + s), ring_parity<NST>(a0.ring, j) ^ 1, st, ST_MBAR_EMPTY_TIMEOUT, phase_id, task, j)) break;
         const uint32_t full = bar(base, B_STFULL + s);
         mbar_expect_tx(full, 16384);
         tma_load_2d(sSt + s * 16384, &mp->qkv64, full, D + h * DH, nrow0 + j * KTILE);
         tma_load_2d(sSt + s * 16384 + 8192, &mp->qkv64, full, 2 * D + h * DH, nrow0 + j * KTILE);
       }
       if (!aborted(st)) take_early_ticket(et);                               // the last copy of the task is on its way
-      if (aborted(st)) drain_ring<NST>(base, ap.ring, j);
+      if (aborted(st)) drain_ring<NST>(base, a0.ring, j);
     }
   } else if (warp == 1) {
     if (lane == 0) {                                                           // ---- issuer of the scores: runs one step ahead of the softmax threads
-      bool ok = wait_or_abort(bar(base, B_QFULL), ap.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
+      bool ok = wait_or_abort(bar(base, B_QFULL), a0.tasks & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 1000);
       for (int j = 0; j < n && ok; j++) {
-        const uint32_t c = ap.a + j; const int s = j % NST;
-        ok = wait_or_abort(bar(base, B_STFULL + s), ring_parity<NST>(ap.ring, j), st, ST_MBAR_FULL_TIMEOUT, phase_id, task, j);
+        const uint32_t c = a0.a + j; const int s = j % NST;
+        ok = wait_or_abort(bar(base, B_STFULL + s), ring_parity<NST>(a0.ring, j), st, ST_MBAR_FULL_TIMEOUT, phase_id, task, j);
         if (ok && j >= 1) ok = wait_or_abort(bar(base, B_AFREE + ((c - 1) & 1)), ((c - 1) >> 1) & 1, st, ST_MBAR_ACC_TIMEOUT, phase_id, task, j);
         if (!ok) break;
         tc_fence_after();
@@ -509,7 +512,7 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
     if (lane == 0) {                                                           // ---- issuer of the products: follows the softmax threads
       bool ok = true;
       for (int j = 0; j < n && ok; j++) {
-        const uint32_t c = ap.a + j; const int s = j % NST;
+        const uint32_t c = a0.a + j; const int s = j % NST;
         ok = wait_or_abort(bar(base, B_WFULL + (c & 1)), (c >> 1) & 1, st, ST_MBAR_FULL_TIMEOUT, phase_id, task, 2000 + j);
         if (!ok) break;
         tc_fence_after();
@@ -524,7 +527,7 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
     const float lse2 = lse[((size_t)b * H + h) * T + qg] * LOG2E, dr = Dr[((size_t)b * H + h) * T + qg];
     bool ok = true;
     for (int j = 0; j < n && ok; j++) {
-      const uint32_t c = ap.a + j;
+      const uint32_t c = a0.a + j;
       const int k0 = j * KTILE;
       ok = mbar_wait(bar(base, B_AFULL + (c & 1)), (c >> 1) & 1, st);
       ok = __all_sync(0xffffffffu, ok);
@@ -553,7 +556,7 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
         }
       }
       if (j >= 1) {                                                            // the previous step's product read the tile about to be rewritten
-        ok = mbar_wait(bar(base, B_STEMPTY + (j - 1) % NST), ring_parity<NST>(ap.ring, j - 1), st);
+        ok = mbar_wait(bar(base, B_STEMPTY + (j - 1) % NST), ring_parity<NST>(a0.ring, j - 1), st);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -562,7 +565,7 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
       fence_async_smem();
       warp_arrive(bar(base, B_WFULL + (c & 1)));
     }
-    if (ok) { ok = mbar_wait(bar(base, B_DONE), ap.done & 1, st); ok = __all_sync(0xffffffffu, ok); }
+    if (ok) { ok = mbar_wait(bar(base, B_DONE), a0.done & 1, st); ok = __all_sync(0xffffffffu, ok); }
     if (ok) {
       tc_fence_after();
       bf16* dst = dqkv + (size_t)(nrow0 + qg) * ld + h * DH;
@@ -580,10 +583,10 @@ __device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const
       }
     }
   }
-  ap.tasks += 1; ap.ring = ring_after<NST>(ap.ring, n); ap.a += (uint32_t)n; ap.done += 1;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (tid == 0) { ap.tasks = a0.tasks + 1; ap.ring = ring_after<NST>(a0.ring, n); ap.a = a0.a + (uint32_t)n; ap.done = a0.done + 1; }
 }
 
 }  // namespace attn_tc

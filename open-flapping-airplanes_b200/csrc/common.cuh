@@ -182,9 +182,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const D
 
 // The next ticket of the block's job, taken by thread 0 from inside a task once its own part of the task is over (the copy
 // producer after its last copy): the fetch-add's round trip then runs beside the rest of the task instead of after it.
-// slot: a word of the control area, 0 = nothing taken, else ticket + 1. counter == nullptr: not offered (serving job).
-struct EarlyTicket { unsigned* counter; volatile int* slot; };
-__device__ __forceinline__ void take_early_ticket(const EarlyTicket& e) { if (e.counter) *e.slot = (int)(atomicAdd(e.counter, 1u) + 1u); }
+// Lives in the control area. taken: 0 = nothing taken, else ticket + 1. counter == nullptr: not offered.
+struct EarlyTicket { unsigned* counter; unsigned taken, pad; };
+__device__ __forceinline__ void take_early_ticket(EarlyTicket& e) { if (e.counter) e.taken = atomicAdd(e.counter, 1u) + 1u; }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 // a descriptor in global memory that the host has written: needed once per block and launch before its first use, else the descriptor

@@ -67,7 +67,7 @@ __device__ __forceinline__ void block_argmax(float& v, int& idx, float* sv, int*
   __syncthreads();
 }
 // counter-based Gumbel(0,1) noise keyed by (seed, step, vocabulary index)
-__device__ __forceinline__ float gumbel(u64 seed, uint32_t step, uint32_t v) {
+static __device__ __noinline__ float gumbel(u64 seed, uint32_t step, uint32_t v) {
   const u64 r = splitmix64(splitmix64(seed ^ ((u64)step << 32)) + v);
   const float u = ((float)(uint32_t)(r >> 40) + 0.5f) * (1.0f / 16777216.0f);
   return -logf(-logf(u));
@@ -175,6 +175,16 @@ __device__ __forceinline__ bool prefetch(const DecodeParams& P, const ModelDims&
   return true;
 }
 
+// the block's fill has landed; out of line what comes after two probes
+static __device__ __noinline__ bool wait_fill_slow(uint32_t bar, uint32_t parity, DevStatus* status, int layer, int t) {
+  const bool ok = mbar_wait_slow(bar, parity, status);
+  if (!ok && !aborted(status)) raise_abort(status, ST_MBAR_FULL_TIMEOUT, -2, t, layer);
+  return ok;
+}
+__device__ __forceinline__ bool wait_fill(uint32_t bar, uint32_t parity, DevStatus* status, int layer, int t) {
+  return mbar_try(bar, parity) || wait_fill_slow(bar, parity, status, layer, t);
+}
+
 // xs[k] = round_T(LN(x)[k] * gamma[k]); x = fixed-point residual `src`, gamma in shared memory once the task's fill has landed. One block
 // reduction of shifted sums. Ends with a block barrier; false (for all threads) if the fill never came.
 template <class T, int D>
@@ -204,8 +214,7 @@ __device__ __forceinline__ bool prologue_ln(const unsigned long long* src, const
   }
   for (int o = 16; o; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
   if ((tid & 31) == 0) { scratch[tid >> 5] = s1; scratch[8 + (tid >> 5)] = s2; }
-  const bool ok = mbar_wait(bar, parity, status);
-  if (!ok && !aborted(status)) raise_abort(status, ST_MBAR_FULL_TIMEOUT, -2, t, layer);
+  const bool ok = wait_fill(bar, parity, status, layer, t);
   __syncthreads();
   float t1 = 0.f, t2 = 0.f;
 #pragma unroll
@@ -261,7 +270,7 @@ __device__ __forceinline__ float gemv_smem(const T* W, const float* xs, float* r
   float a[VN];
 #pragma unroll
   for (int i = 0; i < VN; i++) a[i] = 0.f;
-#pragma unroll 6
+#pragma unroll 4
   for (int k = rg; k < D; k += RG) {
     float f[VN]; cvt16<T>(*reinterpret_cast<const uint4*>(W + (size_t)k * NC + l * VN), f);
     const float x = xs[k];
@@ -291,7 +300,7 @@ __device__ __forceinline__ void gemv_shares(const T* W, const float* x, float* p
     float a[VN];
 #pragma unroll
     for (int i = 0; i < VN; i++) a[i] = 0.f;
-#pragma unroll
+#pragma unroll 4
     for (int q = 0; q < KPT; q++) {
       const int k = kg * KPT + q;
       float f[VN]; cvt16<T>(*reinterpret_cast<const uint4*>(W + (size_t)k * NC + c), f);
@@ -309,8 +318,7 @@ template <class T, int NC> __host__ __device__ constexpr int gemv_nshares() { re
 // Every task: dependent prologue first, then wait (bounded) for its fill, then multiply out of shared memory.
 #define OFA_DEC_WAIT_FILL()                                                                                        \
   {                                                                                                                 \
-    const bool ok_ = mbar_wait(bar, parity, status);                                                                \
-    if (!ok_ && !aborted(status)) raise_abort(status, ST_MBAR_FULL_TIMEOUT, -2, t, layer);                          \
+    const bool ok_ = wait_fill(bar, parity, status, layer, t);                                                      \
     if (__syncthreads_or(!ok_)) return;      /* uniform decision: nobody is left behind at a later barrier */       \
   }
 
@@ -324,11 +332,11 @@ template <class SM> __device__ __forceinline__ void keep_position(const SM& S, i
 }
 
 // QKV: task t = columns [64t, 64t+64) of [q|k|v]; ntasks = 3D/64.
-template <class T, int D, int DH>
+template <class T, int D, int DH, bool PROF>
 __device__ __forceinline__ void task_qkv(const DecodeParams& P, const ModelDims& md, int layer, int t, int step, unsigned char* smem, uint32_t bar, uint32_t parity, DevStatus* status) {
   Smem<T, D, DH> S(smem, md.T);
   const DecodeState& st = P.st;
-  const bool tr = layer == 0 && t == 0;
+  const bool tr = PROF && layer == 0 && t == 0;
   trace(P.trace, tr, 0);
   const int key = position_word(S, st, step);
   if (threadIdx.x == 0) S.meta[2] = 0;                 // xs no longer holds a final-LayerNorm row
@@ -356,7 +364,7 @@ __device__ __forceinline__ void task_qkv(const DecodeParams& P, const ModelDims&
 // LPK lanes share a key; a group takes every KPR-th key, keeps a maximum of its own and weighs its keys against it, so the block meets
 // once, when the eight warps' sums are brought to the largest maximum. With a maximum and a sum over the whole block first the task
 // took 4.2 us on average over a 256-token answer (six block barriers, three round trips to L2 one after the other), now 3.2.
-template <class T, int D, int DH>
+template <class T, int D, int DH, bool PROF>
 __device__ __forceinline__ void task_attwo(const DecodeParams& P, const ModelDims& md, int layer, int t, int step, unsigned char* smem, uint32_t bar, uint32_t parity, DevStatus* status) {
   using G = Geo<T, D, DH>;
   constexpr int VN = G::VN, LPK = G::LPK, KPR = G::KPR, NW = NTHR / 32;
@@ -366,7 +374,7 @@ __device__ __forceinline__ void task_attwo(const DecodeParams& P, const ModelDim
   const DecodeState& st = P.st;
   const int tid = threadIdx.x, g = tid / LPK, l = tid % LPK, w = tid >> 5;
   const int head = t / G::NCB, cb = t % G::NCB;
-  const bool tr = layer == 0 && t == 0;
+  const bool tr = PROF && layer == 0 && t == 0;
   trace(P.trace, tr, 24);
   const int key = position_word(S, st, step), pos = key & 0xFFFF, n = pos + 1;
   const T* Kc = reinterpret_cast<const T*>(st.kv) + (((size_t)layer * 2 + 0) * md.H + head) * md.T * DH;
@@ -502,12 +510,12 @@ __device__ __forceinline__ void task_attwo(const DecodeParams& P, const ModelDim
 }
 
 // UP+DOWN: task t = hidden units [32t, 32t+32); ntasks = FF/32.
-template <class T, int D, int DH>
+template <class T, int D, int DH, bool PROF>
 __device__ __forceinline__ void task_updn(const DecodeParams& P, const ModelDims& md, int layer, int t, unsigned char* smem, uint32_t bar, uint32_t parity, DevStatus* status) {
   using G = Geo<T, D, DH>;
   Smem<T, D, DH> S(smem, md.T);
   const DecodeState& st = P.st;
-  const bool tr = layer == 0 && t == 0;
+  const bool tr = PROF && layer == 0 && t == 0;
   trace(P.trace, tr, 8);
   if (threadIdx.x == 0) S.meta[2] = 0;
   if (!prologue_ln<T, D>(st.xr, reinterpret_cast<const T*>(S.red), S.xs, S.scratch, nullptr, bar, parity, status, layer, t)) return;
@@ -535,7 +543,7 @@ __device__ __forceinline__ void task_updn(const DecodeParams& P, const ModelDims
 template <class T, int D, int DH>
 __device__ __forceinline__ void task_head(const DecodeParams& P, const ModelDims& md, int t, int step, unsigned char* smem, uint32_t bar, uint32_t parity, DevStatus* status) {
   using G = Geo<T, D, DH>;
-  constexpr int VN = G::VN, VPR = D / VN, NCH = (VPR + 31) / 32, RPW = HR / 8;
+  constexpr int VN = G::VN, VPR = D / VN, RPW = HR / 8;
   Smem<T, D, DH> S(smem, md.T);
   const DecodeState& st = P.st;
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, layer = -1;
@@ -544,29 +552,23 @@ __device__ __forceinline__ void task_head(const DecodeParams& P, const ModelDims
     if (!prologue_ln<T, D>(st.xw, reinterpret_cast<const T*>(S.red), S.xs, S.scratch, nullptr, bar, parity, status, layer, t)) return;
     if (tid == 0) S.meta[2] = step + 1;
   } else OFA_DEC_WAIT_FILL();
-  float x[NCH][VN];
-#pragma unroll
-  for (int i = 0; i < NCH; i++) {
-    const int vi = lane + 32 * i;
-#pragma unroll
-    for (int k = 0; k < VN; k += 4) {
-      const float4 v = vi < VPR ? *reinterpret_cast<const float4*>(S.xs + vi * VN + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      x[i][k] = v.x; x[i][k + 1] = v.y; x[i][k + 2] = v.z; x[i][k + 3] = v.w;
-    }
-  }
   const T* Wh = reinterpret_cast<const T*>(S.w) + (size_t)w * RPW * D;
   float s[RPW];                                        // rows past the vocabulary hold whatever the buffer held: they are not read below
 #pragma unroll
-  for (int rr = 0; rr < RPW; rr++) {
-    s[rr] = 0.f;
+  for (int rr = 0; rr < RPW; rr++) s[rr] = 0.f;
+#pragma unroll 1
+  for (int vi = lane; vi < VPR; vi += 32) {
+    float x[VN];
 #pragma unroll
-    for (int i = 0; i < NCH; i++) {
-      const int vi = lane + 32 * i;
-      if (vi < VPR) {
-        float f[VN]; cvt16<T>(*reinterpret_cast<const uint4*>(Wh + (size_t)rr * D + vi * VN), f);
+    for (int k = 0; k < VN; k += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(S.xs + vi * VN + k);
+      x[k] = v.x; x[k + 1] = v.y; x[k + 2] = v.z; x[k + 3] = v.w;
+    }
 #pragma unroll
-        for (int k = 0; k < VN; k++) s[rr] = fmaf(x[i][k], f[k], s[rr]);
-      }
+    for (int rr = 0; rr < RPW; rr++) {
+      float f[VN]; cvt16<T>(*reinterpret_cast<const uint4*>(Wh + (size_t)rr * D + vi * VN), f);
+#pragma unroll
+      for (int k = 0; k < VN; k++) s[rr] = fmaf(x[k], f[k], s[rr]);
     }
   }
   reduce_scatter<RPW, 1>(s);

@@ -363,8 +363,8 @@ __device__ __forceinline__ void ce_task_bulk(int task, bf16* logits, const int* 
   const int t = threadIdx.x;
   const int nvec = V / 8;
   const uint32_t row_bytes = (uint32_t)V * 2u;
-  const uint32_t use0 = uses;
-  uses += CE_ROWS;                                     // every thread, whatever happens below
+  uint32_t use0 = 0;                                   // only the polling thread looks at it
+  if (t == 0) { use0 = uses; uses = use0 + CE_ROWS; }
   for (int rr = 0; rr < CE_ROWS; rr++) {
     const int r = task * CE_ROWS + rr;
     const uint32_t parity = (use0 + rr) & 1u;
@@ -426,7 +426,7 @@ __device__ __forceinline__ void ce_task_bulk(int task, bf16* logits, const int* 
 //   dlogit = (2^(x * log2(e) - M) / S - onehot) * inv_n.
 // The task's rows move through shared memory as one stream of chunks staged by the copy engine, four chunks (96 KB) in flight
 // across row boundaries; nothing waits for a whole row. `bar_lo`, `bar_hi` = two pairs of block-private mbarriers (count 1), `chunks` = running
-// count of chunks this block has staged (advanced identically by every thread). V must be a multiple of 8.
+// count of chunks this block has staged (in shared memory, advanced by thread 0). V must be a multiple of 8.
 constexpr int CE_CHUNK = 12288, CE_STAGES = 4;            // elements per chunk (24 KB of bf16)
 static __device__ __noinline__ void ce_task_stream(int task, bf16* logits, const int* targets, float* loss, const float2* part, int tiles_n,
                                                int N, int V, float inv_n, unsigned char* smem, uint32_t bar_lo, uint32_t bar_hi, uint32_t& chunks,
@@ -438,8 +438,7 @@ static __device__ __noinline__ void ce_task_stream(int task, bf16* logits, const
   const int r0 = task * CE_ROWS, nrows = min(CE_ROWS, N - r0);
   const int cpr = (V + CE_CHUNK - 1) / CE_CHUNK;                                   // chunks per row
   const int total = nrows > 0 ? nrows * cpr : 0;
-  const uint32_t u0 = chunks;
-  chunks += (uint32_t)total;                                                       // every thread, whatever happens below
+  const uint32_t u0 = chunks;                                                      // in shared memory: thread 0 advances it behind the last chunk's barrier
   const uint32_t sbase = smem_u32(smem);
   auto issue = [&](int k) {                                                        // thread 0: chunk k of this task into stage (u0 + k) % 4
     const uint32_t u = u0 + (uint32_t)k, sg = u % CE_STAGES, b = sbar(sg);
@@ -499,10 +498,12 @@ static __device__ __noinline__ void ce_task_stream(int task, bf16* logits, const
           for (int spin = 0; spin < 100000 && !mbar_try(sbar(uu % CE_STAGES), (uu / CE_STAGES) & 1u); spin++) {}
         }
       __syncthreads();
+      if (t == 0) chunks = u0 + (uint32_t)total;
       return;
     }
     if (t == 0 && k + CE_STAGES < total) { fence_proxy_async(); issue(k + CE_STAGES); }
   }
+  if (t == 0) chunks = u0 + (uint32_t)total;
 }
 
 // mean_loss[0] = (sum_r loss[r]) / N, fixed order. One task.
@@ -728,7 +729,7 @@ __device__ __forceinline__ void adamw_task(int task, float* W, const GT* G, floa
 // (cp.async.bulk, completion counted on an mbarrier) of W, M, V and G for tiles of 2,048 elements, three tiles (96 KB) ahead
 // of the arithmetic; the threads read their operands from shared memory and write results straight to global memory.
 // `bar0` = three block-private mbarriers (count 1), `tiles` = running count of tiles this block has staged since it started
-// (advanced identically by every thread). The ragged end of a range (fewer than 2,048 elements) goes through the direct loop.
+// (in shared memory, advanced by thread 0). The ragged end of a range (fewer than 2,048 elements) goes through the direct loop.
 constexpr int ADAM_TILE = 2048, ADAM_STAGES = 3, ADAM_STAGE_BYTES = 32768;
 template <class T, class GT>
 __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, float* M, float* Vv, T* Wact, size_t n, AdamHP hp,
@@ -741,8 +742,7 @@ __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, fl
   const int tid = threadIdx.x;
   const bool aligned = ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(M) | reinterpret_cast<uintptr_t>(Vv) | reinterpret_cast<uintptr_t>(G)) & 15) == 0;
   const int nfull = aligned ? (int)((ce - cs) / ADAM_TILE) : 0;
-  const uint32_t u0 = tiles;
-  tiles += (uint32_t)nfull;                             // every thread, whatever happens below
+  const uint32_t u0 = tiles;                           // in shared memory: thread 0 advances it behind the last tile's barrier
   const uint32_t sbase = smem_u32(smem);
   auto issue = [&](int k) {                            // thread 0: tile k of this task into stage (u0 + k) % 3
     const uint32_t u = u0 + (uint32_t)k, s = u % ADAM_STAGES, b = bar0 + 8u * s, dst = sbase + s * ADAM_STAGE_BYTES;
@@ -778,10 +778,12 @@ __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, fl
           for (int spin = 0; spin < 100000 && !mbar_try(bar0 + 8u * (uu % ADAM_STAGES), (uu / ADAM_STAGES) & 1u); spin++) {}
         }
       __syncthreads();
+      if (tid == 0) tiles = u0 + (uint32_t)nfull;
       return;
     }
     if (tid == 0 && k + ADAM_STAGES < nfull) { fence_proxy_async(); issue(k + ADAM_STAGES); }
   }
+  if (tid == 0 && nfull > 0) tiles = u0 + (uint32_t)nfull;
   adamw_span_direct<T, GT>(A, cs + (size_t)nfull * ADAM_TILE, ce, W, G, M, Vv, Wact);
 }
 

@@ -54,16 +54,16 @@ template <int BN> struct Cfg {
 // control area (1 KB at smem + BAR_OFFSET = the last 1,024 bytes of dynamic shared memory):
 //   [  0, 80) BN128: full[3] empty[3] accf[2] acce[2]     [ 80, 84) TMEM base slot     [ 96,104) serving fill barrier   [104,112) training bulk-copy barrier
 //   [112,128) and [160,176) streamed cross-entropy stage barriers [4]
-//   [128,160) scheduler hand-off words                      [176,224) BN256: full[2] empty[2] accf[1] acce[1]      [224,248) AdamW stage barriers [3]
-//   [256,512) and [512,768) two slots for phase descriptors: the one being worked on and the next phase's, fetched ahead
-//   [768,832) scheduling record (ticket range + dependencies) of the phase the scheduler thread looks at next
+//   [176,224) BN256: full[2] empty[2] accf[1] acce[1]      [224,248) AdamW stage barriers [3]      [248,256), [1008,1024) profiling stamps
+//   [256,448) and [448,640) two slots for phase descriptors: the one being worked on and the next phase's, fetched ahead
+//   [640,832) the block's scheduling state and pipeline counters (BlockState)      [832,1008) attention barriers
 template <int BN> __device__ __forceinline__ uint32_t bar_full(uint32_t base, int s) { return base + BAR_OFFSET + Cfg<BN>::BAR0 + 8u * s; }
 template <int BN> __device__ __forceinline__ uint32_t bar_empty(uint32_t base, int s) { return base + BAR_OFFSET + Cfg<BN>::BAR0 + 8u * (Cfg<BN>::STAGES + s); }
 template <int BN> __device__ __forceinline__ uint32_t bar_accf(uint32_t base, int b) { return base + BAR_OFFSET + Cfg<BN>::BAR0 + 8u * (2 * Cfg<BN>::STAGES + b); }
 template <int BN> __device__ __forceinline__ uint32_t bar_acce(uint32_t base, int b) { return base + BAR_OFFSET + Cfg<BN>::BAR0 + 8u * (2 * Cfg<BN>::STAGES + Cfg<BN>::NBUF + b); }
 constexpr int TMEM_SLOT_OFFSET = BAR_OFFSET + 80;
 
-// Per-thread running counters, one set per tile width; every thread advances them identically at the end of a task.
+// Running counters, one set per tile width; in shared memory, read at the start of a task and advanced by thread 0 behind its closing barrier.
 struct GemmPipe {
   uint32_t stage_count[2];   // pipeline stages produced/consumed since block start
   uint32_t tile_count[2];    // accumulator tiles since block start
@@ -77,7 +77,6 @@ template <int BN> __device__ __forceinline__ void init_bars(uint32_t base) {
 // Once per block, before its first GEMM task. All 256 threads. Returns false (and aborts) if shared memory is misaligned.
 __device__ __forceinline__ bool block_init(GemmPipe& gp, unsigned char* smem, DevStatus* st) {
   const uint32_t base = smem_u32(smem);
-  gp.stage_count[0] = gp.stage_count[1] = 0; gp.tile_count[0] = gp.tile_count[1] = 0; gp.tmem_base = 0;
   const bool ok = (base & 1023u) == 0;
   if (!ok) { if (threadIdx.x == 0) raise_abort(st, ST_SMEM_MISALIGNED, -1, -1, (int)base); }
   if (threadIdx.x == 0) { init_bars<128>(base); init_bars<256>(base); mbar_fence_init(); }
@@ -85,7 +84,8 @@ __device__ __forceinline__ bool block_init(GemmPipe& gp, unsigned char* smem, De
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  gp.tmem_base = *reinterpret_cast<volatile uint32_t*>(smem + TMEM_SLOT_OFFSET);
+  if (threadIdx.x == 0) { gp.stage_count[0] = gp.stage_count[1] = 0; gp.tile_count[0] = gp.tile_count[1] = 0; gp.tmem_base = *reinterpret_cast<volatile uint32_t*>(smem + TMEM_SLOT_OFFSET); }
+  __syncthreads();
   return ok;
 }
 // Once per block before it exits. All 256 threads. TMA copies still in flight when a task gives up are waited for
@@ -142,7 +142,7 @@ __device__ __forceinline__ void epi_store8(const GemmArgs& g, size_t row, int co
 // task index -> (tile_m, first tile_n): consecutive tasks walk down M first so that neighbouring blocks share the B strip.
 template <int LAYOUT, int EPI, int BN>
 __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int task, unsigned char* smem, GemmPipe& gp,
-                                             DevStatus* st, int phase_id, const EarlyTicket& et, int nfast) {
+                                             DevStatus* st, int phase_id, EarlyTicket& et, int nfast) {
   using CF = Cfg<BN>;
   constexpr bool A_MN = (LAYOUT == GL_TN), B_MN = (LAYOUT != GL_NT);
   constexpr bool HAS_AUX_IN = (EPI == GE_RES || EPI == GE_DGELU || EPI == GE_DR);
@@ -151,6 +151,7 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
   constexpr int STAGES = CF::STAGES, W = CF::W;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = smem_u32(smem);
+  const uint32_t stage0 = gp.stage_count[W], tile0 = gp.tile_count[W], tmem = gp.tmem_base;
   const int KT = g.K / BK;
   const int tiles_n = g.N / BN;
   // nfast: consecutive tasks walk along N first, so the tasks that stream the same rows of a large A run side by side and the
@@ -164,7 +165,7 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
   if (warp == 0) {
     if (lane == 0) {                                                           // ---- TMA producer
       fence_proxy_async();     // operands were written with ordinary stores by earlier phases (possibly other SMs)
-      uint32_t sc = gp.stage_count[W];
+      uint32_t sc = stage0;
       bool ok = true;
       for (int t = 0; t < nt && ok; t++) {
         const int n0 = (tn0 + t) * BN;
@@ -188,7 +189,7 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
       }
       if (ok) take_early_ticket(et);     // every copy of the task is on its way: this thread has nothing left to do but the closing barrier
       if (aborted(st)) {       // giving up: wait (bounded) until the copies this task issued into our shared memory have landed
-        const uint32_t issued = sc - gp.stage_count[W];
+        const uint32_t issued = sc - stage0;
         for (uint32_t i = 0; i < issued && i < (uint32_t)STAGES; i++) {
           const uint32_t c = sc - 1 - i; const int s = c % STAGES; const uint32_t use = c / STAGES;
           for (int spin = 0; spin < 100000; spin++) if (mbar_try(bar_full<BN>(base, s), use & 1)) break;
@@ -197,13 +198,13 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
     }
   } else if (warp == 1) {
     if (lane == 0) {                                                           // ---- MMA issuer
-      uint32_t sc = gp.stage_count[W], tc = gp.tile_count[W];
+      uint32_t sc = stage0, tc = tile0;
       bool ok = true;
       for (int t = 0; t < nt && ok; t++, tc++) {
         const int b = tc % CF::NBUF; const uint32_t use = tc / CF::NBUF;
         if (!mbar_wait(bar_acce<BN>(base, b), (use & 1) ^ 1, st)) { if (!aborted(st)) raise_abort(st, ST_MBAR_ACC_TIMEOUT, phase_id, task, 100 + t); ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = gp.tmem_base + (uint32_t)(b * BN);
+        const uint32_t d_tmem = tmem + (uint32_t)(b * BN);
         for (int kt = 0; kt < KT; kt++, sc++) {
           const int s = sc % STAGES; const uint32_t suse = sc / STAGES;
           if (!mbar_wait(bar_full<BN>(base, s), suse & 1, st)) { if (!aborted(st)) raise_abort(st, ST_MBAR_FULL_TIMEOUT, phase_id, task, kt); ok = false; break; }
@@ -223,7 +224,7 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
   } else if (warp >= 4) {                                                      // ---- epilogue warps
     const int e = warp - 4;                      // TMEM lane quadrant == warp % 4
     float* stg = reinterpret_cast<float*>(smem + PIPE_BYTES + e * 4096);
-    uint32_t tc = gp.tile_count[W];
+    uint32_t tc = tile0;
     bool ok = true;
     const int cg = lane & 3;
     // An epilogue's code runs once per tile and has left the instruction caches by the block's next task of the kind (a step runs through
@@ -235,7 +236,7 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
       const int n0 = (tn0 + t) * BN;
 #pragma unroll 1
       for (int half = 0; half < BN / 128; half++) {          // 128 columns at a time
-        const uint32_t tacc = gp.tmem_base + ((uint32_t)(e * 32) << 16) + (uint32_t)(b * BN + half * 128);
+        const uint32_t tacc = tmem + ((uint32_t)(e * 32) << 16) + (uint32_t)(b * BN + half * 128);
         const int nh = n0 + half * 128;
         // Epilogues that read `aux` (residual, pre-activation) fetch this thread's row segments of the first pass BEFORE waiting for the
         // accumulator, so the loads travel while the MMAs run.
@@ -371,18 +372,17 @@ __device__ __forceinline__ void gemm_tc_task(const GemmArgs& g, int tiles_m, int
       }
     }
   }
-  gp.stage_count[W] += (uint32_t)(nt * KT);
-  gp.tile_count[W] += (uint32_t)nt;
   __syncthreads();
+  if (tid == 0) { gp.stage_count[W] = stage0 + (uint32_t)(nt * KT); gp.tile_count[W] = tile0 + (uint32_t)nt; }
 }
 
 template <int LAYOUT, int EPI>
-__device__ __forceinline__ void dispatch_bn(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, const EarlyTicket& et) {
+__device__ __forceinline__ void dispatch_bn(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, EarlyTicket& et) {
   if (d.g.bn == 256) gemm_tc_task<LAYOUT, EPI, 256>(d.g, d.tiles_m, task, smem, gp, st, phase_id, et, d.i0);
   else gemm_tc_task<LAYOUT, EPI, 128>(d.g, d.tiles_m, task, smem, gp, st, phase_id, et, d.i0);
 }
 // run-time dispatch over the (layout, epilogue) pairs the training graph uses
-__device__ __noinline__ void run(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, const EarlyTicket& et) {
+__device__ __noinline__ void run(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, EarlyTicket& et) {
   switch (d.layout * 8 + d.epi) {
     case GL_NN * 8 + GE_STORE: dispatch_bn<GL_NN, GE_STORE>(d, task, smem, gp, st, phase_id, et); break;
     case GL_NN * 8 + GE_RES:   dispatch_bn<GL_NN, GE_RES>(d, task, smem, gp, st, phase_id, et); break;

@@ -44,7 +44,7 @@ struct HostPhase { std::string name; PhaseDesc d; std::vector<Dep> deps; std::ve
 // memory of the caller: a context uploads the tables once and only clears the counters before each launch; ofa_run_phases packs
 // them into its workspace.
 struct HostJob {
-  std::vector<PhaseDesc> pd; std::vector<SchedRec> rec; std::vector<int> prefix, nt, doff, dcnt; std::vector<Dep> deps;
+  std::vector<PhaseDesc> pd; std::vector<int> perm, prefix, nt, doff, dcnt; std::vector<Dep> deps;
   int nph = 0, last_phase = 0, rb_total = 0;
 };
 
@@ -231,7 +231,7 @@ bool make_job(const std::vector<HostPhase>& ph, int last_phase, HostJob& hj, std
     }
     if (nt[i] <= 0) { err = "phase without tasks: " + ph[i].name; return false; }
   }
-  if (nph >= 65536) { err = "too many phases"; return false; }
+  if (nph >= 65536 || (long long)RB_STRIDE * nph * std::max(nrb, 0) >= (1 << 28)) { err = "too many phases"; return false; }
   // which phases count their completions per row block: those that say how their tasks map to row blocks, have a whole number of
   // tasks per row block, and are waited for at that grain by somebody
   std::vector<int> rb_off(nph, -1); int rb_total = 0;
@@ -241,18 +241,18 @@ bool make_job(const std::vector<HostPhase>& ph, int last_phase, HostJob& hj, std
         const int p = ph[i].deps[k].phase;
         if (k < ph[i].rb_grain.size() && ph[i].rb_grain[k] && ph[i].rb_map && ph[p].rb_map && nt[p] % nrb == 0 && rb_off[p] < 0) { rb_off[p] = rb_total; rb_total += nrb; }
       }
-  std::vector<SchedRec>& rec = hj.rec; rec.resize(nph);
+  hj.perm.resize(nph);
   for (int i = 0; i < nph; i++) {
-    SchedRec& r = rec[i]; memset(&r, 0, sizeof(r));
-    r.lo = prefix[i]; r.hi = prefix[i + 1];
+    SchedRec& r = pd[i].rec; memset(&r, 0, sizeof(r));
     const int n = (int)ph[i].deps.size();
     r.ndeps = n <= 4 ? n : -1;
-    r.perm_mul = shuffle_multiplier(g_task_shuffle_seed, i, nt[i]);
+    hj.perm[i] = shuffle_multiplier(g_task_shuffle_seed, i, nt[i]);
     r.rb_off = rb_off[i]; r.rb_map = ph[i].rb_map;
     for (int k = 0; k < n && n <= 4; k++) {
       const Dep& e = ph[i].deps[k];
       const bool rb = k < (int)ph[i].rb_grain.size() && ph[i].rb_grain[k] && ph[i].rb_map && rb_off[e.phase] >= 0;
-      r.dep[2 * k] = e.phase | (e.delta == -1 ? DEP_PREV : 0) | (rb ? DEP_RB : 0);
+      r.dep[2 * k] = (rb ? DONE_STRIDE * nph + RB_STRIDE * rb_off[e.phase] : DONE_STRIDE * e.phase) | (e.delta == -1 ? DEP_PREV : 0) | (rb ? DEP_RB : 0);
+      r.any_rb |= rb ? 1 : 0;
       r.dep[2 * k + 1] = rb ? nt[e.phase] / nrb : nt[e.phase];
     }
   }
@@ -266,7 +266,7 @@ bool tickets_fit(const HostJob& hj, long nsteps, std::string& err) {
 }
 constexpr size_t up64(size_t n) { return (n + 63) / 64 * 64; }
 size_t job_table_bytes(const HostJob& h) {
-  return up64(sizeof(PhaseDesc) * h.nph) + up64(sizeof(SchedRec) * h.nph) + up64(4 * ((size_t)h.nph + 1)) + 3 * up64(4 * (size_t)h.nph) + up64(sizeof(Dep) * h.deps.size());
+  return up64(sizeof(PhaseDesc) * h.nph) + up64(4 * ((size_t)h.nph + 1)) + 4 * up64(4 * (size_t)h.nph) + up64(sizeof(Dep) * h.deps.size());
 }
 size_t job_counter_bytes(const HostJob& h) { return 128 + 4 * (size_t)(DONE_STRIDE * h.nph + RB_STRIDE * std::max(1, h.rb_total)); }
 // writes the tables to `host` (an image of `dev`) and fills the job's pointers; `cnt` = its counters, to be zero before a launch
@@ -275,7 +275,7 @@ Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* 
   size_t o = 0;
   auto put = [&](const void* src, size_t bytes) { memcpy(host + o, src, bytes); const void* d = dev + o; o += up64(bytes); return d; };
   j.ph = reinterpret_cast<const PhaseDesc*>(put(h.pd.data(), sizeof(PhaseDesc) * h.nph));
-  j.rec = reinterpret_cast<const SchedRec*>(put(h.rec.data(), sizeof(SchedRec) * h.nph));
+  j.perm = reinterpret_cast<const int*>(put(h.perm.data(), 4 * (size_t)h.nph));
   j.prefix = reinterpret_cast<const int*>(put(h.prefix.data(), 4 * ((size_t)h.nph + 1)));
   j.ntasks = reinterpret_cast<const int*>(put(h.nt.data(), 4 * (size_t)h.nph));
   j.dep_off = reinterpret_cast<const int*>(put(h.doff.data(), 4 * (size_t)h.nph));
@@ -286,25 +286,31 @@ Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* 
   return j;
 }
 
-// copies a job's scheduling records into the kernel parameter when they fit
+// copies the first tickets of a job's phases into the kernel parameter when they fit
 void fill_param_records(Ctx& C, const HostJob* train, const HostJob* dec) {
-  C.train_rec_n = 0; C.dec_rec_n = 0;
+  C.train_pre_n = 0; C.dec_pre_n = 0;
   C.sched_flags = getenv("OFA_B200_LATE_TICKETS") ? 4 : 0;     // A/B switch for measurements: tickets only at the end of a task
-  if (getenv("OFA_B200_GLOBAL_RECS")) return;      // A/B switch for measurements: keep using the records in global memory
-  if (train && train->nph > 0 && train->nph <= PARAM_TRAIN_PH) { memcpy(C.train_rec, train->rec.data(), sizeof(SchedRec) * train->nph); C.train_rec_n = train->nph; }
-  if (dec && dec->nph > 0 && dec->nph <= PARAM_DEC_PH) { memcpy(C.dec_rec, dec->rec.data(), sizeof(SchedRec) * dec->nph); C.dec_rec_n = dec->nph; }
+  if (g_task_shuffle_seed) C.sched_flags |= 1;
+  if (getenv("OFA_B200_GLOBAL_RECS")) return;      // A/B switch for measurements: keep using the tables in global memory
+  if (train && train->nph > 0 && train->nph <= PARAM_TRAIN_PH) { memcpy(C.train_pre, train->prefix.data(), 4 * ((size_t)train->nph + 1)); C.train_pre_n = train->nph; }
+  if (dec && dec->nph > 0 && dec->nph <= PARAM_DEC_PH) { memcpy(C.dec_pre, dec->prefix.data(), 4 * ((size_t)dec->nph + 1)); C.dec_pre_n = dec->nph; }
 }
 
 // The limit is always the device's (227 KB), whatever this launch needs: two threads cannot lower it under each other, and nothing has to
 // be remembered between launches (a device reset would make it untrue). The two calls take 0.2 us together.
 template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nblocks, int smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
-  if (e != cudaSuccess) return e;
-  // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
-  // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
-  cudaFuncSetAttribute(ofa_kernel<T, D, DH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  ofa_kernel<T, D, DH><<<nblocks, NTHR, smem, s>>>(C);
-  return cudaGetLastError();
+  auto launch = [&](auto kernel) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+    if (e != cudaSuccess) return e;
+    // ask for the largest shared-memory carve-out on every SM: with a smaller split an SM holds one 113 KB block instead of two,
+    // and a persistent block never leaves to let the split be changed (measured: 24 SMs ran with a single block)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    kernel<<<nblocks, NTHR, smem, s>>>(C);
+    return cudaGetLastError();
+  };
+  if (C.sched_flags & 2) return launch(ofa_kernel<T, D, DH, true, true, true>);
+  if (C.use_train && C.use_decode) return launch(ofa_kernel<T, D, DH, true, true, false>);
+  return C.use_train ? launch(ofa_kernel<T, D, DH, true, false, false>) : launch(ofa_kernel<T, D, DH, false, true, false>);
 }
 
 // Tasks whose shared-memory need grows with the batch or the context must fit the block's task area: on the bf16 path that is
@@ -1604,7 +1610,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   std::string err;
   // upper bound of the call's tables, to size the workspace before the phases are prepared: descriptors, records, one dependency
   // per phase (two for the first), at most four TMA descriptors per phase, counters, and what the kernel reports per repeat
-  const size_t map_cap = (size_t)nph * sizeof(attn_tc::Maps), tab_cap = (size_t)nph * (sizeof(PhaseDesc) + sizeof(SchedRec) + 24 + sizeof(Dep)) + 1024;
+  const size_t map_cap = (size_t)nph * sizeof(attn_tc::Maps), tab_cap = (size_t)nph * (sizeof(PhaseDesc) + 32 + sizeof(Dep)) + 1024;
   const size_t rep_bytes = up64(sizeof(unsigned long long) * (size_t)repeats) + up64(sizeof(float) * (size_t)repeats);
   const size_t cnt_cap = 128 + 4 * (size_t)(DONE_STRIDE * nph + RB_STRIDE);
   WorkspaceLease ws(dev, map_cap + tab_cap + 192 + cnt_cap, rep_bytes);
@@ -1615,8 +1621,8 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
     const ofa_phase& s = phases[i];
     HostPhase& hp = P[i]; hp.name = "phase" + std::to_string(i);
     PhaseDesc& d = hp.d; memset(&d, 0, sizeof d);
-    d.kind = s.kind; d.layout = s.layout; d.epi = s.epi; d.i0 = s.i0; d.i1 = s.i1; d.i2 = s.i2; d.n = s.n;
-    for (int k = 0; k < 10; k++) d.p[k] = s.p[k];
+    d.kind = s.kind; d.layout = s.layout; d.epi = s.epi; d.i0 = s.i0; d.i1 = s.i1; d.i2 = s.i2;
+    if (s.kind != TK_GEMM) { d.n = s.n; for (int k = 0; k < 10; k++) d.p[k] = s.p[k]; }
     const int BH = m.B * m.H, rows16 = (m.N + 15) / 16;
     switch (s.kind) {
       case TK_GEMM:
@@ -1665,7 +1671,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   if (total > ws.w.bytes) return fail(nullptr, OFA_CUDA_ERROR, "workspace too small");
   memset(ws.w.host + o_st, 0, total - o_st);
   static thread_local Ctx C;      // 31 KB: not on the stack
-  memset(&C, 0, offsetof(Ctx, train_rec));
+  memset(&C, 0, offsetof(Ctx, train_pre));
   C.train = place_job(hj, repeats, ws.w.host + o_tab, ws.w.dev + o_tab, ws.w.dev + o_cnt); C.md = m;
   fill_param_records(C, &hj, nullptr);
   if (adam) { C.hp.lr_max = adam[0]; C.hp.lr_min = adam[0]; C.hp.beta1 = adam[1]; C.hp.beta2 = adam[2]; C.hp.eps = adam[3]; C.hp.wd = adam[4]; C.hp.grad_scale = adam[5]; C.hp.constant_lr = 1; }

@@ -66,19 +66,9 @@ struct GemmArgs {
   float* dr; int dr_T, dr_H;  // GE_DR: output [B, H, T] and its dimensions (row = b * T + t, head = column / 64). GE_LSE: dr = output [M, N / 128] float2
 };
 
-struct alignas(16) PhaseDesc {
-  int kind, ntasks, layout, epi;
-  int tiles_m, i0, i1, i2;
-  GemmArgs g;
-  void* p[10];
-  size_t n;
-  float f0, f1;
-};
-
 struct Dep { int phase; int delta; };   // need done[phase] >= ntasks[phase] * (step + 1 + delta)
 
-// Everything the scheduler thread needs to place a ticket in a phase and to check that phase's dependencies, in one 64-byte
-// line: one memory round trip per phase change instead of a chain of dependent table look-ups.
+// What the scheduler needs of a phase besides its tickets. It travels with the phase's descriptor.
 //
 // Dependencies come in two grains. A phase-level dependency (the reference's only kind, ofa.cu:245-255) waits until EVERY task of
 // the producer phase has finished. A row-block dependency waits only for the producer tasks that write the 128-token row blocks
@@ -93,23 +83,29 @@ enum RbKind : int {
   RB_ATT_BWD,    // attention backward: dK/dV task (key tile) reads row blocks tile..last of its sequence; dQ task its own row block
 };
 struct alignas(16) SchedRec {
-  int lo, hi;               // tickets [lo, hi) of a step belong to this phase
   int ndeps;                // 0..4 dependencies held in dep[]; -1: more than four, use Job::deps (phase-level only)
-  int perm_mul;             // 0 (production), or a multiplier coprime with the task count: ticket i of the phase runs task (i * perm_mul + perm_mul / 2) % ntasks (test hook: results must not depend on the order)
   int rb_off;               // where this phase counts completions per row block in Job::done_rb, -1: it does not
   int rb_map;               // RbKind | a << 8
-  int dep[8];               // per dependency: {phase | (step delta == -1) << 16 | row-block grain << 17,  completions needed per step: tasks of the phase, or tasks per row block}
-  int pad[2];
+  int any_rb;               // one of the dependencies is of row-block grain
+  int dep[8];               // per dependency: {word of Job::done that counts it (row-block grain: of the producer's row block 0) | flags,  completions needed per step: tasks of the phase, or tasks per row block}
 };
-constexpr int DEP_PREV = 1 << 16, DEP_RB = 1 << 17;
+constexpr int DEP_PREV = 1 << 30, DEP_RB = 1 << 29, DEP_WORD = DEP_RB - 1;      // of the step before; of row-block grain
+struct alignas(16) PhaseDesc {
+  int kind, ntasks, layout, epi;
+  int tiles_m, i0, i1, i2;
+  union {                   // products, everything else
+    GemmArgs g;
+    struct { void* p[10]; size_t n; };
+  };
+  SchedRec rec;
+};
+
 // Completion counters sit in lines (phases) and sectors (row blocks) of their own: every block of the GPU polls the counter of the phase
 // it waits for while others add to it, and 32 phases in one line would put all of that on one L2 slice.
 constexpr int DONE_STRIDE = 32, RB_STRIDE = 8;
 constexpr int CTRL_BYTES = 1024;   // control area at the end of every block's dynamic shared memory
-// The scheduling records of both jobs travel with the launch as part of the kernel parameter (constant bank): a block that
-// claims a ticket finds the phase and its dependencies without a single round trip to global memory. Jobs with more phases than
-// fit (the parameter is limited to 32,764 bytes) fall back to the records in global memory, a copy requested at the end of the task before: no slower
-// for a training step of 268 to 570 phases (12 layers, 1,024 tokens, 396 phases: 4,043 us from the parameter, 4,044 from global memory).
+// The first tickets of the phases of both jobs travel with the launch as part of the kernel parameter (constant bank): a block that claims a
+// ticket finds its phase without a round trip to global memory. Jobs with more phases than fit use the table in global memory.
 constexpr int PARAM_TRAIN_PH = 400, PARAM_DEC_PH = 64;
 
 struct Job {
@@ -120,9 +116,9 @@ struct Job {
   const int* dep_off;       // [nph]
   const int* dep_cnt;       // [nph]
   const Dep* deps;
-  const SchedRec* rec;      // [nph]
+  const int* perm;          // [nph] 0 (production), or a multiplier coprime with the task count: ticket i of the phase runs task (i * perm + perm / 2) % ntasks (test hook: results must not depend on the order)
   int* done;                // [nph] monotonically increasing over steps, DONE_STRIDE words apart
-  int* done_rb;             // completions per (phase that publishes them, row block of 128 tokens), monotonically increasing, RB_STRIDE words apart; see SchedRec
+  int* done_rb;             // behind them: completions per (phase that publishes them, row block of 128 tokens), monotonically increasing, RB_STRIDE words apart; see SchedRec
   unsigned* ticket;         // next (step * tasks_per_step + task) to hand out
 };
 
@@ -190,10 +186,10 @@ struct Ctx {
   int* arrived;             // blocks of this launch that have started (idle partitions leave only when all have)
   int smem_bytes;           // dynamic shared memory per block; its last 1,024 bytes are the control area (barriers, hand-off words, descriptor slots)
   int sched_flags;                          // bit 1: keep the per-phase / per-block time tables
-  int train_rec_n, dec_rec_n;               // phases whose records are held below (0: use Job::rec in global memory)
-  SchedRec train_rec[PARAM_TRAIN_PH];
-  SchedRec dec_rec[PARAM_DEC_PH];
   const unsigned char* maps; int nmaps;     // TMA descriptors (128 bytes each) that the launch is the first to use
+  int train_pre_n, dec_pre_n;               // phases whose first tickets are held below (0: use Job::prefix in global memory)
+  int train_pre[PARAM_TRAIN_PH + 1];
+  int dec_pre[PARAM_DEC_PH + 1];
 };
 static_assert(sizeof(Ctx) <= 32764, "kernel parameter too large");
 

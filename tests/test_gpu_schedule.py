@@ -217,3 +217,41 @@ def test_spread_adamw_gives_the_same_bits_in_every_form(ofa, monkeypatch, layers
     assert out[0][0] > out[1][0]
     np.testing.assert_array_equal(out[0][1], out[1][1])
     np.testing.assert_array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("preset", ["gpt_s", "tiny"])
+@pytest.mark.parametrize("job", ["train", "serve", "both"])
+def test_every_form_of_the_kernel_gives_the_same_bits(ofa, preset, job):
+    """A launch that trains, serves or does both runs a kernel of its own; one that keeps time tables runs the form that can do everything."""
+    out = []
+    for profile in (1, 0):
+        cfg = ofa.default_config(preset)
+        cfg.sched_profile = profile
+        if preset == "gpt_s":
+            cfg.vocab = cfg.valid_vocab = 1152
+            cfg.n_layer, cfg.ctx_len, cfg.batch = 2, 256, 1
+        if job != "train":
+            cfg.use_decode, cfg.infer_sms, cfg.n_prompt, cfg.answer_len, cfg.temperature = 1, 24, 3, 16, 0.0
+        if job == "serve":
+            cfg.mode = ofa.capi.MODE_DECODE_ONLY
+        elif job == "both":
+            cfg.reserved_sms, cfg.train_sms = 8, 116
+            cfg.lr_max = cfg.lr_min = 0.0              # the served weights do not move, so that what is served does not hang on timing
+        mk = ofa.Megakernel(cfg)
+        g = np.random.default_rng(5)
+        mk.load_weights(g.standard_normal(mk.num_params, dtype=np.float32) * 0.02)
+        res = {}
+        if job != "serve":
+            mk.set_tokens(g.integers(0, cfg.vocab, size=1 << 13, dtype=np.uint32))
+        mk.run(40)
+        if job != "serve":
+            res["loss"], res["w"] = mk.losses()[-40:].copy(), mk.read_weights()
+        if job != "train":
+            t = np.asarray(mk.decode_tokens())
+            res["tokens"] = t[t >= 0]                  # beside training, how many depends on how long the steps take
+        out.append(res)
+        mk.close()
+    for k in out[0]:
+        n = min(len(out[0][k]), len(out[1][k]))
+        assert n > 0
+        np.testing.assert_array_equal(out[0][k][:n], out[1][k][:n])
