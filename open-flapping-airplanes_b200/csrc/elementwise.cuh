@@ -670,6 +670,14 @@ __device__ __forceinline__ AdamHP adam_hp(const AdamConst& h, int step) {
 // then the working copy Wact (type T) that forward, backward and the decoder read is refreshed. The gradient is read as GT
 // (fp32 single-GPU buffer, or the all-reduced bf16 bucket) and multiplied by grad_scale (1/world size).
 // nodecay: sorted disjoint [start,end) element ranges relative to W. Task = `chunk` elements (see opt_chunk); n and ranges multiples of 4.
+// which of the elements i .. i + 3 lie in a no-decay range (bit per element); ranges from `r` on. Out of line: one range in a hundred tasks
+static __device__ __noinline__ unsigned no_decay4(const int2* nd, int r, int n, size_t i) {
+  unsigned mask = 0;
+#pragma unroll 1
+  for (; r < n && (size_t)nd[r].x < i + 4; r++)
+    for (int k = 0; k < 4; k++) if (i + k >= (size_t)nd[r].x && i + k < (size_t)nd[r].y) mask |= 1u << k;
+  return mask;
+}
 struct AdamMath {                     // the per-task constants and the four-element update shared by both task bodies
   float step_size, inv_sqrt_bc2, decay_mul, one_minus_b1, one_minus_b2, b2, eps, gscale;
   const int2* nd; int n_nd, first_nd; bool any_nd;
@@ -685,17 +693,12 @@ struct AdamMath {                     // the per-task constants and the four-ele
     first_nd = lo;
     any_nd = lo < n_nodecay && (size_t)nodecay[lo].x < chunk_end;
   }
-  __device__ __forceinline__ bool decays(size_t idx) const {
-    if (!any_nd) return true;
-    int ri = first_nd;
-    while (ri < n_nd && (size_t)nd[ri].y <= idx) ri++;
-    return !(ri < n_nd && idx >= (size_t)nd[ri].x);
-  }
   __device__ __forceinline__ void update4(size_t i, float* w, const float* g, float* m, float* v) const {
+    const unsigned still = any_nd ? no_decay4(nd, first_nd, n_nd, i) : 0u;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const float gg = g[k] * gscale;
-      const float p = decays(i + k) ? w[k] * decay_mul : w[k];
+      const float p = (still >> k) & 1u ? w[k] : w[k] * decay_mul;
       m[k] = m[k] + (gg - m[k]) * one_minus_b1;
       v[k] = fmaf(v[k], b2, one_minus_b2 * gg * gg);
       w[k] = p - step_size * (m[k] / (sqrtf(v[k]) * inv_sqrt_bc2 + eps));
@@ -703,9 +706,9 @@ struct AdamMath {                     // the per-task constants and the four-ele
   }
 };
 // elements [begin, end) with loads issued by the threads themselves (the fp32 preset, and the ragged end of a staged task)
-template <class T, class GT>
+template <class T, class GT, int U = 4>
 __device__ __forceinline__ void adamw_span_direct(const AdamMath& A, size_t begin, size_t end, float* W, const GT* G, float* M, float* Vv, T* Wact) {
-#pragma unroll 4
+#pragma unroll(U)
   for (size_t i = begin + (size_t)threadIdx.x * 4; i < end; i += NTHR * 4) {
     float w[4], g[4], m[4], v[4];
     ld4(W + i, w); ld4(G + i, g); ld4(M + i, m); ld4(Vv + i, v);
@@ -738,7 +741,6 @@ __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, fl
   const size_t cs = (size_t)task * chunk;
   if (cs >= n) return;
   const size_t ce = cs + chunk < n ? cs + chunk : n;
-  AdamMath A; A.init(hp, nodecay, n_nodecay, cs, ce);
   const int tid = threadIdx.x;
   const bool aligned = ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(M) | reinterpret_cast<uintptr_t>(Vv) | reinterpret_cast<uintptr_t>(G)) & 15) == 0;
   const int nfull = aligned ? (int)((ce - cs) / ADAM_TILE) : 0;
@@ -755,13 +757,15 @@ __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, fl
     fence_proxy_async();     // gradients and the previous step's W/M/V were written with ordinary stores; the stages were last read by ordinary loads
     for (int k = 0; k < ADAM_STAGES && k < nfull; k++) issue(k);
   }
+  AdamMath A; A.init(hp, nodecay, n_nodecay, cs, ce);     // while the first tiles travel: powers and a cosine in double
+#pragma unroll 1
   for (int k = 0; k < nfull; k++) {
     const uint32_t u = u0 + (uint32_t)k, s = u % ADAM_STAGES;
     const bool ok = mbar_wait(bar0 + 8u * s, (u / ADAM_STAGES) & 1u, st);
     if (ok) {
       const unsigned char* sp = smem + s * ADAM_STAGE_BYTES;
       const size_t i0 = cs + (size_t)k * ADAM_TILE;
-#pragma unroll
+#pragma unroll 1
       for (int q = 0; q < ADAM_TILE / (NTHR * 4); q++) {
         const int e = q * NTHR * 4 + tid * 4;             // a warp touches 512 contiguous bytes of each array: no bank conflicts
         float w[4], g[4], m[4], v[4];
@@ -784,7 +788,7 @@ __device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, fl
     if (tid == 0 && k + ADAM_STAGES < nfull) { fence_proxy_async(); issue(k + ADAM_STAGES); }
   }
   if (tid == 0 && nfull > 0) tiles = u0 + (uint32_t)nfull;
-  adamw_span_direct<T, GT>(A, cs + (size_t)nfull * ADAM_TILE, ce, W, G, M, Vv, Wact);
+  adamw_span_direct<T, GT, 1>(A, cs + (size_t)nfull * ADAM_TILE, ce, W, G, M, Vv, Wact);
 }
 
 // out[i] = T(part0[i] + part1[i] + ...) in index order: the reduce of a split-K GEMM. Task = 16,384 elements (n % 8 == 0).

@@ -187,6 +187,23 @@ def test_adamw_three_steps(ofa, K, oracle, bf, gbf, direct):
     assert relmax(dWa.download(), rnd(Wr, bf)) <= (1e-2 if bf else 1e-6)
 
 
+@pytest.mark.parametrize("ranges", [[(0, 4)], [(2044, 2052)], [(4, 8), (8, 16), (2048, 4096)], [(65532, 65540), (70000, 70004)], [(5, 6), (4097, 4103), (73726, 73728)]])
+@pytest.mark.parametrize("direct", [0, 1])
+def test_adamw_no_decay_ranges_at_their_edges(ofa, K, oracle, ranges, direct):
+    """Ranges that begin and end at a group of four, a staged tile (2,048) or a task (65,536), and inside a group: exactly their elements keep from decaying."""
+    n = 73728
+    g = torch.Generator().manual_seed(3)
+    W0, G = torch.randn(n, generator=g) + 3.0, torch.randn(n, generator=g)
+    hp = (0.1, 0.9, 0.999, 1e-8, 0.5, 1.0)             # lr * weight decay = 0.05: an element on the wrong side is off by 5 %
+    bufs = [ofa.DeviceBuffer.from_host(t.numpy()) for t in (W0, G, torch.zeros(n), torch.zeros(n))]
+    wa, nd = ofa.DeviceBuffer((n,), "bf16"), ofa.DeviceBuffer.from_host(np.array(ranges, dtype=np.int32).reshape(-1))
+    ofa.run_phases(K.DTYPE_BF16, dict(vocab=128, d_model=768, n_layer=1, n_head=12, ctx_len=128, batch=1),
+                   [ofa.phase(K.TK_ADAMW, bufs + [wa, nd], n=n, i0=len(ranges), i2=direct)], adam=hp)
+    ref, _, _ = oracle.adamw_ref(W0, [G], ranges, lr=hp[0], betas=(hp[1], hp[2]), eps=hp[3], wd=hp[4], grad_scale=hp[5])
+    # decay, quotient, its product with the step size (at most lr here) and the difference round once each: 4 * 2^-24 of |w| + lr, near w = 0 that of lr
+    np.testing.assert_allclose(bufs[0].download(), ref.numpy(), rtol=1e-5, atol=4 * 2.0 ** -24 * hp[0])
+
+
 GEMM_CASES = [  # (layout, epi, M, N, K)
     (0, 0, 256, 256, 128), (0, 1, 256, 384, 192), (0, 2, 128, 512, 64), (1, 0, 384, 256, 256), (1, 3, 256, 256, 128),
     (2, 4, 256, 384, 512), (2, 0, 128, 128, 1024), (0, 4, 256, 256, 256), (0, 0, 512, 2304, 768), (1, 0, 256, 50304, 768), (2, 4, 768, 768, 4096),
