@@ -157,7 +157,7 @@ __device__ __forceinline__ void warp_arrive(uint32_t b) { __syncwarp(); if ((thr
 // written back by its softmax thread between two products. Sum and output share the reference point, so the result is the
 // same softmax; after the first tiles of a row the rescale is rare and the step is one pass over S.
 constexpr float RESCALE_LOG2 = 8.f;
-__device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b, int h, int qt, int T, int H, unsigned char* smem,
+__device__ __forceinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b, int h, int qt, int T, int H, unsigned char* smem,
                                       AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
   const AttnPipe a0 = ap;
   const int D = H * DH;
@@ -325,7 +325,7 @@ __device__ __noinline__ void fwd_task(const Maps* mp, bf16* o, float* lse, int b
 
 // ---------------------------------------------------------------------------------------------- backward: dK, dV
 // Task (b, h, kt): 128 key rows k0 = kt*128; walks query blocks of 64 rows from the diagonal to the end of the sequence.
-__device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int kt, int T, int H,
+__device__ __forceinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int kt, int T, int H,
                                            unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
   const AttnPipe a0 = ap;
   const int D = H * DH, ld = 3 * D;
@@ -466,7 +466,7 @@ __device__ __noinline__ void bwd_dkdv_task(const Maps* mp, const float* lse, con
 
 // ---------------------------------------------------------------------------------------------- backward: dQ
 // Task (b, h, qt): 128 query rows; walks key blocks of 64 rows from 0 to the diagonal.
-__device__ __noinline__ void bwd_dq_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int qt, int T, int H,
+__device__ __forceinline__ void bwd_dq_task(const Maps* mp, const float* lse, const float* Dr, bf16* dqkv, int b, int h, int qt, int T, int H,
                                          unsigned char* smem, AttnPipe& ap, uint32_t tmem, DevStatus* st, int phase_id, int task, EarlyTicket& et) {
   const AttnPipe a0 = ap;
   const int D = H * DH, ld = 3 * D;

@@ -160,7 +160,7 @@ template <int D> __host__ __device__ constexpr size_t ln_bwd_smem_bytes() { retu
 // the dgamma terms, pass 2 recomputes xhat and g from the raw vectors (a few FMAs) instead of keeping them. The two rows of a
 // warp go one after the other: with both in flight the persistent kernel's 128-register budget spilled.
 template <class T, int D>
-__device__ __noinline__ void ln_bwd_task(int task, T* dx, float* dgamma_part, const T* dy, const T* x, const float* mean,
+__device__ __forceinline__ void ln_bwd_task(int task, T* dx, float* dgamma_part, const T* dy, const T* x, const float* mean,
                                             const float* rstd, const T* gamma, const T* dres, int N, unsigned char* smem) {
   using R = RowRegs<T, D>;
   using S = RowShare<T, D>;
@@ -428,7 +428,7 @@ __device__ __forceinline__ void ce_task_bulk(int task, bf16* logits, const int* 
 // across row boundaries; nothing waits for a whole row. `bar_lo`, `bar_hi` = two pairs of block-private mbarriers (count 1), `chunks` = running
 // count of chunks this block has staged (in shared memory, advanced by thread 0). V must be a multiple of 8.
 constexpr int CE_CHUNK = 12288, CE_STAGES = 4;            // elements per chunk (24 KB of bf16)
-static __device__ __noinline__ void ce_task_stream(int task, bf16* logits, const int* targets, float* loss, const float2* part, int tiles_n,
+static __device__ __forceinline__ void ce_task_stream(int task, bf16* logits, const int* targets, float* loss, const float2* part, int tiles_n,
                                                int N, int V, float inv_n, unsigned char* smem, uint32_t bar_lo, uint32_t bar_hi, uint32_t& chunks,
                                                const DevStatus* st) {
   auto sbar = [&](uint32_t sg) { return sg < 2 ? bar_lo + 8u * sg : bar_hi + 8u * (sg - 2); };   // the four barriers sit in two free pairs of the control area
@@ -530,7 +530,7 @@ __host__ __device__ constexpr size_t embed_bwd_wte_smem_bytes(int N) { return 10
 // Without `accumulate` every row of the chunk is written (zeros where the token is absent), so the gradient buffer needs no
 // clearing between steps. Shared memory: 8 warp counts + 128 row counts, then int list[N], then one byte per list entry.
 template <class T, int D, class GT>
-__device__ __noinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0, const int* tok, int N, int V, int vchunk, int accumulate,
+__device__ __forceinline__ void embed_bwd_wte_task(int task, GT* dwte, const T* dx0, const int* tok, int N, int V, int vchunk, int accumulate,
                                                 unsigned char* smem) {
   using R = RowRegs<T, D>;
   constexpr int VN = R::VN, NV = R::NV;
@@ -735,7 +735,7 @@ __device__ __forceinline__ void adamw_task(int task, float* W, const GT* G, floa
 // (in shared memory, advanced by thread 0). The ragged end of a range (fewer than 2,048 elements) goes through the direct loop.
 constexpr int ADAM_TILE = 2048, ADAM_STAGES = 3, ADAM_STAGE_BYTES = 32768;
 template <class T, class GT>
-__device__ __noinline__ void adamw_task_bulk(int task, float* W, const GT* G, float* M, float* Vv, T* Wact, size_t n, AdamHP hp,
+__device__ __forceinline__ void adamw_task_bulk(int task, float* W, const GT* G, float* M, float* Vv, T* Wact, size_t n, AdamHP hp,
                                                 const int2* nodecay, int n_nodecay, int chunk, unsigned char* smem, uint32_t bar0, uint32_t& tiles,
                                                 const DevStatus* st) {
   const size_t cs = (size_t)task * chunk;

@@ -382,7 +382,7 @@ __device__ __forceinline__ void dispatch_bn(const PhaseDesc& d, int task, unsign
   else gemm_tc_task<LAYOUT, EPI, 128>(d.g, d.tiles_m, task, smem, gp, st, phase_id, et, d.i0);
 }
 // run-time dispatch over the (layout, epilogue) pairs the training graph uses
-__device__ __noinline__ void run(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, EarlyTicket& et) {
+__device__ __forceinline__ void run(const PhaseDesc& d, int task, unsigned char* smem, GemmPipe& gp, DevStatus* st, int phase_id, EarlyTicket& et) {
   switch (d.layout * 8 + d.epi) {
     case GL_NN * 8 + GE_STORE: dispatch_bn<GL_NN, GE_STORE>(d, task, smem, gp, st, phase_id, et); break;
     case GL_NN * 8 + GE_RES:   dispatch_bn<GL_NN, GE_RES>(d, task, smem, gp, st, phase_id, et); break;

@@ -48,6 +48,9 @@ static_assert(sizeof(PhaseDesc) == 192 && sizeof(SchedRec) == 48, "control area 
 static_assert(CTRL_STATE + sizeof(BlockState) <= attn_tc::BAR0, "scheduling state does not fit the control area");
 
 // ---------------------------------------------------------------------------------------------- one training task
+// The tasks are inlined here: as functions they saved the registers they use in local memory, which next to no L1 sends to L2, and took their
+// arguments from there (small model of 384 tokens 1,525 -> 1,471 us for two steps, one layer of 4,096 540 -> 520, attention forward 25.2 -> 24.6,
+// GELU' product 35.2 -> 33.3). LayerNorm forward is the exception, 6.4 us as a function and 7.2 inlined, where it spills.
 template <class T, int D, int DH>
 __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d, int ph, int local, int step, unsigned char* smem, BlockState& B) {
   const ModelDims& md = C.md;
