@@ -483,13 +483,15 @@ __device__ __forceinline__ void task_attwo(const DecodeParams& P, const ModelDim
   __syncthreads();
   trace(P.trace, tr, 27);
   if (tid < DH) {
+    static_assert(NW == 8 && DH <= NTHR, "one exponential a lane");
     float M = S.scratch[0];
 #pragma unroll
     for (int i = 1; i < NW; i++) M = fmaxf(M, S.scratch[i]);
+    const float mine = S.scratch[tid & 7], fl = mine == -INFINITY ? 0.f : expf(mine - M);      // lane i: the factor of warp i % 8
     float o = 0.f, sm = 0.f;
 #pragma unroll
     for (int i = 0; i < NW; i++) {
-      const float fw = S.scratch[i] == -INFINITY ? 0.f : expf(S.scratch[i] - M);
+      const float fw = __shfl_sync(DH >= 32 ? 0xffffffffu : (1u << (DH & 31)) - 1u, fl, i);
       o += fw * S.red[i * DH + tid]; sm += fw * S.scratch[NW + i];
     }
     ob[tid] = round_to<T>(o / sm);
