@@ -428,12 +428,13 @@ __device__ __forceinline__ void job_loop(const Ctx& C, const Job& J, unsigned ch
     // for the SM's outstanding stores (about a microsecond after a GEMM epilogue); on its own thread it runs beside the ticket's
     // round trip and the next claim instead of in front of them.
     if (tid == 0) {
+      const u64 t1 = PROF ? gtimer() : 0;              // before the ticket: behind it the task would seem to last until it is there
       unsigned early = 0;
       if constexpr (use_tc) { early = B.early.taken; B.early.taken = 0; }
       if (early != 0) next_g = early - 1u; else next_g = atomicAdd(J.ticket, 1u);
       have_next = true;
       if (PROF) {
-        const u64 t1 = gtimer(), t0 = t_start; t_end = t1;
+        const u64 t0 = t_start; t_end = t1;
         const int4 e = B.sel[turn]; const int ph = e.z;
         if (!TRAIN && C.dp.trace && e.w == 0 && (ph == 0 || ph == 2)) C.dp.trace[17 + ph] = t1;
         t_busy += t1 - t0;
@@ -479,7 +480,7 @@ __device__ __forceinline__ void idle_block(const Ctx& C) {
 // without the fence, 52.2 with the loop inlined and 51.8 so, although later launches have nothing to fence.
 __device__ __noinline__ void fence_maps(const unsigned char* maps, int n) { for (int q = threadIdx.x; q < n; q += NTHR) tmap_fence(maps + 128 * (size_t)q); }
 
-// One kernel for launches that train, one for those that serve, one for both and one that also keeps time tables, because what a launch does not
+// One kernel for launches that train, one for those that serve, one for both, each with and without time tables, because what a launch does not
 // run lies between what it does. Instructions are what most of a small task waits for: measured with straight-line code in a loop, 8 warps on an
 // SM, a warp instruction takes 1.9 clocks of its scheduler when the loop has 2 KB, 2.4 at 16 to 32 KB and 6.3 from 48 KB on (one warp a
 // scheduler: 1.1, 2.7, 6.1), and a task's code is not met again before hundreds of KB of others. So what is executed once per task is kept

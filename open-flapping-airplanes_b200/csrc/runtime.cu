@@ -308,9 +308,10 @@ template <class T, int D, int DH> cudaError_t launch_kernel(const Ctx& C, int nb
     kernel<<<nblocks, NTHR, smem, s>>>(C);
     return cudaGetLastError();
   };
-  if (C.sched_flags & 2) return launch(ofa_kernel<T, D, DH, true, true, true>);
-  if (C.use_train && C.use_decode) return launch(ofa_kernel<T, D, DH, true, true, false>);
-  return C.use_train ? launch(ofa_kernel<T, D, DH, true, false, false>) : launch(ofa_kernel<T, D, DH, false, true, false>);
+  const bool prof = (C.sched_flags & 2) != 0;
+  if (C.use_train && C.use_decode) return prof ? launch(ofa_kernel<T, D, DH, true, true, true>) : launch(ofa_kernel<T, D, DH, true, true, false>);
+  if (C.use_train) return prof ? launch(ofa_kernel<T, D, DH, true, false, true>) : launch(ofa_kernel<T, D, DH, true, false, false>);
+  return prof ? launch(ofa_kernel<T, D, DH, false, true, true>) : launch(ofa_kernel<T, D, DH, false, true, false>);
 }
 
 // Tasks whose shared-memory need grows with the batch or the context must fit the block's task area: on the bf16 path that is

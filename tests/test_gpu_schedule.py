@@ -222,7 +222,7 @@ def test_spread_adamw_gives_the_same_bits_in_every_form(ofa, monkeypatch, layers
 @pytest.mark.parametrize("preset", ["gpt_s", "tiny"])
 @pytest.mark.parametrize("job", ["train", "serve", "both"])
 def test_every_form_of_the_kernel_gives_the_same_bits(ofa, preset, job):
-    """A launch that trains, serves or does both runs a kernel of its own; one that keeps time tables runs the form that can do everything."""
+    """A launch that trains, serves or does both runs a kernel of its own, with or without time tables."""
     out = []
     for profile in (1, 0):
         cfg = ofa.default_config(preset)
