@@ -231,7 +231,9 @@ bool make_job(const std::vector<HostPhase>& ph, int last_phase, HostJob& hj, std
     }
     if (nt[i] <= 0) { err = "phase without tasks: " + ph[i].name; return false; }
   }
-  if (nph >= 65536 || (long long)RB_STRIDE * nph * std::max(nrb, 0) >= (1 << 28)) { err = "too many phases"; return false; }
+  if (nph >= 65536) { err = "too many phases"; return false; }
+  // a dependency names its counter in DEP_WORD bits: a graph with so many row blocks that they might not reach waits per phase
+  if ((long long)DONE_STRIDE * nph + (long long)RB_STRIDE * nph * nrb > DEP_WORD) nrb = 0;
   // which phases count their completions per row block: those that say how their tasks map to row blocks, have a whole number of
   // tasks per row block, and are waited for at that grain by somebody
   std::vector<int> rb_off(nph, -1); int rb_total = 0;

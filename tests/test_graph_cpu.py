@@ -232,3 +232,11 @@ def test_spread_adamw_comes_after_every_reader_of_its_weights(ofa, kw):
             assert p["name"] in above[names.index("step barrier")]
     assert pieces > L
     mk.close()
+
+
+@pytest.mark.parametrize("layers,batch", [(64, 9600), (12, 60000), (1, 120000)])
+def test_forward_graphs_of_many_row_blocks_are_planned(ofa, layers, batch):
+    """However many 128-token row blocks times phases there are: a graph whose counters a dependency cannot name waits per phase."""
+    mk = plan(ofa, "gpt_s", mode=ofa.capi.MODE_FORWARD, n_layer=layers, ctx_len=1024, batch=batch, vocab=128, valid_vocab=128)
+    assert len(mk.phases()) > 7 * layers and all(p["ntasks"] > 0 for p in mk.phases())
+    mk.close()
