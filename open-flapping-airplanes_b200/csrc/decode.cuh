@@ -300,7 +300,7 @@ __device__ __forceinline__ void gemv_shares(const T* W, const float* x, float* p
     float a[VN];
 #pragma unroll
     for (int i = 0; i < VN; i++) a[i] = 0.f;
-#pragma unroll 4
+#pragma unroll                                         // whole: by fours a served token takes 182.2 instead of 181.4 us, on 24 SMs 340.3 instead of 339.7
     for (int q = 0; q < KPT; q++) {
       const int k = kg * KPT + q;
       float f[VN]; cvt16<T>(*reinterpret_cast<const uint4*>(W + (size_t)k * NC + c), f);
