@@ -493,7 +493,7 @@ __device__ __forceinline__ void idle_block(const Ctx& C) {
 // without the fence, 52.2 with the loop inlined and 51.8 so, although later launches have nothing to fence.
 __device__ __noinline__ void fence_maps(const unsigned char* maps, int n) { for (int q = threadIdx.x; q < n; q += NTHR) tmap_fence(maps + 128 * (size_t)q); }
 
-// One kernel for launches that train, one for those that serve, one for both, each with and without time tables, because what a launch does not
+// One kernel for launches that train, one for those that serve (bf16), one for both, each with and without time tables, because what a launch does not
 // run lies between what it does. Instructions are what most of a small task waits for: measured with straight-line code in a loop, 8 warps on an
 // SM, a warp instruction takes 1.9 clocks of its scheduler when the loop has 2 KB, 2.4 at 16 to 32 KB and 6.3 from 48 KB on (one warp a
 // scheduler: 1.1, 2.7, 6.1), and a task's code is not met again before hundreds of KB of others. So what is executed once per task is kept
