@@ -558,8 +558,10 @@ __device__ __forceinline__ void task_head(const DecodeParams& P, const ModelDims
   float s[RPW];                                        // rows past the vocabulary hold whatever the buffer held: they are not read below
 #pragma unroll
   for (int rr = 0; rr < RPW; rr++) s[rr] = 0.f;
-#pragma unroll 1
-  for (int vi = lane; vi < VPR; vi += 32) {
+#pragma unroll                                         // as a rolled loop 181.7 instead of 181.1 us a token, on 24 SMs, where a block runs 16 of these, 340.0 instead of 336.2
+  for (int i = 0; i < (VPR + 31) / 32; i++) {
+    const int vi = lane + 32 * i;
+    if (VPR % 32 != 0 && vi >= VPR) break;
     float x[VN];
 #pragma unroll
     for (int k = 0; k < VN; k += 4) {
