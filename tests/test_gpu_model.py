@@ -227,3 +227,25 @@ def test_phase_windows_follow_the_dependency_chain(ofa, oracle):
                 # the dependency's last task ended before this phase's first began (its end stamp is read just after it signals: 5 us of slack)
                 assert win[dep][1] <= win[i][0] + 5000, (names[dep], names[i])
     mk.close()
+
+
+@pytest.mark.parametrize("check", ["test_tiny_step_matches_oracle", "test_tiny_gradients_match_oracle", "test_tiny_greedy_decode_is_token_exact", "test_bf16_logits_match_oracle", "test_bf16_gradients_match_oracle",
+                                   "test_bf16_loss_curve_and_repeatability", "decode:test_bf16_decode_is_bitwise_independent_of_the_schedule", "decode:test_bf16_decode_restarts_when_the_context_is_full",
+                                   "decode:test_decode_beside_training_equals_decode_only_with_frozen_weights", "decode:test_tiny_fp32_decode_resumes_exactly_across_launches_beside_training"])
+def test_parity_without_time_tables(ofa, oracle, monkeypatch, check):
+    """The presets keep time tables; a launch without them runs other kernels. The checks against the oracle, held by those too."""
+    import inspect
+    preset_of = ofa.default_config
+
+    def plain(preset):
+        cfg = preset_of(preset)
+        cfg.sched_profile = 0
+        return cfg
+
+    monkeypatch.setattr(ofa, "default_config", plain)
+    if check.startswith("decode:"):
+        import test_gpu_decode as where
+        f = getattr(where, check[len("decode:"):])
+    else:
+        f = globals()[check]
+    f(ofa, oracle, *[{"tied": False, "grad_bf16": 1}[a] for a in list(inspect.signature(f).parameters)[2:]])

@@ -255,3 +255,131 @@ def test_every_form_of_the_kernel_gives_the_same_bits(ofa, preset, job):
         n = min(len(out[0][k]), len(out[1][k]))
         assert n > 0
         np.testing.assert_array_equal(out[0][k][:n], out[1][k][:n])
+
+
+def _form(ofa, preset, job, profile=0, **kw):
+    """A context of one kind of launch on the same partition of the SMs, weights and (training) tokens loaded; frozen weights unless told otherwise."""
+    cfg = ofa.default_config(preset)
+    cfg.sched_profile = profile
+    if preset == "gpt_s":
+        cfg.vocab = cfg.valid_vocab = 1152
+        cfg.n_layer, cfg.ctx_len, cfg.batch = 2, 256, 1
+    cfg.infer_sms, cfg.reserved_sms, cfg.train_sms, cfg.adam_interleave = 24, 8, 116, -1
+    cfg.n_prompt, cfg.answer_len, cfg.temperature = 3, 16, 0.0
+    cfg.lr_max = cfg.lr_min = 0.0
+    cfg.use_decode = int(job != "train")
+    if job == "serve":
+        cfg.mode = ofa.capi.MODE_DECODE_ONLY
+    for k, v in kw.items():
+        setattr(cfg, k, v)
+    mk = ofa.Megakernel(cfg)
+    g = np.random.default_rng(5)
+    mk.load_weights(g.standard_normal(mk.num_params, dtype=np.float32) * 0.02)
+    if job != "serve":
+        mk.set_tokens(g.integers(0, cfg.vocab, size=1 << 13, dtype=np.uint32))
+    return mk
+
+
+@pytest.mark.parametrize("tables", ["parameter", "global"])
+@pytest.mark.parametrize("preset", ["gpt_s", "tiny"])
+def test_kinds_of_launch_agree(ofa, monkeypatch, preset, tables):
+    """What a launch that does both trains is what one that only trains does, what it serves is what one that only serves does; first tickets
+    of both jobs in the kernel parameter or in global memory. No time tables."""
+    if tables == "global":
+        monkeypatch.setenv("OFA_B200_GLOBAL_RECS", "1")
+    out = {}
+    for job in ("train", "serve", "both"):
+        mk = _form(ofa, preset, job)
+        mk.run(40, timeout_ms=60000)
+        if job != "serve":
+            out[job, "loss"], out[job, "w"] = mk.losses()[-40:].copy(), mk.read_weights()
+        if job != "train":
+            t = np.asarray(mk.decode_tokens())
+            out[job, "tokens"] = t[t >= 0]
+        mk.close()
+    np.testing.assert_array_equal(out["both", "loss"], out["train", "loss"])
+    np.testing.assert_array_equal(out["both", "w"], out["train", "w"])
+    n = min(len(out["both", "tokens"]), len(out["serve", "tokens"]))
+    assert n > 0
+    np.testing.assert_array_equal(out["both", "tokens"][:n], out["serve", "tokens"][:n])
+
+
+@pytest.mark.parametrize("profile", [0, 1])
+@pytest.mark.parametrize("preset,job", [("gpt_s", "serve"), ("gpt_s", "both"), ("tiny", "serve"), ("tiny", "both")])
+def test_abort_of_a_launch_that_serves(ofa, preset, job, profile):
+    """The abort word reaches a claim as a copy and a wait directly; the context can be used again."""
+    mk = _form(ofa, preset, job, profile)
+    n = 400000 if job == "serve" else 100000 if preset == "tiny" else 40000             # 8 s and more
+    mk.launch(n)
+    with pytest.raises(ofa.OfaError) as e:
+        mk.wait(100)
+    assert e.value.code == ofa.capi.TIMEOUT
+    assert mk.abort() == ofa.capi.OK
+    t0 = time.monotonic()
+    with pytest.raises(ofa.OfaError) as e:
+        mk.wait(10000)
+    assert time.monotonic() - t0 < 1.5
+    assert e.value.code == ofa.capi.DEVICE_ABORT and e.value.status.dev_code == 0
+    mk.run(20, timeout_ms=60000)
+    mk.close()
+
+
+def test_expired_wait_of_a_launch_that_serves(ofa):
+    """Serving alone, every wait given 1.5 us: one runs out, the kernel returns and says which (ST_DEP_TIMEOUT)."""
+    mk = _form(ofa, "gpt_s", "serve", infer_sms=0, timeout_s=1e-6)
+    mk.launch(2000)
+    with pytest.raises(ofa.OfaError) as e:
+        mk.wait(20000)
+    assert e.value.code == ofa.capi.DEVICE_ABORT and e.value.status.dev_code == 1
+    assert 0 <= e.value.status.phase < len(mk.decode_phases())
+    mk.close()
+
+
+def test_expired_external_wait_beside_a_serving_job(ofa):
+    """The training job gives up (a flag that nobody raises); the serving blocks leave with it."""
+    mk = _form(ofa, "gpt_s", "both", ext_sync=1, grad_bf16=1, timeout_s=0.2, adam_interleave=0)
+    mk.launch(2)
+    t0 = time.monotonic()
+    with pytest.raises(ofa.OfaError) as e:
+        mk.wait(20000)
+    assert time.monotonic() - t0 < 5.0
+    assert e.value.code == ofa.capi.DEVICE_ABORT and e.value.status.dev_code == 6 and mk.decode_steps > 0
+    mk.close()
+
+
+@pytest.mark.parametrize("ctx,profile", [(1152, 0), (2048, 0), (2048, 1)])
+def test_waits_for_more_than_eight_row_blocks(ofa, oracle, monkeypatch, ctx, profile):
+    """Beyond 1,024 tokens a sequence has more row blocks than a wait's lanes take at once: gradients against the oracle (bounds of the model
+    tests), and the same bits in a permuted task order and when every dependency is of whole phases."""
+    lib = ofa.capi.load()
+    ocfg = oracle.OracleConfig(V=512, D=768, L=1, H=12, T=ctx, B=1, tied=False)
+    w0 = oracle.init_weights(ocfg)
+    tokens = oracle.synthetic_tokens(ocfg.V, 1 << 14, 0)
+    starts = oracle.batch_starts(ocfg, 1 << 14, 1)
+    cfg = ofa.default_config("gpt_s")
+    cfg.vocab, cfg.valid_vocab, cfg.n_layer, cfg.ctx_len, cfg.batch, cfg.mode, cfg.sched_profile = ocfg.V, ocfg.V, 1, ctx, 1, ofa.capi.MODE_NO_OPT, profile
+    got = []
+    try:
+        for seed, phase_deps in ((0, False), (4711, False), (0, True)):
+            lib.ofa_debug_set_task_shuffle(seed)
+            if phase_deps:
+                monkeypatch.setenv("OFA_B200_PHASE_DEPS", "1")
+            mk = ofa.Megakernel(cfg)
+            mk.load_weights(oracle.flatten(ocfg, w0)); mk.set_tokens(tokens); mk.set_starts(starts.astype(np.uint32))
+            mk.run(1, timeout_ms=60000)
+            got.append((float(mk.losses()[0]), mk.read_grads()))
+            spans = {n: mk.param_span(n) for n in ("wte", "wpe", "lm_head", "gf", "L0.g1", "L0.Wqkv", "L0.Wo", "L0.g2", "L0.Wup", "L0.Wdn")}
+            mk.close()
+    finally:
+        lib.ofa_debug_set_task_shuffle(0)
+    for loss, grads in got[1:]:
+        assert loss == got[0][0]
+        np.testing.assert_array_equal(grads, got[0][1])
+    if profile:
+        return
+    ref = oracle.train(ocfg, w0, tokens, starts, 1, precision="bf16_points", grab_step0=True)
+    assert abs(got[0][0] - ref["losses"][0]) <= 1e-2 * ref["losses"][0]
+    gref = oracle.flatten(ocfg, ref["grads0"])
+    for name, (off, cnt) in spans.items():
+        a, b = got[0][1][off:off + cnt].astype(np.float64), gref[off:off + cnt].astype(np.float64)
+        assert np.linalg.norm(a - b) <= 3e-2 * np.linalg.norm(b), name

@@ -204,6 +204,25 @@ def test_adamw_no_decay_ranges_at_their_edges(ofa, K, oracle, ranges, direct):
     np.testing.assert_allclose(bufs[0].download(), ref.numpy(), rtol=1e-5, atol=4 * 2.0 ** -24 * hp[0])
 
 
+@pytest.mark.parametrize("n", [2048, 73728, 65536 + 2044])
+def test_adamw_of_a_gradient_that_cannot_be_staged(ofa, K, n):
+    """A bf16 gradient that begins 8 bytes past a 16-byte boundary is read directly for the whole range: the bits of the staged update."""
+    g = torch.Generator().manual_seed(4)
+    W0, G, M0 = torch.randn(n, generator=g), torch.randn(n + 4, generator=g), 0.1 * torch.randn(n, generator=g)
+    V0 = torch.rand(n, generator=g)
+    nd = ofa.DeviceBuffer.from_host(np.array([4, 12, 2040, 2048], dtype=np.int32))
+    out = []
+    for off in (0, 4):
+        bufs = [ofa.DeviceBuffer.from_host(t.numpy()) for t in (W0, M0, V0)]
+        grad, wa = ofa.DeviceBuffer.from_host(torch.roll(G, off).numpy(), "bf16"), ofa.DeviceBuffer((n,), "bf16")
+        assert grad.ptr.value % 16 == 0
+        ofa.run_phases(K.DTYPE_BF16, dict(vocab=128, d_model=768, n_layer=1, n_head=12, ctx_len=128, batch=1),
+                       [ofa.phase(K.TK_ADAMW, [bufs[0], grad.ptr.value + 2 * off, bufs[1], bufs[2], wa, nd], n=n, i0=2, i1=1)], adam=(0.1, 0.9, 0.999, 1e-8, 0.5, 1.0))
+        out.append([b.download() for b in (*bufs, wa)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
 GEMM_CASES = [  # (layout, epi, M, N, K)
     (0, 0, 256, 256, 128), (0, 1, 256, 384, 192), (0, 2, 128, 512, 64), (1, 0, 384, 256, 256), (1, 3, 256, 256, 128),
     (2, 4, 256, 384, 512), (2, 0, 128, 128, 1024), (0, 4, 256, 256, 256), (0, 0, 512, 2304, 768), (1, 0, 256, 50304, 768), (2, 4, 768, 768, 4096),
