@@ -54,7 +54,7 @@ template <int BN> struct Cfg {
 // control area (1 KB at smem + BAR_OFFSET = the last 1,024 bytes of dynamic shared memory):
 //   [  0, 80) BN128: full[3] empty[3] accf[2] acce[2]     [ 80, 84) TMEM base slot     [ 96,104) serving fill barrier   [104,112) training bulk-copy barrier
 //   [112,128) and [160,176) streamed cross-entropy stage barriers [4]
-//   [176,224) BN256: full[2] empty[2] accf[1] acce[1]      [224,248) AdamW stage barriers [3]      [248,256), [1008,1024) profiling stamps
+//   [176,224) BN256: full[2] empty[2] accf[1] acce[1]      [224,248) AdamW stage barriers [3]      [248,256), [1008,1024) time tables (CTRL_T_*)
 //   [256,448) and [448,640) two slots for phase descriptors: the one being worked on and the next phase's, fetched ahead
 //   [640,832) the block's scheduling state and pipeline counters (BlockState)      [832,1008) attention barriers
 template <int BN> __device__ __forceinline__ uint32_t bar_full(uint32_t base, int s) { return base + BAR_OFFSET + Cfg<BN>::BAR0 + 8u * s; }

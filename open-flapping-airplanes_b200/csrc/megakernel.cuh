@@ -40,12 +40,15 @@ struct BlockState {
   int rbw[2];                        // thread 32: counter of the row block that the task writes, -1: none
   EarlyTicket early;
   attn_tc::AttnPipe ap; gemm_tc::GemmPipe gp;
-  uint32_t bulk_uses, adam_tiles, ce_chunks;       // uses of the bulk-copy barrier (control area byte 104), tiles staged by AdamW (224), chunks staged by the streamed cross-entropy (112, 120, 160, 168)
+  uint32_t bulk_uses, adam_tiles, ce_chunks;       // uses of the bulk-copy barrier (control area byte 104), tiles staged by AdamW (CTRL_ADAM_BAR), chunks staged by the streamed cross-entropy (112, 120, 160, 168)
 };
 constexpr int CTRL_DESC = 256, CTRL_STATE = CTRL_DESC + 2 * (int)sizeof(PhaseDesc);
+constexpr int CTRL_ADAM_BAR = 224, CTRL_T_END = 248, CTRL_T_BUSY = 1008, CTRL_T_START = 1016;      // the time tables' words
 static_assert(offsetof(DevStatus, abort) == 20 && sizeof(DevStatus) <= 32, "copied as its second 16 bytes");
 static_assert(sizeof(PhaseDesc) == 192 && sizeof(SchedRec) == 48, "control area map");
 static_assert(CTRL_STATE + sizeof(BlockState) <= attn_tc::BAR0, "scheduling state does not fit the control area");
+static_assert(attn_tc::BAR0 + 8 * attn_tc::NBAR <= CTRL_T_BUSY && CTRL_T_START + 8 <= CTRL_BYTES, "attention barriers reach into the time tables' words");
+static_assert(CTRL_ADAM_BAR + 8 * ew::ADAM_STAGES <= CTRL_T_END && CTRL_T_END + 8 <= CTRL_DESC, "AdamW barriers reach into the time tables' words");
 
 // ---------------------------------------------------------------------------------------------- one training task
 // The tasks are inlined here: as functions they saved the registers they use in local memory, which next to no L1 sends to L2, and took their
@@ -145,7 +148,7 @@ __device__ __forceinline__ void run_train_task(const Ctx& C, const PhaseDesc& d,
     case TK_ADAMW: {
       const ew::AdamHP hp = ew::adam_hp(C.hp, step + C.step_base);
       if constexpr (IsBf16<T>::value) {               // inputs staged by the copy engine (the fp32 preset's blocks have no room for the stages)
-        const uint32_t bar0 = smem_u32(smem + C.smem_bytes - CTRL_BYTES + 224);
+        const uint32_t bar0 = smem_u32(smem + C.smem_bytes - CTRL_BYTES + CTRL_ADAM_BAR);
         if (d.i2 == 0) {
           if (d.i1) ew::adamw_task_bulk<T, bf16>(local, (float*)d.p[0], (const bf16*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m, smem, bar0, B.adam_tiles, C.status);
           else ew::adamw_task_bulk<T, float>(local, (float*)d.p[0], (const float*)d.p[1], (float*)d.p[2], (float*)d.p[3], (T*)d.p[4], d.n, hp, (const int2*)d.p[5], d.i0, d.tiles_m, smem, bar0, B.adam_tiles, C.status);
@@ -274,7 +277,7 @@ __device__ __forceinline__ void job_loop(const Ctx& C, const Job& J, unsigned ch
   constexpr bool TRAIN = JOB == 0, RB = TRAIN && IsBf16<T>::value;        // RB: phases may count completions per row block
   unsigned char* ctrl = smem + (IsBf16<T>::value ? gemm_tc::SMEM_BYTES : C.smem_bytes) - CTRL_BYTES;   // the last bytes of dynamic shared memory are the block's control area (map in gemm_tc.cuh)
   BlockState& B = *reinterpret_cast<BlockState*>(ctrl + CTRL_STATE);
-  u64 &t_busy = *reinterpret_cast<u64*>(ctrl + 1008), &t_start = *reinterpret_cast<u64*>(ctrl + 1016), &t_end = *reinterpret_cast<u64*>(ctrl + 248);   // profiling only: thread 0, serving the end of a task by thread 64
+  u64 &t_busy = *reinterpret_cast<u64*>(ctrl + CTRL_T_BUSY), &t_start = *reinterpret_cast<u64*>(ctrl + CTRL_T_START), &t_end = *reinterpret_cast<u64*>(ctrl + CTRL_T_END);   // profiling only: thread 0, serving the end of a task by thread 64
   const int* pre = TRAIN ? C.train_pre : C.dec_pre;   // first tickets of the phases inside the kernel parameter, when they fit
   const bool ptab = (TRAIN ? C.train_pre_n : C.dec_pre_n) > 0;
   int tid = thread_index();
@@ -289,7 +292,7 @@ __device__ __forceinline__ void job_loop(const Ctx& C, const Job& J, unsigned ch
   if constexpr (use_tc) {
     if (tid == 0) {
       mbar_init(smem_u32(ctrl + 104), 1);
-      for (int q = 0; q < ew::ADAM_STAGES; q++) mbar_init(smem_u32(ctrl + 224 + 8 * q), 1);
+      for (int q = 0; q < ew::ADAM_STAGES; q++) mbar_init(smem_u32(ctrl + CTRL_ADAM_BAR + 8 * q), 1);
       for (int q = 0; q < 2; q++) { mbar_init(smem_u32(ctrl + 112 + 8 * q), 1); mbar_init(smem_u32(ctrl + 160 + 8 * q), 1); }   // streamed cross-entropy: four stages
     }
     attn_tc::block_init(B.ap, smem); gemm_tc::block_init(B.gp, smem, C.status);
