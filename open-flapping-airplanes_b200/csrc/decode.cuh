@@ -175,7 +175,7 @@ __device__ __forceinline__ bool prefetch(const DecodeParams& P, const ModelDims&
   return true;
 }
 
-// the block's fill has landed; out of line what comes after two probes
+// the block's fill has landed; out of line what comes after the first probe
 static __device__ __noinline__ bool wait_fill_slow(uint32_t bar, uint32_t parity, DevStatus* status, int layer, int t) {
   const bool ok = mbar_wait_slow(bar, parity, status);
   if (!ok && !aborted(status)) raise_abort(status, ST_MBAR_FULL_TIMEOUT, -2, t, layer);

@@ -4,8 +4,9 @@
 //
 // Scheduling model (same contract as the reference's job_loop / ofa_kernel, llm/b200/megakernel/ofa.cu:220-326):
 //   thread 0 of a block takes the next ticket g of its job with one fetch-add; g -> (step, phase, task) through the prefix
-//   table; it then waits until every dependency (phase p, step delta d) satisfies done[p] >= ntasks[p]*(step+1+d); the
-//   whole block runs the task; after a device-scope fence thread 0 bumps done[phase]. Phases are topologically ordered and
+//   table; warp 0 then waits until every dependency (phase p, step delta d) satisfies done[p] >= ntasks[p]*(step+1+d); the
+//   whole block runs the task; thread 32 then bumps done[phase], training and the last phase of a serving step after a
+//   device-scope fence, other serving phases with a releasing increment. Phases are topologically ordered and
 //   cross-step dependencies point backwards, so every dependency is a lower ticket and the lowest unfinished ticket is
 //   always runnable: no deadlock as long as every claimed ticket is eventually run, which holds because a block holds at
 //   most one ticket.
@@ -219,8 +220,9 @@ static __device__ __noinline__ bool wait_over(DevStatus* st, u64 t0, u64 limit, 
   return true;
 }
 // Dependency wait (bounded) of warp 0, whose lanes share the counters: up to four dependencies of the phase's record, the row blocks of one
-// that has them over eight lanes each; more than four (AdamW, the end of a step) over all lanes. cnt, w, nt = the record's number of dependencies and, for lane l, its dependency l % 4; h = {.., step, phase, task}, rb = {.., first, number of} row
-// blocks that the task reads. Returns 0 when every dependency is satisfied, -2 when the block must leave (job finished elsewhere, abort, or deadline).
+// that has them over eight lanes each; more than four (AdamW, the end of a step) over all lanes. cnt, w, nt = the record's number of
+// dependencies and, for lane l, its dependency l % 4; h = {.., step, phase, task}, rb = {first, number} of the row blocks that the task
+// reads. Returns 0 when every dependency is satisfied, -2 when the block must leave (job finished elsewhere, abort, or deadline).
 // Acquire loads: relaxed ones and a fence behind the last cost 310 clocks more per wait.
 template <int JOB>
 __device__ __forceinline__ int wait_deps(const Ctx& C, const Job& J, const int cnt, const int w, const int nt, const int4 h, const int2 rb) {
@@ -491,16 +493,16 @@ __device__ __forceinline__ void idle_block(const Ctx& C) {
   }
 }
 
-// For the first launch that uses TMA descriptors the host has just written. Out of line because of what a few more instructions in front of
-// the loop do: the code of a decoded token is larger than the instruction caches, and where it lies counts. A 256-token answer took 51.3 ms
-// without the fence, 52.2 with the loop inlined and 51.8 so, although later launches have nothing to fence.
+// For the first launch that uses TMA descriptors the host has just written. Out of line: later launches, which have nothing to fence, run past
+// a call (a served token takes the same with the loop inlined, 180.9 / 180.6 us, on 24 SMs 336.0 / 336.3).
 __device__ __noinline__ void fence_maps(const unsigned char* maps, int n) { for (int q = threadIdx.x; q < n; q += NTHR) tmap_fence(maps + 128 * (size_t)q); }
 
 // One kernel for launches that train, one for those that serve (bf16), one for both, each with and without time tables, because what a launch does not
-// run lies between what it does. Instructions are what most of a small task waits for: measured with straight-line code in a loop, 8 warps on an
-// SM, a warp instruction takes 1.9 clocks of its scheduler when the loop has 2 KB, 2.4 at 16 to 32 KB and 6.3 from 48 KB on (one warp a
-// scheduler: 1.1, 2.7, 6.1), and a task's code is not met again before hundreds of KB of others. So what is executed once per task is kept
-// short, loops are unrolled no further than their latency asks for, and what a sound run never executes is out of line.
+// run lies between what it does: a served token takes 182.4 us from the form that only serves and 182.9 from the one that does both, a step of 384
+// tokens 3,332 and 3,345, a char step 364 and 366. The char model alone serves faster from the form that does both (launch_kernel). Code that is not met
+// again before the instruction caches have lost it is slow to run, 6 clocks a warp instruction in a loop of 48 KB or more, 2 in one of 16 KB, but it is not
+// what a block waits for most: of the warps that are not held at a block barrier, 9 % wait for an instruction in small training steps and 4 % while
+// serving, 33 and 37 % for a load (profiles/scheduler_parts_and_stalls.md). So only what a sound run never executes is out of line, and loops are as timed.
 template <class T, int D, int DH, bool TRAIN, bool SERVE, bool PROF>
 __global__ void __launch_bounds__(NTHR, 2) ofa_kernel(const __grid_constant__ Ctx C) {
   extern __shared__ __align__(1024) unsigned char dsm[];

@@ -40,7 +40,7 @@ int shuffle_multiplier(unsigned seed, int phase, int n) {
 struct HostPhase { std::string name; PhaseDesc d; std::vector<Dep> deps; std::vector<char> rb_grain;   // per dependency: 1 = wait per 128-token row block instead of for the whole producer phase
                    int rb_map = 0; };                                                                   // how this phase's tasks map to row blocks (RbKind | a << 8), 0 = they do not
 
-// A job on the device: its tables (phase descriptors, scheduling records, prefix sums, dependencies) and its counters. Both live in
+// A job on the device: its tables (phase descriptors with their scheduling records, prefix sums, dependencies) and its counters. Both live in
 // memory of the caller: a context uploads the tables once and only clears the counters before each launch; ofa_run_phases packs
 // them into its workspace.
 struct HostJob {
@@ -289,7 +289,7 @@ Job place_job(const HostJob& h, int nsteps, unsigned char* host, unsigned char* 
 }
 
 // copies the first tickets of a job's phases into the kernel parameter when they fit
-void fill_param_records(Ctx& C, const HostJob* train, const HostJob* dec) {
+void fill_first_tickets(Ctx& C, const HostJob* train, const HostJob* dec) {
   C.train_pre_n = 0; C.dec_pre_n = 0;
   C.sched_flags = getenv("OFA_B200_LATE_TICKETS") ? 4 : 0;     // A/B switch for measurements: tickets only at the end of a task
   if (g_task_shuffle_seed) C.sched_flags |= 1;
@@ -620,18 +620,18 @@ bool build_train_graph(ofa_ctx* c) {
     // still has one thing to wait for.
     // n = 0, the default, chooses by how many blocks the chain's [tokens, d_model] products (128 x 128 tiles) leave idle. us per step with none / 16 / 32 tasks after
     // a phase, 12 layers and V = 50,304 (then 3 layers and V = 1,152 where measured):
-    //   whole GPU, 296 blocks    18 tiles  3,812 / 3,679 / 3,693 (840 / 836 / 806)    24 tiles  3,852 / 3,690 / 3,689    48 tiles  4,228 / 4,043 / 4,040
-    //                            96 tiles  4,834 / 4,683 / 4,703 (1,058 / 1,033 / 1,013)    108 tiles  4,868 / 4,781 / 4,833
-    //                            120 tiles 5,009 / 4,990 / 5,033 (1,072 / 1,074 / 1,068)    144 tiles  5,794 / 5,803 / 5,851 (1,232 / 1,234 / 1,215)
-    //   116 of 148 SMs, 232      18 tiles  3,915 / 3,676 / 3,692    48 tiles  4,506 / 4,389 / 4,407    72 tiles  4,611 / 4,514 / 4,566 (1,014 / 994 / 980)
-    //                            96 tiles  5,230 / 5,232 / 5,318 (1,144 / 1,143 / 1,132)    108 tiles  5,338 / 5,380 / 5,420
-    // So 32 up to an eighth of the blocks, where the smallest models gain most by it, and 16 above, up to half of them: from 0.4 of the blocks on there is next to
-    // nothing to gain. On a partition it costs there (an AdamW task is bound by what one block keeps in flight, and the chain loses its
-    // earliest blocks), so 16 only up to three eighths. How many phases come of it does not matter: scheduling records that no longer fit the kernel parameter are
-    // read from global memory at the same speed (14 layers, 48 tiles: 454 phases 4,557, 381 phases 4,557, not spread, 310 phases, 4,765; 12 layers, 396 phases 4,043 and 4,044).
-    // Not beside a serving job: its tokens/s fall by what the optimizer takes from it closer together (24 SMs, us per step and tokens/s without / with: 384
-    // tokens 4,272 and 2,286 / 3,972 and 2,216, 1,024 4,764 and 2,215 / 4,644 and 2,153, 1,536 4,817 and 2,182 / 4,717 and 2,117, 2,304 5,556 and
-    // 2,178 / 5,579 and 2,111). Which of the two counts more is the caller's to say.
+    //   whole GPU, 296 blocks    18 tiles  3,474 / 3,322 / 3,328 (727 / 729 / 702)    24 tiles  3,509 / 3,310 / 3,321    48 tiles  3,877 / 3,624 / 3,657
+    //                            96 tiles  4,346 / 4,101 / 4,159 (919 / 898 / 877)    108 tiles  4,386 / 4,191 / 4,331
+    //                            120 tiles 4,545 / 4,412 / 4,544 (919 / 917 / 913)    144 tiles  5,147 / 5,096 / 5,181 (1,039 / 1,047 / 1,024)
+    //   116 of 148 SMs, 232      18 tiles  3,579 / 3,364 / 3,379    48 tiles  4,065 / 3,824 / 3,860    72 tiles  4,161 / 3,984 / 4,062 (883 / 865 / 850)
+    //                            96 tiles  4,637 / 4,584 / 4,651 (979 / 982 / 969)    108 tiles  4,702 / 4,642 / 4,687
+    // So 32 up to an eighth of the blocks, where the smallest models gain most by it, and 16 above, up to half of them: there it gains 1 %, less than a step varies
+    // by. On a partition an AdamW task, bound by what one block keeps in flight, takes the chain's earliest blocks, so 16 only up to three eighths: from there on
+    // it gains 1 % of a large model and nothing of a small one (it cost as much while a task's hand-over took twice as long, which is when the line was drawn). How many phases come of it does not matter: first tickets that no longer fit the kernel parameter are
+    // read from global memory at the same speed (PARAM_TRAIN_PH).
+    // Not beside a serving job, unless asked for: while a hand-over took twice as long its tokens/s fell by 2 to 3 %. At present they hardly do (24 SMs, us per step and
+    // tokens/s without / with 16: 384 tokens 3,865 and 2,514 / 3,602 and 2,518, 1,024 4,226 and 2,471 / 3,993 and 2,479, 1,536 4,313 and 2,454 / 4,136 and
+    // 2,451, 2,048 4,815 and 2,438 / 4,739 and 2,432, 2,304 4,922 and 2,438 / 4,860 and 2,392). Which of the two counts more is the caller's to say.
     const int chain_tiles = bf ? (int)(N / 128 * (D / 128)) : train_blocks;
     const int most_tiles = train_blocks < c->nblocks ? train_blocks * 3 / 8 : train_blocks / 2;
     const int interleave = cfg.adam_interleave != 0 ? cfg.adam_interleave : cfg.use_decode ? -1 : 8 * chain_tiles <= train_blocks ? 32 : chain_tiles <= most_tiles ? 16 : -1;
@@ -889,7 +889,7 @@ bool place_jobs(ofa_ctx* c) {
   if (train) C.train = place_job(c->train_job, 0, img.data(), c->d_jobs, cnt);
   if (dec) C.dec = place_job(c->dec_job, 0, img.data() + tt, c->d_jobs + tt, cnt + ct);
   c->ar.h2d(c->d_jobs, img.data(), tab);
-  fill_param_records(C, train ? &c->train_job : nullptr, dec ? &c->dec_job : nullptr);
+  fill_first_tickets(C, train ? &c->train_job : nullptr, dec ? &c->dec_job : nullptr);
   C.use_train = train ? 1 : 0;
   C.status = c->d_status; C.finished = c->d_finished; C.arrived = c->d_finished + 1;
   return true;
@@ -1613,7 +1613,7 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   if (major != 10) return fail(nullptr, OFA_CUDA_ERROR, "sm_100a code only");
   const int nblocks = 2 * num_sms;
   std::string err;
-  // upper bound of the call's tables, to size the workspace before the phases are prepared: descriptors, records, one dependency
+  // upper bound of the call's tables, to size the workspace before the phases are prepared: descriptors, tables, one dependency
   // per phase (two for the first), at most four TMA descriptors per phase, counters, and what the kernel reports per repeat
   const size_t map_cap = (size_t)nph * sizeof(attn_tc::Maps), tab_cap = (size_t)nph * (sizeof(PhaseDesc) + 32 + sizeof(Dep)) + 1024;
   const size_t rep_bytes = up64(sizeof(unsigned long long) * (size_t)repeats) + up64(sizeof(float) * (size_t)repeats);
@@ -1675,10 +1675,9 @@ extern "C" int ofa_run_phases(int dtype, const ofa_dims* dims, const ofa_phase* 
   const size_t o_tab = map_cap, o_st = o_tab + job_table_bytes(hj), o_cnt = o_st + 192, total = o_cnt + job_counter_bytes(hj);
   if (total > ws.w.bytes) return fail(nullptr, OFA_CUDA_ERROR, "workspace too small");
   memset(ws.w.host + o_st, 0, total - o_st);
-  static thread_local Ctx C;      // 31 KB: not on the stack
-  memset(&C, 0, offsetof(Ctx, train_pre));
+  Ctx C{};
   C.train = place_job(hj, repeats, ws.w.host + o_tab, ws.w.dev + o_tab, ws.w.dev + o_cnt); C.md = m;
-  fill_param_records(C, &hj, nullptr);
+  fill_first_tickets(C, &hj, nullptr);
   if (adam) { C.hp.lr_max = adam[0]; C.hp.lr_min = adam[0]; C.hp.beta1 = adam[1]; C.hp.beta2 = adam[2]; C.hp.eps = adam[3]; C.hp.wd = adam[4]; C.hp.grad_scale = adam[5]; C.hp.constant_lr = 1; }
   C.train_sms = num_sms; C.use_train = 1;
   C.status = reinterpret_cast<DevStatus*>(ws.w.dev + o_st); C.finished = reinterpret_cast<int*>(ws.w.dev + o_st + 64); C.t_end = reinterpret_cast<unsigned long long*>(ws.w.dev + o_st + 128);

@@ -188,10 +188,10 @@ def test_spread_adamw_gives_the_same_bits(ofa, ctx, layers, vocab):
     (3, 8192, 384, 2, dict(tied_head=1, grad_bf16=1), None, 0),
     (3, 8192, 384, 2, dict(), None, 31337),
     (3, 1152, 384, 1, dict(), "OFA_B200_GLOBAL_RECS", 0),
-    (16, 1152, 384, 1, dict(), None, 0),                                                            # 412 phases: more records than fit the kernel parameter
+    (16, 1152, 384, 1, dict(), None, 0),                                                            # 412 phases: more first tickets than fit the kernel parameter
     (3, 1152, 384, 1, dict(infer_sms=24, reserved_sms=8, train_sms=116, use_decode=1, n_prompt=6, adam_interleave=16), None, 0)])
 def test_spread_adamw_gives_the_same_bits_in_every_form(ofa, monkeypatch, layers, vocab, ctx, batch, kw, env, shuffle):
-    """Tied head with bf16 gradients, permuted task order, scheduling records in global memory (asked for, or because they do not fit), live serving."""
+    """Tied head with bf16 gradients, permuted task order, first tickets in global memory (asked for, or because they do not fit), live serving."""
     lib = ofa.capi.load()
     out = []
     if env:
