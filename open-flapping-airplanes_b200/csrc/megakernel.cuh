@@ -251,11 +251,12 @@ __device__ __forceinline__ int wait_deps(const Ctx& C, const Job& J, const int c
       const bool over = lane == 0 && wait_over(C.status, t0, C.dep_timeout_ns + (C.dep_timeout_ns >> 1), h.z, h.w, h.y);
       if (__any_sync(0xffffffffu, over)) return -2;
     }
-    // A short wait, the rule along a chain of small phases, is polled without a pause, 32 polls being 5 to 10 us. Pausing later gains nothing: with limits of
-    // 32, 128 and 512 a step of 4 x 1,024 tokens took 6,087, 6,127 and 6,119 us, of 384 tokens 3,334, 3,334 and 3,328, beside a serving job 7,285, 7,282 and 7,285
-    // (2,352, 2,352 and 2,358 tokens/s), a served token 182.4 with 32 and 512; a copy by other SMs while all wait for an external flag 0.186 ms each time.
+    // No pause for 512 polls, 80 to 180 us, which is longer than nearly every wait: best of four with limits of 32 / 128 / 512 / 2,048, char step 359.5 / 356.3 /
+    // 354.7 / 355.1 us, two steps of 384 tokens (3 layers) 1,489 / 1,488 / 1,485 / 1,486, a layer as a list of phases 525.5 / 524.7 / 524.6 / 524.5. Nothing is
+    // slower for it: a step of 4 x 1,024 tokens 6,087 / 6,127 / 6,119, beside a serving job 7,285 / 7,282 / 7,285 (2,352 / 2,352 / 2,358 tokens/s), a served
+    // token 182.4 with 32 and 512, and a copy by other SMs while all blocks wait for an external flag takes 0.186 ms each time.
     // A counter seen complete is read again with the others: a step takes the same either way, a served token is 3 % slower if each lane remembers.
-    if (spins > 32u) __nanosleep(JOB == 1 ? 20 : 80);
+    if (spins > 512u) __nanosleep(JOB == 1 ? 20 : 80);
   }
 }
 static __device__ __noinline__ void end_of_step(unsigned long long* done, Live* live, int step, unsigned long long* t_end, int* finished) {
