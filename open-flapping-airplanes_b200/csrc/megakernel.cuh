@@ -17,6 +17,7 @@
 #pragma once
 #include "common.cuh"
 #include "task_api.h"
+#include "tickets.h"
 #include "elementwise.cuh"
 #include "gemm_tc.cuh"
 #include "attn_common.cuh"
@@ -319,9 +320,10 @@ __device__ __forceinline__ void job_loop(const Ctx& C, const Job& J, unsigned ch
       int4 h = make_int4(-2, 0, 0, 0);
       const unsigned g = have_next ? next_g : atomicAdd(J.ticket, 1u);
       if (g < total) {
-        int r = (int)(g - (unsigned)pos.y);
-        if (r >= J.tasks_per_step) {                     // a new step
-          do { r -= J.tasks_per_step; pos.x++; pos.y = (int)((unsigned)pos.y + (unsigned)J.tasks_per_step); } while (r >= J.tasks_per_step);
+        int step = pos.x; unsigned first = (unsigned)pos.y;
+        const int r = (int)place_ticket(g, (unsigned)J.tasks_per_step, step, first);
+        if (step != pos.x) {                             // a new step
+          pos = make_int2(step, (int)first);
           cur.x = -1; cur.z = 0;
           B.pos = pos;
         }
